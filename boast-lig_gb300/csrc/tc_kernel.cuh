@@ -219,9 +219,8 @@ __device__ __forceinline__ int imod(int a, int n) {
 }
 
 // Y * 2^se as an FP64, Y rounded to 53 bits to nearest-even (the rounding of
-// an int64 -> FP64 conversion), built from bits on the integer pipes: the
-// conversion instruction runs on the narrow FP64 pipe of this GPU.  ldexp
-// when the result is not a normal number.
+// an int64 -> FP64 conversion), for any se; ldexp when the result is not a
+// normal number.
 __device__ __forceinline__ double ll_scaled(long long Y, int se) {
     if (Y == 0) return 0.0;
     const unsigned long long sg = (unsigned long long)Y & 0x8000000000000000ull;
@@ -243,51 +242,46 @@ __device__ __forceinline__ double ll_scaled(long long Y, int se) {
     return ldexp(__longlong_as_double((long long)(sg | (1075ull << 52) | m)), e - 52 + se);
 }
 
-// The same conversion without branches, for the common case: `bad` records
-// a subnormal-or-infinite result exponent (the caller then redoes the
-// conversion with ll_scaled).  |Y| is normalised so its leading one is bit
-// 63; the 11 bits below the 53-bit mantissa and its last bit give
-// round-to-nearest-even (an increment exactly when low + lsb + 0x3FF carries
-// into bit 11), and a carry out of the mantissa moves into the exponent field.
-__device__ __forceinline__ double ll_scaled_fast(long long Y, int se, bool &bad) {
-    const unsigned long long u = (unsigned long long)Y;
-    const unsigned long long s = (unsigned long long)(Y >> 63);
-    const unsigned long long a = (u ^ s) - s;                    // |Y|
-    const int lz = __clzll((long long)a);                        // 64 when Y == 0
-    const unsigned long long nrm = a << (lz & 63);
-    const unsigned long long mant = nrm >> 11;                   // leading one at bit 52
-    const uint32_t nl = (uint32_t)nrm;
-    const uint32_t inc = ((nl & 0x7FFu) + ((nl >> 11) & 1u) + 0x3FFu) >> 11;
-    const int be = 1086 - lz + se;                               // exponent field
-    bad |= (unsigned)(be - 1) > 2045u;
-    const unsigned long long bits = (u & 0x8000000000000000ull) +
-                                    (((unsigned long long)(be - 1) << 52) + mant + inc);
-    return Y == 0 ? 0.0 : __longlong_as_double((long long)bits);
+// The same value with one conversion instruction when every non-zero result is
+// a normal number (-1022 <= se <= 961): the conversion rounds to nearest-even,
+// and se is added to its exponent field.  On this GPU the FP64 pipe takes 2
+// lanes a clock per SM and the integer pipes 64 each, so one FP64 instruction
+// per output (4.1 K cycles of a tile's ~20 K) costs less than the ~27 integer
+// instructions of the same normalisation, and a second one (a multiply by
+// 2^se) already sets the pace: MagicFilter3D on 32 x 128^3 1.87 ms all integer,
+// 1.80 with conversion and multiply, 1.56 with the conversion alone.
+__device__ __forceinline__ double ll_scaled_fast(long long Y, int se) {
+    const double t = __ll2double_rn(Y);
+    const int hi = __double2hiint(t);
+    return __hiloint2double(hi ? hi + (se << 20) : 0, __double2loint(t));
 }
 
 // Y = sum_k Acc_k 2^(46 - 8k) over the 8 order accumulators of one output,
 // from their biased bits b_k = Acc_k + 0x4B400000 (the bits of an FP32
-// accumulator that started at 1.5 * 2^23, |Acc_k| <= 2^22): orders 0-5 by
-// Horner modulo 2^64 (three 32x32+64 multiply-adds for the low terms, a
-// 32-bit add into the high word for the two top terms), orders 6-7 as the
-// nearest integer of Acc_6 / 4 + Acc_7 / 1024 (one 32-bit multiply-add and
-// an arithmetic shift, exact because that sum fits in 31 bits), then the
-// bias of every term removed by one 64-bit constant.  The wrap-around is
+// accumulator that started at 1.5 * 2^23, |Acc_k| <= 2^22), orders 6-7 as the
+// nearest integer of Acc_6 / 4 + Acc_7 / 1024.  Two neighbouring orders fit one
+// 32-bit word: w = 256 b_k + b_{k+1} = 257 * 0x4B400000 + (256 Acc_k +
+// Acc_{k+1}) modulo 2^32 stays within [0x4B000000, 0xCB800000], so it can be
+// taken as unsigned and the pair's bias removed by one constant for the whole
+// sum.  One multiply-add per pair and two 32x32+64 ones to join them, which run
+// on the multiply-add pipe beside the producers' ALU work.  The wrap-around is
 // exact because the true sum fits in 62 bits.
 template <int ORD>
 __device__ __forceinline__ long long horner_bal(const uint32_t (&b)[ORD]) {
     static_assert(ORD == 8, "eight order accumulators");
-    constexpr unsigned long long kW = (1ull << 46) + (1ull << 38) + (1ull << 30) + (1ull << 22) +
-                                      (1ull << 14) + (1ull << 6);
-    constexpr unsigned long long kBias = 0x4B400000ull * kW;
-    unsigned long long v = (unsigned long long)b[5] << 6;
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(b[4]), "r"(16384u), "l"(v));
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(b[3]), "r"(4194304u), "l"(v));
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(b[2]), "r"(1073741824u), "l"(v));
-    v += (unsigned long long)(b[1] * 64u + b[0] * 16384u) << 32;
-    // (Acc_6 * 256 + Acc_7 + 512) >> 10, the biases folded into one constant
-    const int lo = (int)(b[6] * 256u + b[7] + (512u - 257u * 0x4B400000u)) >> 10;
-    return (long long)(v + (unsigned long long)(long long)lo + (0ull - kBias));
+    constexpr uint32_t kPair = 257u * 0x4B400000u;              // bias of a pair, modulo 2^32
+    constexpr unsigned long long kBias =
+        (unsigned long long)kPair * ((1ull << 38) + (1ull << 22) + (1ull << 6));
+    // the low word of -kBias joins lo: 0 < lo + kLo < 2^32 (|lo| <= 2^20 + 1)
+    constexpr uint32_t kLo = (uint32_t)(0ull - kBias), kHi = (uint32_t)((0ull - kBias) >> 32);
+    static_assert(kLo > (1u << 21) && kLo < 0xFFE00000u, "no carry out of the low word");
+    const uint32_t w01 = b[0] * 256u + b[1], w23 = b[2] * 256u + b[3], w45 = b[4] * 256u + b[5];
+    const int lo = (int)(b[6] * 256u + b[7] + (512u - kPair)) >> 10;
+    unsigned long long v = ((unsigned long long)kHi << 32) | (kLo + (uint32_t)lo);
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(w45), "r"(64u), "l"(v));
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(w23), "r"(4194304u), "l"(v));
+    v += (unsigned long long)(w01 * 64u) << 32;
+    return (long long)v;
 }
 
 // FP32 bits -> FP64 value, integer only (normal, zero, subnormal flushed, inf/nan).
@@ -879,8 +873,12 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             const long long x2s = grow ? ys : S.nL;
             const int x2lo = grow ? S.out_lo : S.in_lo;
             const double *const xrow = xa + l + (long long)S.nL * S.in_ext * rr;
-            const int se = Er + F.ef - 58;
+            // a row holding an Inf or NaN gives NaN; farrow: the row's scale 2^se
+            // is outside the range of the fast conversion
             const bool nanrow = SCH == SCH_EXACT && Er == 0x7FFFFFFF;
+            const int se = nanrow ? 0 : Er + F.ef - 58;
+            const bool farrow = nanrow || se < -1022 || se > 961;
+            const double scale = __longlong_as_double((long long)(se + 1023) << 52);
             // no dot, a_x or a_y term: every output is its value (plus x2), stored
             const bool lean = !S.has_dot && !S.has_ax && S.ay_mode == 0;
 #pragma unroll 1
@@ -889,6 +887,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 const int e0 = 16 * (2 * hf + jj) + n0;         // first output element of the step
                 const int q0 = qc0 + e0 / NCH;                  // e0 is a multiple of 8
                 const int nv = (S.qhi - q0 + 1) * NCH;          // valid elements of the step
+                const bool plain = lean && nv >= 8;
                 // the x2 partials first, so their loads overlap the TMEM loads
                 double add[8];
                 if (KIND == KCONV && x2 && valid) {
@@ -912,7 +911,6 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 // one rare fix-up), then their memory side
                 double outv[8];
                 if constexpr (SCH == SCH_EXACT) {
-                    bool bad = false;
                     long long Y[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
@@ -921,15 +919,21 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                         for (int k = 0; k < G::ORD; ++k) bb[k] = acc[k][i];
                         Y[i] = horner_bal<G::ORD>(bb);
                     }
+                    if (farrow) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) outv[i] = ll_scaled_fast(Y[i], se, bad);
-                    if (bad) {                    // result not a normal number
+                        for (int i = 0; i < 8; ++i) {
+                            outv[i] = nanrow ? __longlong_as_double(0x7FF8000000000000LL)
+                                             : ll_scaled(Y[i], se);
+                            if (KIND == KCONV && x2 && plain) outv[i] += add[i];
+                        }
+                    } else if (KIND == KCONV && x2 && plain) {
+                        // scale and partial sum in one FP64 instruction (the
+                        // product is exact)
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) outv[i] = ll_scaled(Y[i], se);
-                    }
-                    if (nanrow) {
+                        for (int i = 0; i < 8; ++i) outv[i] = fma(__ll2double_rn(Y[i]), scale, add[i]);
+                    } else {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) outv[i] = __longlong_as_double(0x7FF8000000000000LL);
+                        for (int i = 0; i < 8; ++i) outv[i] = ll_scaled_fast(Y[i], se);
                     }
                 } else {                          // sum of the order accumulators
 #pragma unroll
@@ -941,8 +945,8 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     }
                 }
                 double *yq = ystep;
-                if (lean && nv >= 8) {
-                    if (KIND == KCONV && x2) {
+                if (plain) {
+                    if (SCH != SCH_EXACT && KIND == KCONV && x2) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) outv[i] += add[i];
                     }
