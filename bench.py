@@ -148,9 +148,9 @@ class MfKin128:
     a = [-0.5 / HGRID ** 2] * 3
     launches = 6                                     # 3 sweeps per operator
     # exact tensor-core mode: one shared line-exponent pass over x for the three kinetic
-    # sweeps; the first MagicFilter sweep takes its tile windows' exponents itself and hands
-    # the next sweep its line exponents, which hands them on to the third
-    exact_prepasses = 1
+    # sweeps and one before the first MagicFilter sweep, which hands the next sweep its line
+    # exponents, as that one does the third
+    exact_prepasses = 2
     # the whole step's algorithmic bytes per grid point: as separate sweeps (MagicFilter 3 x 16;
     # kinetic 16 + 24 + 24, its y and z sweeps reading x beside their partial sum) and with x
     # read once and both outputs written once (the floor of any fusion of the two operators)
@@ -220,7 +220,7 @@ class Wavelet96:
     n_out = 96 ** 3
     ops = ('idwt3d', 'dwt3d')
     launches = 6
-    exact_prepasses = 6                              # one line-exponent pass per sweep
+    exact_prepasses = 2                              # one per operator; its sweeps hand on theirs
     desc = ('{B} grids per GPU per step: d_idwt_sym8_narr (8 subbands of 48^3 -> 96^3) then '
             'd_dwt_sym8_narr (96^3 -> 8 x 48^3)')
 
@@ -1466,9 +1466,8 @@ def run_poisson(args, W):
                      'achieved_gbs': W.bytes_per_pt * N / step_s / 1e9,
                      'frac': W.bytes_per_pt * N / step_s / 1e9 / pk['hbm']}}
     # six sweeps, the edge kernels of the two sweeps along the non-periodic axis and the cc
-    # kernel; in the exact mode those two sweeps also make a line-exponent pass (the four
-    # periodic ones take their tile windows' exponents themselves)
-    launches = {'tc_exact': 11, 'fp64': 9}.get(args.mode, 9)
+    # kernel; in the exact mode every sweep makes a line-exponent pass
+    launches = {'tc_exact': 15, 'fp64': 9}.get(args.mode, 9)
     exact = args.mode in ('fp64', 'tc_exact')
     line = {'metric': W.metric, 'value': value, 'unit': UNIT, 'n_gpus': world, 'steps': args.steps,
             'warmup': max(args.warmup, 3), 'ms_per_step': ms / args.steps,

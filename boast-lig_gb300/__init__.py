@@ -340,10 +340,12 @@ class Hamiltonian:
         self.work = torch.empty(nwork, dtype=torch.float64, device=device)
         self.energies = torch.zeros(self.norb, 4, dtype=torch.float64, device=device)
 
-    # kernel launches of one call: 15 sweeps, in the exact tensor-core mode 13
-    # line-exponent passes (one shared by the three kinetic sweeps), the
-    # potential kernel and its reduction, and the three kinetic-energy reductions
-    LAUNCHES = {'exact': 33, 'other': 20}
+    # kernel launches of one call on free boundaries: 15 sweeps, the potential
+    # kernel and its reduction, and the three kinetic-energy reductions; in the
+    # exact tensor-core mode also 11 line-exponent passes (one for the three
+    # kinetic sweeps, one for the synthesis, whose sweeps hand on theirs when 2n
+    # is a multiple of 32; with other sizes 13)
+    LAUNCHES = {'exact': 31, 'other': 20}
 
     def __call__(self, psig, pot, hpsig, rho=None, stream=None, energies=None):
         """energies: optional device tensor of norb * 4 doubles to receive the

@@ -149,19 +149,21 @@ int configure(libconv_batch *b, int o, int engine, const int *ord) {
         if (tc && !sweep_tc_batch_supported(st.kind, st.ntaps))
             return report(LIBCONV_EMODE, "no batched tensor-core sweep for this filter");
         std::vector<long long> prefix(G + 1, 0);
-        for (int g = 0; g < G; ++g)
-            prefix[g + 1] = prefix[g] + (tc ? sweep_tc_tiles(st.sw[g]) : sweep_fp64_batch_blocks(st.sw[g], qc));
+        long long blocks = 0;                    // 128-line blocks of the launch
+        for (int g = 0; tc && g < G; ++g) blocks += sweep_tc_line_blocks(st.sw[g]);
+        for (int g = 0; g < G; ++g) {
+            if (tc && !tc_prepare(st.sw[g], blocks))
+                return report(LIBCONV_EARG, "batch grid too large for the tensor-core sweep");
+            prefix[g + 1] = prefix[g] + (tc ? sweep_tc_strips(st.sw[g]) : sweep_fp64_batch_blocks(st.sw[g], qc));
+        }
         st.units = prefix[G];
         if (tc) {
             const Sweep &S0 = st.sw[0];
             const int sch = scheme_of(b->mode);
             const double a = S0.has_a ? S0.a : 1.0;
-            if (sch == SCH_EXACT) tc_filter_digits(ftab + S0.ftab, S0.ntaps, a, st.F);
+            if (sch == SCH_EXACT) tc_filter_digits(S0.kind, ftab + S0.ftab, S0.ntaps, a, st.F);
             else tc_filter_split(ftab + S0.ftab, S0.ntaps, a, sch, st.F);
-            for (Sweep &S : st.sw) {
-                S.has_a = 0;   // folded into the filter operands
-                if (!tc_prepare(S)) return report(LIBCONV_EARG, "batch grid too large for the tensor-core sweep");
-            }
+            for (Sweep &S : st.sw) S.has_a = 0;   // folded into the filter operands
             if (sch == SCH_EXACT) {
                 // one pre-pass per stage writes every line's largest exponent
                 long long lines = 0, most = 0;
@@ -190,7 +192,7 @@ int configure(libconv_batch *b, int o, int engine, const int *ord) {
             return report(LIBCONV_ENOMEM, "batch descriptor allocation failed");
         }
         e = cudaMemcpy(st.d_prefix, prefix.data(), sizeof(long long) * (G + 1), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return report_cuda(e, "upload tile prefix");
+        if (e != cudaSuccess) return report_cuda(e, "upload strip prefix");
     }
     C.engine = engine;
     for (int i = 0; i < 3; ++i) C.order[i] = ord[i];
@@ -229,7 +231,7 @@ int launch_op(libconv_batch *b, int o, int *status, cudaStream_t stream) {
     for (Stage &st : C.stages) {
         cudaError_t e;
         if (C.engine == LIBCONV_ENGINE_TC)
-            e = launch_sweep_tc_batch(st.kind, st.ntaps, st.d_desc, st.d_prefix, b->ngrids, st.F,
+            e = launch_sweep_tc_batch(st.kind, st.ntaps, st.bound[0], st.d_desc, st.d_prefix, b->ngrids, st.F,
                                       scheme_of(b->mode), status, st.d_lineE, st.exp_blocks, stream);
         else
             e = launch_sweep_fp64_batch(st.kind, st.ntaps, C.engine == LIBCONV_ENGINE_FP64_Q32 ? 32 : 64,

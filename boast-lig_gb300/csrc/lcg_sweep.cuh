@@ -31,23 +31,25 @@ struct Sweep {
     double a, a_x, a_y;
     double *dot_part;         // one partial per block (device), when has_dot
     long long le_off = 0;     // first entry of this sweep's lines in a batched line-exponent array
-    // tensor-core sweeps: the divisors of the tile index (output chunks per
+    // tensor-core sweeps (filled by tc_prepare): the output blocks of a strip
+    // (a segment of a line), and the divisors of the strip index (segments per
     // line block, line blocks per array, nL) with their multiplicative
-    // inverses, q = (n * m) >> s for every n < 2^31 (filled by tc_prepare)
+    // inverses, q = (n * m) >> s for every n < 2^31
+    int seg_blocks = 0;
     unsigned int tdiv_d[3] = {1, 1, 1}, tdiv_m[3] = {0, 0, 0}, tdiv_s[3] = {0, 0, 0};
-    // tensor-core convolution sweeps: the tile's input window starts woff
+    // tensor-core convolution sweeps: a strip's input window starts woff
     // elements before the first input position, so that along contiguous
     // lines its 8-element groups start on 32-byte boundaries (0 otherwise)
     int woff = 0;
     // per array: 0 = skip the array's lines (its output is left as it is); null:
     // every array (sweeps without a dot product only)
     const int *active = nullptr;
-    // exact tensor-core transposed convolution sweeps whose tiles hold whole
-    // lines of the next sweep (run_plan decides): the epilogue writes the
-    // largest exponent field of each of the next sweep's lines,
-    // le_next[a le_next_lines + i2 + le_n2 (q - out_lo)], for this sweep's line
-    // i1 + le_n1 i2 and output q (le_n1 = the next sweep's line length: 32, 64
-    // or 128, so that every tile column covers whole lines)
+    // exact tensor-core transposed sweeps that hand the next sweep its line
+    // exponents (run_plan decides): the epilogue raises the largest exponent
+    // field of each of the next sweep's lines, zeroed before the launch,
+    // le_next[a le_next_lines + i2 + le_n2 e], for this sweep's line i1 + le_n1
+    // i2 and output element e (le_n1 = the next sweep's line length, a multiple
+    // of 32: a warp's 32 rows belong to one of its lines)
     int *le_next = nullptr;
     long long le_next_lines = 0;
     int le_n1 = 0, le_n2 = 0;

@@ -418,35 +418,40 @@ struct Scratch {
     size_t nle = 0;
 };
 
-// Elements of dot partials and of line exponents that run_plan(P) needs in
-// the calling thread's mode.
 // Exact tensor-core step k hands its successor the line exponents of its
-// output (the epilogue writes them, Sweep::le_next) instead of a pre-pass
-// over that output: k is a periodic transposed convolution with the plain
-// store path (no dot, a_x, a_y or x2) over whole tiles of valid lines, k + 1 a
-// periodic convolution reading k's output along its fastest axis (length n1
-// = 32, 64 or 128, so that every tile column holds whole lines of k + 1: k's
-// line i1 + n1 i2 and output q are k + 1's line i2 + n2 q at position i1).
+// output (the epilogue's atomics, Sweep::le_next) instead of a pre-pass over
+// that output: k is a transposed sweep (16 taps, or a wavelet's) without dot, a_x,
+// a_y or x2, k + 1 reads
+// k's output along its fastest axis (n1 elements a line, none of them padding),
+// and n1 and k's lines are multiples of 32, so that each epilogue warp's rows
+// belong to one line of k + 1 in every output column: k's line i1 + n1 i2 and
+// output e are k + 1's line i2 + n2 e at element i1.
+// 32 arrays of 128^3: the pre-pass takes 81 us.
 bool exp_handoff(const Plan &P, size_t k, int &n1, int &n2) {
     if (t_mode != LIBCONV_MODE_TC_EXACT || k + 1 >= P.steps.size()) return false;
     const PlanStep &a = P.steps[k], &b = P.steps[k + 1];
     const Sweep &A = a.S, &B = b.S;
-    if (!(A.kind == KCONV && A.transpose && A.nL == 1 && A.bc == BC_PERIODIC && !A.has_dot &&
-          !A.has_ax && A.ay_mode == 0 && a.src2 < 0 && sweep_tc_supported(A)))
+    if (!(A.transpose && A.nL == 1 && (A.kind != KCONV || A.ntaps == 16) && !A.has_dot && !A.has_ax && A.ay_mode == 0 && a.src2 < 0 &&
+          sweep_tc_supported(A)))
         return false;
-    if (!(B.kind == KCONV && B.nL == 1 && B.bc == BC_PERIODIC && b.src == a.dst && b.exp_axis < 0 &&
-          B.narr == A.narr && B.x_arr == A.y_arr && sweep_tc_supported(B)))
+    if (!(B.nL == 1 && b.src == a.dst && b.exp_axis < 0 && B.narr == A.narr && B.x_arr == A.y_arr &&
+          sweep_tc_supported(B)))
         return false;
-    const long long lines = (long long)A.nL * A.nR;
-    if (!(B.n == 32 || B.n == 64 || B.n == 128) || lines % 128 || lines % B.n) return false;
-    if ((A.qhi - A.qlo + 1) % 64 || A.out_lo != 0 || A.qlo != 0 || B.in_lo != 0 || B.in_ext != B.n)
-        return false;
-    if ((long long)B.nR != lines / B.n * A.out_ext) return false;
-    n1 = B.n;
-    n2 = (int)(lines / B.n);
+    const int mA = A.kind == KCONV ? 1 : 2, mB = B.kind == KCONV ? 1 : 2;
+    const long long lines = A.nR, len = (long long)B.in_ext * mB;
+    if (len % 32 || lines % 32 || lines % len) return false;
+    // every element of A's output is written, and every one of B's lines is used
+    if (A.qhi - A.qlo + 1 != A.out_ext || A.qlo != A.out_lo) return false;
+    const int used = B.bc == BC_SHRINK ? B.qhi + B.lowfil + B.ntaps - B.in_lo : B.n;
+    if (used != B.in_ext) return false;
+    if ((long long)B.nR != lines / len * A.out_ext * mA) return false;
+    n1 = (int)len;
+    n2 = (int)(lines / len);
     return true;
 }
 
+// Elements of dot partials and of line exponents that run_plan(P) needs in
+// the calling thread's mode.
 void plan_scratch(const Plan &P, size_t &ndot, size_t &nle) {
     ndot = nle = 0;
     const bool exact = t_mode == LIBCONV_MODE_TC_EXACT;
@@ -458,7 +463,7 @@ void plan_scratch(const Plan &P, size_t &ndot, size_t &nle) {
         const Sweep &S = ps.S;
         const bool tc = t_mode != LIBCONV_MODE_FP64 && sweep_tc_supported(S);
         if (S.has_dot) {
-            const size_t nb = tc ? (size_t)sweep_tc_blocks(S) * 8 * S.narr : (size_t)sweep_fp64_blocks(S);
+            const size_t nb = tc ? (size_t)sweep_tc_blocks(S) * kTcDotSlots * S.narr : (size_t)sweep_fp64_blocks(S);
             if (nb > ndot) ndot = nb;
         }
         const bool shared = exact && P.exp3[0] > 0 && ps.exp_axis >= 0 && ps.src == B_X;
@@ -537,14 +542,14 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
         long long nb = 0, seg = 0;   // dot partials: total, and per array (array-major)
         if (S.has_dot) {
             if (tc) {
-                seg = sweep_tc_blocks(S) * 8;
+                seg = sweep_tc_blocks(S) * kTcDotSlots;
                 nb = seg * S.narr;
             } else {
                 nb = sweep_fp64_blocks(S);
                 seg = nb / S.narr;
             }
             S.dot_part = sc.dot;
-            if (tc && S.narr > 1) {   // slots of arrays a CTA has no tile of stay 0
+            if (tc && S.narr > 1) {   // slots of arrays a CTA has no strip of stay 0
                 cudaError_t e = cudaMemsetAsync(S.dot_part, 0, (size_t)nb * sizeof(double), st);
                 if (e != cudaSuccess) return cuda_fail(e, "clear dot partials");
             }
@@ -556,7 +561,7 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
                             : t_mode == LIBCONV_MODE_TC_BF16X3 ? SCH_BF16X3
                                                                : SCH_TF32X3;
             const int flat = S.kind == KCONV ? S.ntaps : 4 * S.ntaps;   // LE|LO|HE|HO
-            if (sch == SCH_EXACT) tc_filter_digits(h_ftab + S.ftab, flat, S.has_a ? S.a : 1.0, F);
+            if (sch == SCH_EXACT) tc_filter_digits(S.kind, h_ftab + S.ftab, flat, S.has_a ? S.a : 1.0, F);
             else tc_filter_split(h_ftab + S.ftab, flat, S.has_a ? S.a : 1.0, sch, F);
             S.has_a = 0;   // folded into the filter operands
             int *lineE = nullptr;
@@ -576,6 +581,8 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
                     S.le_n1 = n1;
                     S.le_n2 = n2;
                     handed = true;
+                    e = cudaMemsetAsync(le_other, 0, (size_t)S.le_next_lines * B.narr * sizeof(int), st);
+                    if (e != cudaSuccess) return cuda_fail(e, "clear line exponents");
                 }
             }
             e = launch_sweep_tc(S, F, sch, status, lineE, st, ready);

@@ -25,13 +25,6 @@ int sm_count() {
     return g_sms[dev];
 }
 
-// 128-line x qp-output-position tiles of one sweep (all narr arrays).
-long long tile_count_for(const Sweep &S, int qp) {
-    const long long nlines = (long long)S.nL * S.nR;
-    const long long nq = S.qhi - S.qlo + 1;
-    return ((nlines + 127) / 128) * ((nq + qp - 1) / qp) * S.narr;
-}
-
 // Largest exponent field over the elements each line of S uses (positions
 // 0..plen-1 of every channel; ld padding is not read), one int per line of
 // every array.  Contiguous lines (nL == 1): a warp per line, lanes along the
@@ -204,12 +197,45 @@ static void fast_div(unsigned int d, unsigned int &dd, unsigned int &m, unsigned
     m = (unsigned int)(((1ull << s) + d - 1) / d);
 }
 
-bool tc_prepare(Sweep &S) {
-    const int qp = S.kind == KCONV ? 64 : 32;
-    const long long nlines = (long long)S.nL * S.nR;
-    const long long nch = (S.qhi - S.qlo + qp) / qp, nlb = (nlines + 127) / 128;
-    if (nlines < 1 || nlines >= (1LL << 31) || nch * nlb * S.narr >= (1LL << 31)) return false;
-    fast_div((unsigned int)nch, S.tdiv_d[0], S.tdiv_m[0], S.tdiv_s[0]);
+// 128-line blocks of one sweep (all narr arrays), 16-element output blocks
+// along a line, and slabs a block reads (Geom::W).
+static long long line_blocks(const Sweep &S) {
+    return ((long long)S.nL * S.nR + 127) / 128 * S.narr;
+}
+static int out_blocks(const Sweep &S) {
+    const int pb = S.kind == KCONV ? 16 : 8;
+    return (S.qhi - S.qlo + pb) / pb;
+}
+static int window_slabs(const Sweep &S) {
+    const int nch = S.kind == KCONV ? 1 : 2;
+    return (nch * (16 / nch + S.ntaps - 1) + 15) / 16;
+}
+
+// Output blocks per strip, for `blocks` line blocks in the launch: the split
+// of the lines that gives the busiest CTA the least slabs to convert (its
+// strips times nb + W - 1); whole lines unless a launch has few of them.
+static int strip_blocks(const Sweep &S, long long blocks) {
+    const int n = out_blocks(S), halo = window_slabs(S) - 1, sms = tck::sm_count();
+    int best = n;
+    long long cost = -1;
+    for (int seg = 1; seg <= n && seg <= 64; ++seg) {
+        const int nb = (n + seg - 1) / seg;
+        const long long strips = blocks * ((n + nb - 1) / nb);
+        const long long c = (strips + sms - 1) / sms * (nb + halo);
+        if (cost < 0 || c < cost) {
+            cost = c;
+            best = nb;
+        }
+    }
+    return best;
+}
+
+bool tc_prepare(Sweep &S, long long blocks) {
+    const long long nlines = (long long)S.nL * S.nR, nlb = (nlines + 127) / 128;
+    S.seg_blocks = strip_blocks(S, blocks > 0 ? blocks : line_blocks(S));
+    const long long seg = (out_blocks(S) + S.seg_blocks - 1) / S.seg_blocks;
+    if (nlines < 1 || nlines >= (1LL << 31) || seg * nlb * S.narr >= (1LL << 31)) return false;
+    fast_div((unsigned int)seg, S.tdiv_d[0], S.tdiv_m[0], S.tdiv_s[0]);
     fast_div((unsigned int)nlb, S.tdiv_d[1], S.tdiv_m[1], S.tdiv_s[1]);
     fast_div((unsigned int)S.nL, S.tdiv_d[2], S.tdiv_m[2], S.tdiv_s[2]);
     return true;
@@ -220,10 +246,17 @@ bool sweep_tc_supported(const Sweep &S) {
     return (S.kind == KDEC || S.kind == KREC) && (S.ntaps == 8 || S.ntaps == 16);
 }
 
+long long sweep_tc_strips(const Sweep &S) {
+    const int nb = S.seg_blocks > 0 ? S.seg_blocks : strip_blocks(S, line_blocks(S));
+    return line_blocks(S) * ((out_blocks(S) + nb - 1) / nb);
+}
+
+long long sweep_tc_line_blocks(const Sweep &S) { return line_blocks(S); }
+
 long long sweep_tc_blocks(const Sweep &S) {
-    const long long tiles = tck::tile_count_for(S, S.kind == KCONV ? 64 : 32);
+    const long long strips = sweep_tc_strips(S);
     const int sms = tck::sm_count();
-    return tiles < sms ? tiles : sms;
+    return strips < sms ? strips : sms;
 }
 
 // Filter digits with the operator scalar folded in exactly: a*f is formed as
@@ -234,8 +267,15 @@ long long sweep_tc_blocks(const Sweep &S) {
 // the kernel's recombined 64-bit result below 2^61).  F is cut into 8
 // balanced byte digits e_0 (top) .. e_7 in [-128, 127]:
 // F = sum_t e_t 256^(7-t), the bytes of F + 0x8080808080808080 minus 128.
-void tc_filter_digits(const double *taps, int ntaps, double a, TcFilter &F) {
-    memset(&F, 0, sizeof(F));
+// The operand holds the data's balanced digits plus 128 (0..255), so order k's
+// accumulator lies between minus and plus 255 times the sums of the negative
+// and of the positive digits e_0 .. e_k of an output's taps; both must stay
+// within the 2^22 units that the biased FP32 accumulator holds exactly.  The
+// library's filters reach half of that; where a scalar's digits do not fit, ef
+// is raised by one and the digits cut again.
+void tc_filter_digits(int kind, const double *taps, int ntaps, double a, TcFilter &F) {
+    F = TcFilter{};
+    memset(F.dig, 0, sizeof(F.dig));
     int ea = 0;
     const double fa = frexp(fabs(a), &ea);                          // |a| = fa 2^ea
     const unsigned long long ma = (unsigned long long)ldexp(fa, 53);  // 53-bit integer
@@ -258,20 +298,47 @@ void tc_filter_digits(const double *taps, int ntaps, double a, TcFilter &F) {
     }
     if (ef == -100000) ef = 0;
     while (sum >= ldexp(8.0, ef)) ++ef;
-    F.ef = ef;
-    for (int i = 0; i < ntaps; ++i) {
-        const int sh = ep[i] + 62 - ef;                             // |F| = prod 2^sh <= 2^62
-        const unsigned __int128 v = prod[i];
-        unsigned long long M;
-        if (sh >= 0) M = (unsigned long long)(v << sh);
-        else if (-sh >= 127) M = 0;
-        else M = (unsigned long long)((v + ((unsigned __int128)1 << (-sh - 1))) >> (-sh));
-        const bool neg = (a < 0) != (taps[i] < 0);
-        const unsigned long long X = neg ? 0ull - M : M;           // two's complement
-        const unsigned long long U = X + 0x8080808080808080ull;
-        for (int t = 0; t < TcFilter::kSlices; ++t) {
-            const int digit = (int)((U >> (8 * (7 - t))) & 0xFF) - 128;
-            F.dig[t][i] = __half_as_ushort(__int2half_rn(digit));
+    // output channel of a tap of the flat filter: wavelet decompose LE, LO give
+    // the first and HE, HO the second; recompose LO, HO the first, LE, HE the second
+    const int nt = kind == KCONV ? ntaps : ntaps / 4;
+    auto channel = [&](int i) {
+        return kind == KCONV ? 0 : kind == KDEC ? (i / nt >= 2) : (i / nt) % 2 == 0;
+    };
+    constexpr long long kMost = 1ll << 22;
+    for (bool fits = false; !fits; ++ef) {
+        F.ef = ef;
+        long long esum[TcFilter::kSlices][2] = {}, pos[2] = {}, neg[2] = {};
+        fits = true;
+        for (int t = 0; t < TcFilter::kSlices; ++t)
+            for (int i = 0; i < ntaps; ++i) {
+                const int sh = ep[i] + 62 - ef;                     // |F| = prod 2^sh <= 2^62
+                const unsigned __int128 v = prod[i];
+                unsigned long long M;
+                if (sh >= 0) M = (unsigned long long)(v << sh);
+                else if (-sh >= 127) M = 0;
+                else M = (unsigned long long)((v + ((unsigned __int128)1 << (-sh - 1))) >> (-sh));
+                const bool negative = (a < 0) != (taps[i] < 0);
+                const unsigned long long X = negative ? 0ull - M : M;   // two's complement
+                const unsigned long long U = X + 0x8080808080808080ull;
+                const int digit = (int)((U >> (8 * (7 - t))) & 0xFF) - 128, c = channel(i);
+                F.dig[t][i] = __half_as_ushort(__int2half_rn(digit * 256));
+                esum[t][c] += digit;
+                (digit > 0 ? pos[c] : neg[c]) += digit > 0 ? digit : -digit;
+                fits = fits && 255 * pos[c] <= kMost && 255 * neg[c] <= kMost;
+            }
+        // biases of the eight accumulators (modulo 2^32 for a pair of orders) and the
+        // offsets C_k = 128 sum_t<=k esum[t] of the data digits, subtracted
+        constexpr uint32_t kPair = 257u * kAccBias;
+        for (int c = 0; c < 2; ++c) {
+            unsigned long long k64 = (unsigned long long)kPair * ((1ull << 38) + (1ull << 22) + (1ull << 6));
+            long long ck = 0;
+            for (int k = 0; k < 6; ++k) {
+                ck += 128 * esum[k][c];
+                k64 += (unsigned long long)ck << (46 - 8 * k);
+            }
+            const long long c6 = ck + 128 * esum[6][c], c7 = c6 + 128 * esum[7][c];
+            F.k64[c] = (long long)(0ull - k64);
+            F.k67[c] = 512u - kPair - (uint32_t)(256 * c6 + c7);
         }
     }
 }
@@ -298,10 +365,6 @@ void tc_filter_split(const double *taps, int ntaps, double a, int sch, TcFilter 
     }
 }
 
-long long sweep_tc_tiles(const Sweep &S) {
-    return tck::tile_count_for(S, S.kind == KCONV ? 64 : 32);
-}
-
 bool sweep_tc_batch_supported(int kind, int ntaps) {
     return kind == KCONV && (ntaps == 16 || ntaps == 29);
 }
@@ -312,7 +375,7 @@ int line_exp_batch_blocks(long long max_lines, bool contiguous) {
     return (int)(want < 1 ? 1 : want > 64 ? 64 : want);
 }
 
-cudaError_t launch_sweep_tc_batch(int kind, int ntaps, const Sweep *descs, const long long *prefix,
+cudaError_t launch_sweep_tc_batch(int kind, int ntaps, const Sweep &like, const Sweep *descs, const long long *prefix,
                                   int nsweeps, const TcFilter &F, int sch, int *status,
                                   int *lineE, int exp_blocks, cudaStream_t st) {
     if (sch == SCH_EXACT) {
@@ -322,27 +385,16 @@ cudaError_t launch_sweep_tc_batch(int kind, int ntaps, const Sweep *descs, const
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }
-        return tck::launch_exact_batch(kind, ntaps, descs, prefix, nsweeps, F, status, lineE, st);
+        return tck::launch_exact_batch(kind, ntaps, like, descs, prefix, nsweeps, F, status, lineE, st);
     }
-    if (sch == SCH_BF16X3) return tck::launch_bf16x3_batch(kind, ntaps, descs, prefix, nsweeps, F, status, st);
-    if (sch == SCH_TF32X3) return tck::launch_tf32x3_batch(kind, ntaps, descs, prefix, nsweeps, F, status, st);
+    if (sch == SCH_BF16X3) return tck::launch_bf16x3_batch(kind, ntaps, like, descs, prefix, nsweeps, F, status, st);
+    if (sch == SCH_TF32X3) return tck::launch_tf32x3_batch(kind, ntaps, like, descs, prefix, nsweeps, F, status, st);
     return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_sweep_tc(const Sweep &S, const TcFilter &F, int sch, int *status, int *lineE,
                             cudaStream_t st, bool lineE_ready) {
     if (sch == SCH_EXACT) {
-        // Periodic convolution lines at least one tile window long: the
-        // producers load each 8-element group as one or two runs (vectors on
-        // contiguous lines, one coalesced load per element across the warp's
-        // lines otherwise), and a first pass over those loads gives each tile
-        // window's largest exponent at less cost than a pass over the array
-        // (32 x 128^3: MagicFilter3D 2.00 -> 1.93 ms; a 1D MagicFilter sweep
-        // along axis 1 0.686 -> 0.613 ms).  The window's scale is the line's
-        // or a finer one.
-        if (lineE && !lineE_ready && S.kind == KCONV && S.bc == BC_PERIODIC &&
-            S.n >= tck::exact_conv_window(S.ntaps))
-            lineE = nullptr;
         if (lineE && !lineE_ready) {
             const int plen = tck::line_exp_plen(S);
             const long long total = sweep_tc_lines(S);

@@ -18,12 +18,12 @@ cudaError_t launch_tf32x3(const Sweep &S, const TcFilter &F, int *status, const 
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_tf32x3_batch(int kind, int ntaps, const Sweep *descs, const long long *prefix,
+cudaError_t launch_tf32x3_batch(int kind, int ntaps, const Sweep &like, const Sweep *descs, const long long *prefix,
                                int nsweeps, const TcFilter &F, int *status, cudaStream_t st) {
     if (kind == KCONV && ntaps == 16)
-        return launch_batch<KCONV, 16, SCH_TF32X3>(descs, prefix, nsweeps, F, status, nullptr, st);
+        return launch_batch<KCONV, 16, SCH_TF32X3>(like, descs, prefix, nsweeps, F, status, nullptr, st);
     if (kind == KCONV && ntaps == 29)
-        return launch_batch<KCONV, 29, SCH_TF32X3>(descs, prefix, nsweeps, F, status, nullptr, st);
+        return launch_batch<KCONV, 29, SCH_TF32X3>(like, descs, prefix, nsweeps, F, status, nullptr, st);
     return cudaErrorInvalidValue;
 }
 

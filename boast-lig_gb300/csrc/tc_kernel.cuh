@@ -1,26 +1,30 @@
 // tcgen05 tensor-core sweep, shared by the exact-digit and split-precision
-// forms (instantiated in sweep_tc_exact.cu and sweep_tc_split.cu).
+// forms (instantiated in sweep_tc_exact.cu, sweep_tc_bf16x3.cu, sweep_tc_tf32x3.cu
+// and sweep_tc_fd.cu).
 //
 // One sweep = one banded Toeplitz product per 16-output block:
 //   D[line, n] = sum_kk A[line, kk] * B[kk, n]
-// A holds the tile's input elements (128 lines x KT elements), B the filter:
+// A holds a window of input elements (128 lines x K elements), B the filter:
 // B[kk, n] = f_{c,c'}(kk/NCH - n/NCH) with c = n mod NCH, c' = kk mod NCH, where
 // NCH = 1 for a convolution and 2 for the wavelet polyphase pairs (elements are
 // (pair, channel), interleaved), so K = 32 or 48 for every filter here.
 //
 // Scheme SCH_EXACT (FP64-accurate, exact integer arithmetic on FP16 operands)
-//   * each line segment of a tile is scaled by the power of two above its
-//     largest magnitude to signed 62-bit integers X = x 2^(62-E) (|X| <=
+//   * each line is scaled by the power of two above its largest magnitude
+//     (line_exp_kernel, or the sweep before: Sweep::le_next) to signed 62-bit integers X = x 2^(62-E) (|X| <=
 //     2^62, truncated toward zero); X is cut into 8 balanced byte digits
 //     d_0 (top) .. d_7 in [-128, 127], X = sum_s d_s 256^(7-s): the bytes
-//     of X + 0x8080808080808080 minus 128, exact in FP16;
+//     of X + 0x8080808080808080 minus 128.  The operand keeps the bytes d_s +
+//     128 themselves, as FP16 subnormals (units of 2^-24), and the 128 leaves
+//     with a constant per order, 128 sum_t<=k sum_taps e_t;
 //   * the filter, with the operator scalar a folded in exactly (128-bit
 //     product of the two mantissas), is cut the same way into e_0..e_7;
-//   * byte-pair products are at most 2^14 in magnitude and every partial
-//     sum over <= 32 products x 8 pairs stays within 2^22; every TMEM
-//     accumulator starts at 1.5 * 2^23 (one MMA of a constant tile per output
-//     block), so all its values are integers in [2^23, 2^24], where FP32 is
-//     exact, and its bits are 0x4B400000 plus the sum;
+//   * every partial sum of byte products stays within 2^22 units (checked on
+//     the filter's digits, tc_filter_digits); every TMEM accumulator starts at
+//     1.5 * 2^23 units (one MMA of a constant tile per output block), so all
+//     its values are integers in [2^23, 2^24] units, where FP32 is exact, and
+//     its bits are kAccBias plus the sum (the filter's digits are stored times
+//     2^8, so the unit is 2^-16);
 //   * the 36 pairs of order k = s + t <= 7 are accumulated, one TMEM
 //     accumulator per order; the epilogue recombines
 //     Y = sum_k Acc_k 2^(46-8k) in int64 (the orders 6-7 rounded to an
@@ -28,8 +32,7 @@
 //   Dropped orders (k >= 8) weigh below 2^-70 of the product of the line and
 //   filter scales; the data truncation (2^-62 of the line scale) and the
 //   final roundings stay below the rounding of an FP64 FMA chain.
-//   Lines never share a scale; a line segment holding an Inf or NaN gives
-//   NaN on that tile row.
+//   Lines never share a scale; a line holding an Inf or NaN gives NaN.
 //
 // Split-precision schemes (FP32-class accuracy, reported per operator)
 //   * every element is rounded to FP32 (magnitudes outside the normal float
@@ -41,30 +44,49 @@
 //     elements, K = 8 per MMA);
 //   * one FP32 accumulator per output: relative error near 1e-7.
 //
-// Persistent, warp-specialised CTA (one per SM), 512 threads at <= 128
-// registers, one A buffer used as a ring of three chunk pairs (input elements
-// [0, 32), [32, 64), [64, KT)) and two TMEM accumulator halves (output blocks
-// 0-1, which read pairs 0-1, and blocks 2-3, which read pairs 1-2):
-//   warps 0-7  producers: thread = (row, half of every pair); exact scheme:
-//              largest exponent of the row, then its byte digits; split
-//              schemes: bfloat16 / tf32 terms; coalesced or vector loads.  The
-//              pairs of a tile are written in order, pair 0 as soon as the
-//              previous tile's half-0 MMAs completed, pairs 1-2 once both
-//              halves' did, so the next tile's production overlaps the MMAs;
-//   warps 8-15 epilogue: group 0 (warps 8-11) owns TMEM half 0, group 1
-//              (12-15) half 1.  The group's first warp issues its half's MMAs
-//              (lane 0, fully unrolled, precomputed descriptors) once the
-//              pairs they read are written, then the group drains the half:
-//              thread = TMEM lane = tile row; TMEM -> FP64 -> global.
-// Every hand-off is an mbarrier whose phase can never run two phases ahead of
-// its waiter; every wait gives up after ~2 s of SM clock (status word set,
-// TMEM freed, kernel returns).  In single-sweep launches every role skips the
-// tiles of an array whose S0.active flag is 0 (flags fixed for the launch), so
-// the roles still meet on the same tiles and count only those.
+// Persistent, warp-specialised CTA (one per SM), 512 threads at 128 registers.
+// The unit of work is a strip: 128 lines and a run of consecutive 16-element
+// output blocks along them (the whole line, or one of the segments it is cut
+// into when a launch has few lines, tc_prepare).  Along a strip the input is cut
+// into 16-element slabs; output block j reads slabs j .. j + W - 1 (W = 2, or 3
+// for 29 and 2 x 16 taps), so neighbouring blocks share them: each element is
+// converted once per strip, and the operand buffer is a ring of 6 slabs that
+// conversion, MMAs and epilogue walk at their own pace, across strip ends too:
+//   warps 0-7  producers: thread = (row, half of the slab's 16 elements); exact
+//              scheme: byte digits; split schemes: bfloat16 / tf32 terms;
+//              coalesced or vector loads, the next slab's in flight;
+//   warps 8-15 epilogue: thread = TMEM lane = row; warps 8-11 take the even
+//              blocks, warps 12-15 the odd ones; TMEM -> FP64 -> global.  Before
+//              it drains a block, one of the group's warps in turn (lane 0,
+//              unrolled) issues the MMAs of the group's next one into the other
+//              of its two TMEM slots.
+// Hand-offs (mbarriers): full[slab] producers -> issuer, empty[slab] MMAs ->
+// producers (every block that reads a slab commits to it; the issuer of the
+// first reader adds the arrivals of the readers a strip's ends do not have),
+// tfull[slot] MMAs and issuer -> epilogue, drained[slot] epilogue -> issuer.
+// No phase can run two ahead of its waiter; every wait gives up after kWaitPolls
+// polls (status word set, TMEM freed, kernel returns).  In single-sweep launches
+// every role skips the strips of an array whose S0.active flag is 0 (flags fixed
+// for the launch), so the roles still meet on the same strips.
+//
+// What bounds it (32 grids of 128^3, a launch of 67 M outputs): the instructions
+// of the two roles and their latency with 16 warps per SM.  Before, tiles of 64
+// outputs held the whole operand buffer, so conversion, MMAs and drain of a tile
+// ran one after the other, and every tile converted its halo again; the kernel
+// was 190 KB of code with one epilogue for every case.  MagicFilter sweep 520 ->
+// 325 us, kinetic sweep along x 600 -> 361 us, with partial sums 640 -> 566 us
+// (issue slots 46 %, FP64 pipe 31 %, tensor pipe 20 %, HBM 25-50 %).  What
+// mattered: the ring; one kernel per form of sweep with a short straight
+// epilogue loop (no spills, 50 KB: 436 -> 325 us for the MagicFilter sweep alone);
+// digits as FP16 subnormals; polls and shared-memory stores in few instructions.
+// Measured and slower: three epilogue groups and an issuer warp on 24 warps (80
+// registers: 1.58 ms against 1.52 for MagicFilter3D), TMEM loads one step ahead,
+// global loads two slabs ahead (kinetic 1.60 -> 1.65 ms), larger unrolled loops.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "lcg_sweep.cuh"
 #include "lcg_tc.cuh"
@@ -72,22 +94,27 @@
 namespace lcg {
 namespace tck {
 
-constexpr int kM = 128;          // lines per tile (MMA M)
-constexpr int kQE = 64;          // output elements per tile
-constexpr int kNB = kQE / 16;    // 16-element output blocks per tile
+constexpr int kM = 128;          // lines per strip (MMA M)
+constexpr int kSlots = 6;        // slabs in the operand ring
 constexpr int kThreads = 512;    // 8 producer warps + 8 epilogue warps
-constexpr int kProducers = 256;
-constexpr long long kWaitCycles = 4000000000LL;
+constexpr int kProdWarps = 8, kEpiWarps = 8;
+static_assert(kEpiWarps == kTcDotSlots, "dot partials per CTA");
+constexpr uint32_t kWaitSleep = 64;                  // ns
+constexpr uint32_t kWaitPolls = 1u << 26;            // polls of a wait: seconds at the least rate seen
+
+// Forms of a sweep, one kernel each, so that the epilogue of the common ones is
+// a short loop (code and registers): plain stores; plus a partial sum x2; plus
+// the next sweep's line exponents; anything (dot products, a_x, a_y).
+enum Form { FORM_PLAIN = 0, FORM_X2 = 1, FORM_HAND = 2, FORM_ANY = 3 };
 
 template <int KIND, int NT, int SCH> struct Geom {
     static constexpr int NCH = KIND == KCONV ? 1 : 2;            // elements per position
     static constexpr int PROD = NCH * NT;                        // products per output
     static constexpr int KB = ((NCH * (16 / NCH + NT - 1)) + 15) / 16 * 16;   // K per block
-    static constexpr int KT = 16 * (kNB - 1) + KB;               // input elements per tile
-    static constexpr int QP = kQE / NCH;                         // output positions per tile
+    static constexpr int W = KB / 16;                            // slabs a block reads
+    static constexpr int PB = 16 / NCH;                          // positions per block or slab
     static constexpr int ESZ = SCH == SCH_TF32X3 ? 4 : 2;         // operand element bytes
     static constexpr int CE = 16 / ESZ;                          // elements per core-matrix row
-    static constexpr int MK = 32 / ESZ;                          // K of one MMA
     static constexpr int ND = SCH == SCH_EXACT ? 8 : SCH == SCH_BF16X3 ? 3 : 2;
     static constexpr int ORD = ND;                               // order accumulators per block
     // operand planes interleaved along K: the exact scheme keeps its digit
@@ -98,21 +125,26 @@ template <int KIND, int NT, int SCH> struct Geom {
     static constexpr int NS = ND / PL;                           // A slices (MMAs per K step)
     static constexpr int BN = 16 * ORD;                          // rows of the stacked filter
     static constexpr int LBO_B = BN * 16;                        // its K-direction chunk stride
-    static constexpr int A_SLICE = kM * KT * PL * ESZ;
-    static constexpr int A_BYTES = NS * A_SLICE;
+    // a slab: NS slices of CH core-matrix columns (kM rows x 16 bytes each)
+    static constexpr int CH = 16 * PL / CE;
+    static constexpr int SLICE = CH * kM * 16;
+    static constexpr int SLAB = NS * SLICE;
+    static constexpr int KS = CH / 2;                            // MMA K steps per slab and slice
+    static constexpr int A_BYTES = kSlots * SLAB;
     static constexpr int KBP = KB * PL;                          // K of a block window
     static constexpr int B_BYTES = BN * KBP * ESZ;
-    // exact scheme: a 128 x 16 FP16 tile holding 2048 at K = 0, 1, 2 of every
-    // row; as both operands of an N = 128 MMA it sets an output block's eight
-    // order accumulators to 3 * 2048^2 = 1.5 * 2^23
+    // exact scheme: a 128 x 16 FP16 tile holding 8 at K = 0, 1, 2 of every row;
+    // as both operands of an N = 128 MMA it sets an output block's eight order
+    // accumulators to 3 * 8^2 = 192 = 1.5 * 2^23 units of 2^-16
     static constexpr int Z_BYTES = SCH == SCH_EXACT ? kM * 16 * 2 : 0;
-    static constexpr int AUX = 1024 + 3 * 4 * kM + 2 * 4 * 32 * 4;   // barriers, slots, row exponents,
-                                                                 // next-sweep column maxima
+    // barriers and TMEM address; row exponents of the last 8 strips
+    static constexpr int AUX = 256 + 8 * kM * 2;
     static constexpr int SMEM = A_BYTES + B_BYTES + Z_BYTES + AUX + 1024;
-    static constexpr int HALF_COLS = 2 * ORD * 16;               // one TMEM half (2 blocks)
-    static constexpr uint32_t TMEM_COLS = 2 * HALF_COLS <= 32 ? 32 : 2 * HALF_COLS <= 64 ? 64 : 2 * HALF_COLS <= 128 ? 128 : 2 * HALF_COLS <= 256 ? 256 : 512;
-    static_assert(2 * HALF_COLS <= 512, "TMEM columns");
-    static_assert(ND % PL == 0, "plane slices");
+    static constexpr int SLOT_COLS = ORD * 16;                   // one TMEM slot (a block)
+    static constexpr uint32_t TMEM_COLS = 4 * SLOT_COLS <= 128 ? 128 : 4 * SLOT_COLS <= 256 ? 256 : 512;
+    static_assert(4 * SLOT_COLS <= 512, "TMEM columns");
+    static_assert(W >= 2 && W < kSlots, "slab ring");
+    static_assert(ND % PL == 0 && CH % 2 == 0, "plane slices");
     static_assert(SMEM <= 232448, "shared memory");
     // Instruction descriptor (kind::f16 / kind::tf32): D F32; A and B F16
     // (exact), BF16 or TF32 (formats 0, 1, 2); both K-major; M = 128; N is
@@ -168,34 +200,43 @@ __device__ __forceinline__ void bar_arrive(uint32_t bar) {
         : "memory");
 }
 
-__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ void bar_arrive_n(uint32_t bar, uint32_t n) {
+    asm volatile(
+        "{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0], %1;\n\t}\n" ::"r"(bar), "r"(n)
+        : "memory");
+}
+
+// Bounded wait for the phase of the given parity; false after kWaitPolls polls.
+// The loop is a few instructions: a waiting warp's polls come out of the working
+// warps' issue slots.
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n"
+        "WAIT_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE_%=;\n\t"
+        "nanosleep.u32 %4;\n\tsub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra WAIT_%=;\n"
+        "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "n"(kWaitPolls), "n"(kWaitSleep)
         : "memory");
     return ok != 0;
 }
 
-// Bounded wait for the phase of the given parity; false after ~2 s.  Between
-// polls the warp sleeps briefly so waiting warps leave the issue slots to the
-// working ones.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-    if (bar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!bar_try(bar, parity)) {
-        __nanosleep(128);
-        if (clock64() - t0 > kWaitCycles) return false;
-    }
-    return true;
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
                    "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr)
                  : "memory");
 }
@@ -218,70 +259,42 @@ __device__ __forceinline__ int imod(int a, int n) {
     return r < 0 ? r + n : r;
 }
 
-// Y * 2^se as an FP64, Y rounded to 53 bits to nearest-even (the rounding of
-// an int64 -> FP64 conversion), for any se; ldexp when the result is not a
-// normal number.
-__device__ __forceinline__ double ll_scaled(long long Y, int se) {
-    if (Y == 0) return 0.0;
-    const unsigned long long sg = (unsigned long long)Y & 0x8000000000000000ull;
-    unsigned long long a = Y < 0 ? 0ull - (unsigned long long)Y : (unsigned long long)Y;
-    int e = 63 - __clzll((long long)a);                         // a in [2^e, 2^(e+1))
-    if (e <= 52) {
-        a <<= (52 - e);
-    } else {
-        const int sh = e - 52;                                  // 1..10
-        const unsigned long long rem = a & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-        a >>= sh;
-        if (rem > half || (rem == half && (a & 1ull))) ++a;
-        if (a >> 53) { a >>= 1; ++e; }
-    }
-    const int be = e + 1023 + se;
-    const unsigned long long m = a & 0xFFFFFFFFFFFFFull;
-    if (be >= 1 && be <= 2046)
-        return __longlong_as_double((long long)(sg | ((unsigned long long)be << 52) | m));
-    return ldexp(__longlong_as_double((long long)(sg | (1075ull << 52) | m)), e - 52 + se);
-}
-
-// The same value with one conversion instruction when every non-zero result is
-// a normal number (-1022 <= se <= 961): the conversion rounds to nearest-even,
-// and se is added to its exponent field.  On this GPU the FP64 pipe takes 2
-// lanes a clock per SM and the integer pipes 64 each, so one FP64 instruction
-// per output (4.1 K cycles of a tile's ~20 K) costs less than the ~27 integer
-// instructions of the same normalisation, and a second one (a multiply by
-// 2^se) already sets the pace: MagicFilter3D on 32 x 128^3 1.87 ms all integer,
-// 1.80 with conversion and multiply, 1.56 with the conversion alone.
+// Y * 2^se as an FP64, Y rounded to 53 bits to nearest-even, when every non-zero
+// result is a normal number (-1022 <= se <= 961): one conversion instruction,
+// and se added to its exponent field.  On this GPU the FP64 pipe takes 2 lanes a
+// clock per SM and the integer pipes 64 each, so one FP64 instruction per output
+// (1.0 K of a block's 3.1 K cycles) costs less than the ~27 integer instructions
+// of the same normalisation, and a second one (a multiply by 2^se) already sets
+// the pace: MagicFilter3D on 32 x 128^3 1.87 ms all integer, 1.80 with conversion
+// and multiply, 1.56 with the conversion alone (64-output tiles).
 __device__ __forceinline__ double ll_scaled_fast(long long Y, int se) {
     const double t = __ll2double_rn(Y);
-    const int hi = __double2hiint(t);
-    return __hiloint2double(hi ? hi + (se << 20) : 0, __double2loint(t));
+    int hi = __double2hiint(t);
+    if (hi) hi += se << 20;
+    return __hiloint2double(hi, __double2loint(t));
 }
 
-// Y = sum_k Acc_k 2^(46 - 8k) over the 8 order accumulators of one output,
-// from their biased bits b_k = Acc_k + 0x4B400000 (the bits of an FP32
-// accumulator that started at 1.5 * 2^23, |Acc_k| <= 2^22), orders 6-7 as the
-// nearest integer of Acc_6 / 4 + Acc_7 / 1024.  Two neighbouring orders fit one
-// 32-bit word: w = 256 b_k + b_{k+1} = 257 * 0x4B400000 + (256 Acc_k +
-// Acc_{k+1}) modulo 2^32 stays within [0x4B000000, 0xCB800000], so it can be
-// taken as unsigned and the pair's bias removed by one constant for the whole
-// sum.  One multiply-add per pair and two 32x32+64 ones to join them, which run
-// on the multiply-add pipe beside the producers' ALU work.  The wrap-around is
-// exact because the true sum fits in 62 bits.
+// Y = sum_k Acc_k 2^(46 - 8k) over the 8 order accumulators of one output
+// (channel c of the filter), orders 6-7 as the nearest integer of Acc_6 / 4 +
+// Acc_7 / 1024, from the accumulators' bits b_k = kAccBias + Acc_k + C_k (C_k:
+// the digits' offset of 128, tc_filter_digits).  Two neighbouring orders fit
+// one 32-bit word: w = 256 b_k + b_{k+1} modulo 2^32 stays within [0x43000000,
+// 0xC3800000], so it can be taken as unsigned, and biases and offsets of all
+// orders leave by two constants (F.k64, F.k67).  One multiply-add per pair and
+// three 32x32+64 ones to join them, with multipliers the compiler cannot turn
+// into shifts (F.c...): they run on the multiply-add pipe, beside the
+// producers' ALU work.  The wrap-around is exact because the true sum fits in
+// 62 bits.
 template <int ORD>
-__device__ __forceinline__ long long horner_bal(const uint32_t (&b)[ORD]) {
+__device__ __forceinline__ long long horner_bal(const uint32_t (&b)[ORD], const TcFilter &F, int c) {
     static_assert(ORD == 8, "eight order accumulators");
-    constexpr uint32_t kPair = 257u * 0x4B400000u;              // bias of a pair, modulo 2^32
-    constexpr unsigned long long kBias =
-        (unsigned long long)kPair * ((1ull << 38) + (1ull << 22) + (1ull << 6));
-    // the low word of -kBias joins lo: 0 < lo + kLo < 2^32 (|lo| <= 2^20 + 1)
-    constexpr uint32_t kLo = (uint32_t)(0ull - kBias), kHi = (uint32_t)((0ull - kBias) >> 32);
-    static_assert(kLo > (1u << 21) && kLo < 0xFFE00000u, "no carry out of the low word");
-    const uint32_t w01 = b[0] * 256u + b[1], w23 = b[2] * 256u + b[3], w45 = b[4] * 256u + b[5];
-    const int lo = (int)(b[6] * 256u + b[7] + (512u - kPair)) >> 10;
-    unsigned long long v = ((unsigned long long)kHi << 32) | (kLo + (uint32_t)lo);
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(w45), "r"(64u), "l"(v));
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(w23), "r"(4194304u), "l"(v));
-    v += (unsigned long long)(w01 * 64u) << 32;
-    return (long long)v;
+    const uint32_t w01 = b[0] * F.c256 + b[1], w23 = b[2] * F.c256 + b[3], w45 = b[4] * F.c256 + b[5];
+    const int lo = (int)(b[6] * F.c256 + b[7] + F.k67[c]) >> 10;
+    long long v;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(v) : "r"(w45), "r"(F.c64), "l"(F.k64[c]));
+    asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(v) : "r"(w23), "r"(F.c22));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(v) : "r"(lo), "r"(F.c1));
+    return v + (long long)((unsigned long long)(w01 * F.c64) << 32);
 }
 
 // FP32 bits -> FP64 value, integer only (normal, zero, subnormal flushed, inf/nan).
@@ -312,19 +325,37 @@ __device__ __forceinline__ void fixed_bal(long long bits, int mx, uint32_t &ul, 
     uh = (uint32_t)(U >> 32);
 }
 
-// FP16 pair of balanced digits 2p, 2p+1 (bytes 7-2p and 6-2p) of one biased
-// fixed point (ul/uh): PRMT takes the two bytes with a 0x64 byte above each,
-// which makes them 1024 + byte in FP16, and one HADD2 subtracts 1024 + 128
-// (exact).  The lower half is plane 2p (the more significant digit).
+// The same for a row whose largest exponent field mx is at least 64, with mxs =
+// (mx + 1) << 20: a zero or subnormal element then lies below one unit, and its
+// shift of mx + 1 > 64 gives 0 whatever the mantissa's leading bit, so neither
+// it nor the shift needs a special case.  c10 = 1024 (a multiplier the compiler
+// cannot turn into shifts: the multiply-add pipe has room, the ALU pipe has not).
+__device__ __forceinline__ void fixed_fast(long long bits, uint32_t mxs, uint32_t c10, uint32_t &ul, uint32_t &uh) {
+    const uint32_t lo = (uint32_t)bits, hi = (uint32_t)((unsigned long long)bits >> 32);
+    const uint32_t c = (mxs - (hi & 0x7FF00000u)) >> 20;        // mx + 1 - ex
+    const uint32_t mh = (hi & 0xFFFFFu) | 0x100000u;
+    unsigned long long m = (unsigned long long)lo * c10;
+    m += (unsigned long long)(mh * c10) << 32;
+    asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(c));              // 0 for c > 63
+    const uint32_t sg = (uint32_t)((int)hi >> 31);              // 0 or all ones
+    // (m ^ sg) - sg + 0x8080808080808080
+    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, %5;"
+        : "=r"(ul), "=r"(uh)
+        : "r"((uint32_t)m ^ sg), "r"(0x80808080u | (sg & 1u)), "r"((uint32_t)(m >> 32) ^ sg), "r"(0x80808080u));
+}
+
+// FP16 pair of digits 2p, 2p+1 (bytes 7-2p and 6-2p) of one biased fixed point
+// (ul/uh): PRMT takes the two bytes with a zero byte above each.  As FP16 bits
+// a byte u is the subnormal u 2^-24, exact; the operand is the balanced digit
+// plus 128, and the 128 leaves with the accumulators' bias (horner_bal).  The
+// lower half is plane 2p (the more significant digit).
 __device__ __forceinline__ uint32_t digit_pair_elem(int p, uint32_t ul, uint32_t uh) {
     const uint32_t w = p < 2 ? uh : ul;
-    // bytes (3, 2) of the word for even p, (1, 0) for odd p; selector 4 = 0x64
+    // bytes (3, 2) of the word for even p, (1, 0) for odd p; selector 4 = 0
     const uint32_t sel = (p & 1) ? 0x4041u : 0x4243u;
     uint32_t t;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(w), "r"(0x64646464u), "r"(sel));
-    const uint32_t off = 0xE480E480u;                            // (-1152, -1152) in FP16
-    __half2 h = __hadd2(*reinterpret_cast<__half2 *>(&t), *reinterpret_cast<const __half2 *>(&off));
-    return *reinterpret_cast<uint32_t *>(&h);
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(w), "r"(0u), "r"(sel));
+    return t;
 }
 
 // FP64 bit pattern -> FP32 bit pattern, rounded to nearest (ties away) on the
@@ -356,41 +387,36 @@ __device__ __forceinline__ void split_f32(uint32_t f, uint32_t (&h)[SPLITS]) {
     }
 }
 
-// Issue the MMAs of one TMEM half (output blocks 2h, 2h+1) of a tile.  The
-// filter planes t = 0..ORD-1 are stacked along N in one matrix (rows 16t + n),
-// and the ORD accumulators of a block (order k = s + t at columns 16k) are
-// contiguous in TMEM, so ONE MMA per data plane s covers all its pairs:
-// D = columns 16s.. of the block, N = 16 (ORD - s) (a prefix of the stacked
-// filter), giving pair (s, t) at order s + t.  The s = 0 MMA of the first K
-// step initialises every order (split schemes); in the exact scheme one MMA of
-// the constant tile (z_desc, N = 128) first sets all eight orders of the block
-// to 1.5 * 2^23 and every data MMA accumulates.  Output block j starts 16
-// elements into the A planes; one MMA covers 32 bytes of K (two core
-// matrices).  Descriptors are advanced by adding the (16-byte unit) offset to
-// the start-address field (addresses < 256 KB never carry out of it).
-template <int KIND, int NT, int SCH, int H>
-__device__ __forceinline__ void issue_half(uint32_t tmem, uint64_t a_desc0, uint64_t b_desc0,
-                                           uint64_t z_desc) {
+// Issue the MMAs of one output block.  The filter planes t = 0..ORD-1 are
+// stacked along N in one matrix (rows 16t + n), and the ORD accumulators of the
+// block (order k = s + t at columns 16k of its TMEM slot) are contiguous, so
+// ONE MMA per data plane s covers all its pairs at once: D = columns 16s.. of
+// the slot, N = 16 (ORD - s) (a prefix of the stacked filter), giving pair
+// (s, t) at order s + t.  The s = 0 MMA of the first K step initialises every
+// order (split schemes); in the exact scheme one MMA of the constant tile
+// (z_desc, N = 128) first sets all eight orders to 1.5 * 2^23 and every data
+// MMA accumulates.  One MMA covers 32 bytes of K (two core matrices); a[w] is
+// the descriptor of the window's slab w.  Descriptors are advanced by adding
+// the (16-byte unit) offset to the start-address field (addresses < 256 KB
+// never carry out of it).
+template <int KIND, int NT, int SCH>
+__device__ __forceinline__ void issue_block(uint32_t d0, const uint64_t (&a)[Geom<KIND, NT, SCH>::W],
+                                            uint64_t b_desc0, uint64_t z_desc) {
     using G = Geom<KIND, NT, SCH>;
     constexpr bool TF = SCH == SCH_TF32X3;
     constexpr bool EX = SCH == SCH_EXACT;
-    constexpr int NKS = G::KBP / G::MK;
+    if (EX) mma<false>(d0, z_desc, z_desc, G::idesc(16 * G::ORD), 0u);
 #pragma unroll
-    for (int jj = 0; jj < 2; ++jj) {
-        const int j = 2 * H + jj;
-        const int a_blk = (16 * G::PL / G::CE) * j * 2048;
-        if (EX) mma<false>(tmem + (uint32_t)(H * G::HALF_COLS + jj * G::ORD * 16), z_desc, z_desc,
-                           G::idesc(16 * G::ORD), 0u);
+    for (int sl = 0; sl < G::NS; ++sl) {
+        const int sd = sl * G::PL;                               // first plane (order) of the slice
+        const uint32_t id = G::idesc(16 * (G::ORD - sd));
 #pragma unroll
-        for (int sl = 0; sl < G::NS; ++sl) {
-            const int sd = sl * G::PL;                           // first plane (order) of the slice
-            const uint32_t d = tmem + (uint32_t)(H * G::HALF_COLS + (jj * G::ORD + sd) * 16);
-            const uint32_t id = G::idesc(16 * (G::ORD - sd));
+        for (int w = 0; w < G::W; ++w) {
 #pragma unroll
-            for (int ks = 0; ks < NKS; ++ks) {
-                const uint64_t ad = a_desc0 + (uint64_t)((sl * G::A_SLICE + a_blk + 2 * ks * 2048) >> 4);
-                const uint64_t bd = b_desc0 + (uint64_t)((2 * ks * G::LBO_B) >> 4);
-                mma<TF>(d, ad, bd, id, (EX || sl > 0 || ks > 0) ? 1u : 0u);
+            for (int ks = 0; ks < G::KS; ++ks) {
+                const uint64_t ad = a[w] + (uint64_t)((sl * G::SLICE + 2 * ks * 2048) >> 4);
+                const uint64_t bd = b_desc0 + (uint64_t)((2 * (w * G::KS + ks) * G::LBO_B) >> 4);
+                mma<TF>(d0 + (uint32_t)(sd * 16), ad, bd, id, (EX || sl > 0 || w > 0 || ks > 0) ? 1u : 0u);
             }
         }
     }
@@ -410,37 +436,43 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, uint32_t m, uint32_t s) {
     return (uint32_t)(((unsigned long long)n * m) >> s);
 }
 
-// Where tile `tile` of a launch lives: its sweep, its output chunk `ch`
-// along the lines, its block of kM lines `lb` and its array.  Tiles are
-// numbered chunk fastest, then line block, then array.  A batched launch
-// (BATCH) covers a list of sweeps of the same kind and filter, one per grid
-// of a batch of uneven grids, whose tiles are numbered consecutively
-// (prefix[i] = first tile of sweep i).
-struct TileLoc {
+// Where strip `strip` of a launch lives: its sweep, its segment `seg` along the
+// lines, its block of kM lines `lb` and its array.  Strips are numbered
+// segment fastest, then line block, then array.  A batched launch (BATCH)
+// covers a list of sweeps of the same kind and filter, one per grid of a
+// batch of uneven grids, whose strips are numbered consecutively (prefix[i] =
+// first strip of sweep i).
+struct StripLoc {
     const Sweep *S;
-    int ch;
+    int seg;
     uint32_t lb;
     int arr;
 };
 
 template <bool BATCH>
-__device__ __forceinline__ TileLoc locate(const Sweep &S0, const Sweep *descs,
-                                          const long long *prefix, int nsweeps, long long tile) {
+__device__ __forceinline__ StripLoc locate(const Sweep &S0, const Sweep *descs,
+                                           const long long *prefix, int nsweeps, long long strip) {
     const Sweep *S = &S0;
-    uint32_t t = (uint32_t)tile;
+    uint32_t t = (uint32_t)strip;
     if (BATCH) {
-        int lo = 0, hi = nsweeps - 1;                    // last i with prefix[i] <= tile
+        int lo = 0, hi = nsweeps - 1;                    // last i with prefix[i] <= strip
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (prefix[mid] <= tile) lo = mid;
+            if (prefix[mid] <= strip) lo = mid;
             else hi = mid - 1;
         }
         S = descs + lo;
-        t = (uint32_t)(tile - prefix[lo]);
+        t = (uint32_t)(strip - prefix[lo]);
     }
-    const uint32_t q = fdiv(t, S->tdiv_m[0], S->tdiv_s[0]);          // t / chunks
+    const uint32_t q = fdiv(t, S->tdiv_m[0], S->tdiv_s[0]);          // t / segments
     const uint32_t arr = fdiv(q, S->tdiv_m[1], S->tdiv_s[1]);        // / line blocks
     return {S, (int)(t - q * S->tdiv_d[0]), q - arr * S->tdiv_d[1], (int)arr};
+}
+
+// Output blocks of segment `seg` of a sweep (PB positions each).
+template <int PB>
+__device__ __forceinline__ int strip_blocks(const Sweep &S, int seg) {
+    return min(S.seg_blocks, (S.qhi - S.qlo + PB) / PB - seg * S.seg_blocks);
 }
 
 // Line g of a sweep as (l, r): g = l + nL r.
@@ -449,41 +481,40 @@ __device__ __forceinline__ void line_lr(const Sweep &S, uint32_t g, uint32_t &l,
     l = g - r * S.tdiv_d[2];
 }
 
-template <int KIND, int NT, int SCH, bool BATCH>
+template <int KIND, int NT, int SCH, bool BATCH, int FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilter F, int *status,
                 const Sweep *__restrict__ descs, const long long *__restrict__ prefix, int nsweeps,
                 const int *__restrict__ lineE) {
     using G = Geom<KIND, NT, SCH>;
-    constexpr int NCH = G::NCH;
+    constexpr int NCH = G::NCH, W = G::W, PB = G::PB;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *A = smem;
     uint8_t *B = smem + G::A_BYTES;
     uint8_t *Z = B + G::B_BYTES;                      // exact scheme: accumulator bias tile
     uint8_t *aux = Z + G::Z_BYTES;
-    uint64_t *bars = (uint64_t *)aux;                 // 9 barriers (16 slots)
-    uint32_t *tslot = (uint32_t *)(aux + 128);
-    int *rowE3 = (int *)(aux + 1024);                 // row exponents, by tile index mod 3
-    int *colE = (int *)(aux + 1024 + 3 * 4 * kM);     // [group][warp][column]: next-sweep line maxima
-    // pfull[p]: chunk pair p of the tile is written (producer arrivals);
-    // pfree0: pair 0 may be rewritten (the MMAs of TMEM half 0 completed);
-    // pfree12: pairs 1 and 2 may be rewritten (both halves' MMAs completed:
-    //          one commit from each issuer);
-    // bT_full[h]: TMEM half h holds the tile's accumulators;
-    // gsync[h]: the 4 warps of epilogue group h have drained TMEM half h.
-    const uint32_t pfull[3] = {saddr(&bars[0]), saddr(&bars[1]), saddr(&bars[2])};
-    const uint32_t pfree0 = saddr(&bars[3]), pfree12 = saddr(&bars[4]);
-    const uint32_t bT_full[2] = {saddr(&bars[5]), saddr(&bars[6])};
-    const uint32_t gsync[2] = {saddr(&bars[7]), saddr(&bars[8])};
+    uint32_t *tslot = (uint32_t *)(aux + 192);
+    short *rowE8 = (short *)(aux + 256);              // row exponents, by strip mod 8
+    const uint32_t bar0 = saddr(aux);
+    auto full = [&](uint32_t s) { return bar0 + 8 * s; };
+    auto empty = [&](uint32_t s) { return bar0 + 8 * (kSlots + s); };
+    auto tfull = [&](uint32_t s) { return bar0 + 8 * (2 * kSlots + s); };
+    auto drained = [&](uint32_t s) { return bar0 + 8 * (2 * kSlots + 4 + s); };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long ntiles = BATCH ? prefix[nsweeps]
-                                   : ((long long)S0.nL * S0.nR + kM - 1) / kM *
-                                         ((S0.qhi - S0.qlo + G::QP) / G::QP) * S0.narr;
+    const long long nstrips =
+        BATCH ? prefix[nsweeps]
+              : ((long long)S0.nL * S0.nR + kM - 1) / kM * (long long)S0.tdiv_d[0] * S0.narr;
     // window offset of the convolution sweeps (0 in batched launches)
     const int woff = (!BATCH && KIND == KCONV) ? S0.woff : 0;
-    const int kneed = NCH * (G::QP + NT - 1) + woff;  // window elements the tile's outputs use
+    // the strip after `strip` for this CTA, skipping inactive arrays
+    auto skip_inactive = [&](long long strip) -> long long {
+        if (!BATCH && S0.active)
+            while (strip < nstrips && !S0.active[locate<BATCH>(S0, descs, prefix, nsweeps, strip).arr])
+                strip += gridDim.x;
+        return strip;
+    };
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
@@ -493,12 +524,13 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        for (int p = 0; p < 3; ++p) bar_init(pfull[p], kProducers);
-        bar_init(pfree0, 1);
-        bar_init(pfree12, 2);
-        for (int h = 0; h < 2; ++h) {
-            bar_init(bT_full[h], 1);
-            bar_init(gsync[h], 128);
+        for (int s = 0; s < kSlots; ++s) {
+            bar_init(full(s), kProdWarps);
+            bar_init(empty(s), W);                    // one arrival per block of a window
+        }
+        for (int s = 0; s < 4; ++s) {
+            bar_init(tfull(s), 2);                    // the issuer's commit and its own arrival
+            bar_init(drained(s), kEpiWarps / 2);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -519,10 +551,10 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
         else *(unsigned short *)b = (unsigned short)v;
     }
     // bias tile, K-major core matrices like A: (row, k) at (k / 8) * 2048 +
-    // (row / 8) * 128 + (row % 8) * 16 + (k % 8) * 2; FP16 2048 = 0x6800
+    // (row / 8) * 128 + (row % 8) * 16 + (k % 8) * 2; FP16 8 = 0x4800
     for (int idx = tid; idx < G::Z_BYTES / 2; idx += kThreads) {
         const int k8 = idx / 1024, rem = idx % 1024, k = rem % 8;
-        ((unsigned short *)Z)[idx] = (k8 == 0 && k < 3) ? (unsigned short)0x6800 : (unsigned short)0;
+        ((unsigned short *)Z)[idx] = (k8 == 0 && k < 3) ? (unsigned short)0x4800 : (unsigned short)0;
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -531,324 +563,314 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
     const uint32_t tmem = *tslot;
     bool alive = true;
 
-    const uint64_t a_desc0 = umma_desc(saddr(A), 2048, 128);
-    const uint64_t b_desc0 = umma_desc(saddr(B), G::LBO_B, 128);
-    const uint64_t z_desc = umma_desc(saddr(Z), 2048, 128);
-    if (warp < kProducers / 32) {
-        // ============ producers: thread = (row, half of every chunk pair);
-        // half-warps cover 16 consecutive rows.  The KT elements of a row are
-        // 8-element groups in three chunk pairs (elements [0, 32), [32, 64),
-        // [64, KT)); lanes 0-15 take the first half of every pair's groups,
-        // lanes 16-31 the second half, and both write the pairs in order, so
-        // pair 0 of the next tile (read only by the MMAs of TMEM half 0) is
-        // written while the MMAs of half 1 still read pairs 1 and 2.
-        constexpr int NG = G::KT / 8;                                 // 10 or 12 groups
-        constexpr int NGH = NG / 2;                                   // groups per thread
-        constexpr int G2 = (NG - 8) / 2;                              // per thread in pair 2
-        static_assert(NG == 10 || NG == 12, "three chunk pairs");
+    if (warp < kProdWarps) {
+        // ============ producers: thread = (row, half of every slab); lanes 0-15
+        // take 16 consecutive rows' elements 0-7, lanes 16-31 elements 8-15
+        constexpr int PG = 8 / NCH;                      // positions of a thread's group
         const int half = lane >> 4;
         const int row = warp * 16 + (lane & 15);
-        auto group_of = [&](int c) -> int {          // c-th group of this thread
-            return c < 2 ? 2 * half + c : c < 4 ? 4 + 2 * half + (c - 2) : 8 + G2 * half + (c - 4);
-        };
-        uint32_t it = 0;                                  // tiles processed (inactive arrays skipped)
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const TileLoc loc = locate<BATCH>(S0, descs, prefix, nsweeps, tile);
-            if (!BATCH && S0.active && !S0.active[loc.arr]) continue;
-            const Sweep &S = *loc.S;
-            const uint32_t nlines = (uint32_t)S.nL * (uint32_t)S.nR;
-            const int plast = S.qhi + S.lowfil + NT - 1;                // last input position used
-            const long long in_ext = S.in_ext;
-            const int p0 = S.qlo + loc.ch * G::QP + S.lowfil - woff;    // window start position
-            const int pstart = S.bc == BC_PERIODIC ? imod(p0, S.n) : 0;
-            const bool onewrap = S.n >= G::KT;
-            // element kk of the tile -> offset (in elements) in the line, -1 for a zero
-            auto off_of = [&](int kk) -> long long {
-                const int pp = kk / NCH, c = kk % NCH;
-                const int p = p0 + pp;
-                if (kk >= kneed || p > plast) return -1;
-                int ps;
-                if (S.bc == BC_PERIODIC) {
-                    if (onewrap) { const int q = pstart + pp; ps = q >= S.n ? q - S.n : q; }
-                    else ps = imod(p, S.n);
-                } else if (S.bc == BC_SHRINK) {
-                    ps = p - S.in_lo;
-                } else {
-                    if (p < 0 || p >= S.n) return -1;
-                    ps = p;
-                }
-                return KIND == KCONV ? ps : KIND == KDEC ? (long long)c + 2LL * ps : ps + in_ext * c;
-            };
-            const uint32_t g = loc.lb * kM + row;
-            const bool valid = g < nlines;
-            uint32_t l = 0, r = 0;
-            if (valid) line_lr(S, g, l, r);
-            const long long *base = reinterpret_cast<const long long *>(S.x) + (long long)loc.arr * S.x_arr +
-                                    l + (long long)S.nL * (in_ext * NCH) * r;
-            const long long stride = S.nL;
-            const int klim = min(kneed, NCH * (plast - p0 + 1));
-            // the 8 elements of group gi.  The group's first cnt elements are
-            // used (the same for every row of the tile).  Periodic
-            // convolution lines (the common case) take their positions as at
-            // most two runs (before and after the wrap): contiguous lines by
-            // 32- or 16-byte vectors when the group is one aligned run,
-            // strided lines by one pointer stepping the stride.  Other
-            // boundaries: one pointer when the group's line offsets are one
-            // consecutive run, else element by element.
-            auto load8 = [&](int gi, long long (&bits)[8]) {
-                const int i0 = gi * 8;
-                const int cnt = max(0, min(8, klim - i0));
-#pragma unroll
-                for (int e = 0; e < 8; ++e) bits[e] = 0ll;
-                if (cnt <= 0 || !valid) return;
-                if (KIND == KCONV && S.bc == BC_PERIODIC && onewrap) {
-                    int ps0 = pstart + i0;                           // < 2n
-                    if (ps0 >= S.n) ps0 -= S.n;
-                    const int w = S.n - ps0;                         // elements before the wrap
-                    if (stride == 1) {
-                        const long long *q = base + ps0;
-                        if (cnt == 8 && w >= 8) {
-                            if ((((uintptr_t)q) & 31) == 0) {
-                                ld256(q, bits[0], bits[1], bits[2], bits[3]);
-                                ld256(q + 4, bits[4], bits[5], bits[6], bits[7]);
-                                return;
-                            }
-                            if ((((uintptr_t)q) & 15) == 0) {
-                                const double2 *v = reinterpret_cast<const double2 *>(q);
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const double2 t = v[e];
-                                    bits[2 * e] = __double_as_longlong(t.x);
-                                    bits[2 * e + 1] = __double_as_longlong(t.y);
-                                }
-                                return;
-                            }
-                        }
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (e < cnt) bits[e] = e < w ? q[e] : base[e - w];
-                    } else {
-                        const long long *q = base + (long long)ps0 * stride;
-                        if (cnt == 8 && w >= 8) {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) {
-                                bits[e] = *q;
-                                q += stride;
-                            }
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) {
-                                if (e == w) q = base;
-                                if (e < cnt) bits[e] = *q;
-                                q += stride;
-                            }
-                        }
-                    }
-                    return;
-                }
-                if (KIND == KREC && S.bc == BC_PERIODIC && S.n * NCH >= G::KT) {
-                    // synthesis input: 4 positions x 2 channels, channel c of
-                    // position ps at ps + in_ext c: two runs of 4, read as
-                    // vectors on contiguous lines, interleaved into the group
-                    int ps0 = pstart + i0 / 2;                       // < 2n
-                    if (ps0 >= S.n) ps0 -= S.n;
-                    const int np = cnt / 2, w = S.n - ps0;           // positions, before the wrap
-                    const long long *qL = base + (long long)ps0 * stride, *qH = qL + in_ext * stride;
-                    if (np == 4 && w >= 4) {
-                        if (stride == 1 && ((((uintptr_t)qL) | ((uintptr_t)qH)) & 31) == 0) {
-                            ld256(qL, bits[0], bits[2], bits[4], bits[6]);
-                            ld256(qH, bits[1], bits[3], bits[5], bits[7]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                bits[2 * j] = qL[j * stride];
-                                bits[2 * j + 1] = qH[j * stride];
-                            }
-                        }
+        const uint32_t a_addr = saddr(A);
+        // the strip being loaded: the row's line, and the thread's next group of 8
+        // elements: its position in the line and the used positions left
+        const Sweep *S = &S0;
+        const long long *base = nullptr;
+        long long stride = 0;
+        int ps = 0, left = 0, nsl = 0;
+        int wrap = 0, last = 0;                          // ps wraps at; runs end by `last`
+        int mx = 0;                                      // largest exponent field of the row
+        // the group's elements; those past the used positions, and outside a free
+        // boundary's line, are zero
+        auto load8 = [&](long long (&bits)[8]) {
+            if (left >= PG && ps >= 0 && ps + PG <= last) {      // one run of positions
+                if (KIND == KREC) {
+                    // channel c of position ps at ps + in_ext c: two runs of 4,
+                    // interleaved into the group
+                    const long long *qL = base + (long long)ps * stride;
+                    const long long *qH = qL + (long long)S->in_ext * stride;
+                    if (stride == 1 && ((((uintptr_t)qL) | ((uintptr_t)qH)) & 31) == 0) {
+                        ld256(qL, bits[0], bits[2], bits[4], bits[6]);
+                        ld256(qH, bits[1], bits[3], bits[5], bits[7]);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            if (j >= np) break;
-                            int ps = ps0 + j;
-                            if (ps >= S.n) ps -= S.n;
-                            bits[2 * j] = base[(long long)ps * stride];
-                            bits[2 * j + 1] = base[((long long)ps + in_ext) * stride];
+                            bits[2 * j] = qL[j * stride];
+                            bits[2 * j + 1] = qH[j * stride];
                         }
                     }
-                    return;
-                }
-                long long oa = -1;
-                if (KIND != KREC) {
-                    const long long a0 = off_of(i0);
-                    if (a0 >= 0 && off_of(i0 + cnt - 1) == a0 + cnt - 1) oa = a0;
-                }
-                if (oa >= 0) {
-                    const long long *q = base + oa * stride;
-                    if (stride == 1 && cnt == 8 && ((((uintptr_t)q) & 31) == 0)) {
+                } else {
+                    const long long *q = base + (long long)(NCH * ps) * stride;
+                    if (stride == 1 && (((uintptr_t)q) & 31) == 0) {
                         ld256(q, bits[0], bits[1], bits[2], bits[3]);
                         ld256(q + 4, bits[4], bits[5], bits[6], bits[7]);
-                    } else if (stride == 1 && ((((uintptr_t)q) & 15) == 0)) {
+                    } else if (stride == 1 && (((uintptr_t)q) & 15) == 0) {
                         const double2 *v = reinterpret_cast<const double2 *>(q);
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            if (2 * e + 1 < cnt) {
-                                const double2 t = v[e];
-                                bits[2 * e] = __double_as_longlong(t.x);
-                                bits[2 * e + 1] = __double_as_longlong(t.y);
-                            } else if (2 * e < cnt) {
-                                bits[2 * e] = q[2 * e];
-                            }
+                            const double2 t = v[e];
+                            bits[2 * e] = __double_as_longlong(t.x);
+                            bits[2 * e + 1] = __double_as_longlong(t.y);
                         }
                     } else {
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
-                            if (e < cnt) bits[e] = *q;
+                            bits[e] = *q;
                             q += stride;
                         }
                     }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const long long o = e < cnt ? off_of(i0 + e) : -1;
-                        if (o >= 0) bits[e] = base[o * stride];
-                    }
                 }
-            };
-            int mx = 0;
-            if (SCH == SCH_EXACT && lineE) {
-                // largest exponent field of the line (line_exp_kernel)
-                mx = valid ? lineE[S.le_off + (long long)loc.arr * nlines + g] : 0;
-            } else if (SCH == SCH_EXACT) {
+            } else {
 #pragma unroll
-                for (int c0 = 0; c0 < NGH; c0 += 2) {            // 16 loads in flight
-                    long long b0[8], b1[8];
-                    load8(group_of(c0), b0);
-                    if (c0 + 1 < NGH) load8(group_of(c0 + 1), b1);
-                    else {
+                for (int e = 0; e < 8; ++e) bits[e] = 0ll;
+                const int n = S->n, bc = S->bc;
+                int p = ps;
+                if (bc == BC_PERIODIC && n < 32) p = imod(p, n);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) b1[e] = 0ll;
+                for (int j = 0; j < PG; ++j) {
+                    if (bc == BC_PERIODIC && p >= n) p -= n;
+                    if (j < left && (bc == BC_PERIODIC || bc == BC_SHRINK || (p >= 0 && p < n))) {
+                        const long long *q = base + (long long)(KIND == KDEC ? 2 * p : p) * stride;
+                        if (KIND == KCONV) {
+                            bits[j] = *q;
+                        } else {
+                            bits[2 * j] = *q;
+                            bits[2 * j + 1] = q[(KIND == KDEC ? 1 : S->in_ext) * stride];
+                        }
                     }
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        mx = max(mx, max((int)(((unsigned long long)b0[e] >> 52) & 0x7FF),
-                                         (int)(((unsigned long long)b1[e] >> 52) & 0x7FF)));
+                    ++p;
                 }
-                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
             }
-            const int mxe = max(mx, 1);
-            // software pipeline: the next group's loads are in flight while the
-            // current group is cut into digits
-            long long bits[8], nxt[8];
-            load8(group_of(0), bits);
-            bool ok = true;
-#pragma unroll 1
-            for (int c = 0; c < NGH; ++c) {
-                if (c + 1 < NGH) load8(group_of(c + 1), nxt);
-                // pair 0 rewrites what the previous tile's TMEM-half-0 MMAs read,
-                // pairs 1 and 2 what both halves read
-                if (it > 0 && (c == 0 || c == 2) && !bar_wait(c == 0 ? pfree0 : pfree12, (it - 1) & 1)) {
-                    ok = false;
-                    break;
+            ps += PB;                                    // on to the next slab
+            if (ps >= wrap) ps -= wrap;
+            left -= PB;
+        };
+        auto open = [&](long long strip) {               // make `strip` the strip being loaded
+            const StripLoc loc = locate<BATCH>(S0, descs, prefix, nsweeps, strip);
+            if (BATCH) S = loc.S;
+            const uint32_t nlines = (uint32_t)S->nL * (uint32_t)S->nR;
+            const uint32_t g = loc.lb * kM + row;
+            const bool valid = g < nlines;
+            uint32_t l = 0, r = 0;
+            if (valid) line_lr(*S, g, l, r);
+            stride = S->nL;
+            base = reinterpret_cast<const long long *>(S->x) + (long long)loc.arr * S->x_arr + l +
+                   stride * ((long long)S->in_ext * NCH) * r;
+            const int nb = strip_blocks<PB>(*S, loc.seg);
+            nsl = nb + W - 1;
+            const int p0 = S->qlo + loc.seg * S->seg_blocks * PB + S->lowfil - woff;   // window start
+            // positions the strip's outputs use, none past the sweep's last input
+            left = min(nb * PB + NT - 1 + woff, S->qhi + S->lowfil + NT - p0) - half * PG;
+            ps = p0 + half * PG;
+            wrap = 0x40000000;
+            last = S->n;
+            if (S->bc == BC_SHRINK) {
+                ps -= S->in_lo;
+                last = 0x40000000;
+            } else if (S->bc == BC_PERIODIC) {
+                // filters reach less than 32 positions: shorter lines may wrap more
+                // than once and go element by element
+                if (last < 32) {
+                    last = -1;
+                } else {
+                    wrap = last;
+                    ps = ps < 0 ? ps + last : ps >= last ? ps - last : ps;
                 }
-                // 8 elements = 8 PL / CE core-matrix chunks of 2048 bytes (128 rows)
-                const int off = group_of(c) * (8 * G::PL / G::CE) * 2048 + (row >> 3) * 128 + (row & 7) * 16;
-                if (SCH == SCH_EXACT) {
-                    uint32_t ul[8], uh[8];
+            }
+            // largest exponent field of the line (line_exp_kernel); a row past the
+            // last line is all zeros under any scale
+            mx = 0x7FE;
+            if (!valid) left = 0;
+            else if (SCH == SCH_EXACT) mx = lineE[S->le_off + (long long)loc.arr * nlines + g];
+        };
+        long long strip = skip_inactive(blockIdx.x);
+        uint32_t slot = 0, par = 1;                      // ring position; empty phase to wait for
+        uint32_t si = 0;                                 // strips begun
+        long long bits[8];
+        int sl = 0, n_cur = 0, mxe = 1;                  // slab in `bits`, slabs of its strip
+        uint32_t mxs = 0;
+        bool fast = true;
+#pragma unroll 1
+        for (bool first = true;; first = false) {
+            // the slab's elements as operands-to-be in registers; then the next
+            // slab's loads (of the next strip after the last one) into the registers
+            // these leave, in flight while the operands wait for their slot and are
+            // stored
+            uint32_t ul[8], uh[8];                       // exact: biased fixed point
+            if (!first) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    if (SCH == SCH_EXACT) fixed_fast(bits[e], mxs, F.c10, ul[e], uh[e]);
+                    else ul[e] = f64_to_f32_bits(bits[e]);
+                }
+                if (SCH == SCH_EXACT && !fast) {
 #pragma unroll
                     for (int e = 0; e < 8; ++e) fixed_bal(bits[e], mxe, ul[e], uh[e]);
-                    // slice p holds digit planes 2p, 2p+1 = bytes 7-2p, 6-2p of
-                    // the biased fixed point: one 16-byte core-matrix row per
-                    // 4 elements
+                }
+            }
+            const bool ends = sl + 1 >= n_cur;           // the strip's last slab
+            if (ends) {
+                if (!first) strip = skip_inactive(strip + gridDim.x);
+                left = 0;
+                if (strip < nstrips) open(strip);
+            }
+            load8(bits);
+            if (!first) {
+                if (!bar_wait(empty(slot), par)) {       // the ring's first pass finds it free
+                    alive = false;
+                    break;
+                }
+                const uint32_t dst = a_addr + slot * G::SLAB + half * (8 * G::PL / G::CE) * 2048 +
+                                     (row >> 3) * 128 + (row & 7) * 16;
+                if (SCH == SCH_EXACT) {
+                    // slice p holds digit planes 2p, 2p+1 = bytes 7-2p, 6-2p: one
+                    // 16-byte core-matrix row per 4 elements
 #pragma unroll
-                    for (int sl = 0; sl < G::NS; ++sl) {
+                    for (int s = 0; s < G::NS; ++s) {
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             uint32_t wds[4];
 #pragma unroll
                             for (int w = 0; w < 4; ++w)
-                                wds[w] = digit_pair_elem(sl, ul[4 * h + w], uh[4 * h + w]);
-                            *(uint4 *)(A + sl * G::A_SLICE + off + h * 2048) = make_uint4(wds[0], wds[1], wds[2], wds[3]);
+                                wds[w] = digit_pair_elem(s, ul[4 * h + w], uh[4 * h + w]);
+                            sts128(dst + s * G::SLICE + h * 2048, wds[0], wds[1], wds[2], wds[3]);
                         }
                     }
                 } else if (SCH == SCH_BF16X3) {
                     uint32_t h[8][3];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) split_f32<3, 0xFFFF0000u>(f64_to_f32_bits(bits[e]), h[e]);
+                    for (int e = 0; e < 8; ++e) split_f32<3, 0xFFFF0000u>(ul[e], h[e]);
 #pragma unroll
                     for (int sd = 0; sd < 3; ++sd) {
                         uint32_t wds[4];
 #pragma unroll
                         for (int w = 0; w < 4; ++w) wds[w] = (h[2 * w][sd] >> 16) | (h[2 * w + 1][sd] & 0xFFFF0000u);
-                        *(uint4 *)(A + sd * G::A_SLICE + off) = make_uint4(wds[0], wds[1], wds[2], wds[3]);
+                        sts128(dst + sd * G::SLICE, wds[0], wds[1], wds[2], wds[3]);
                     }
                 } else {
                     uint32_t h[8][2];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) split_f32<2, 0xFFFFE000u>(f64_to_f32_bits(bits[e]), h[e]);
+                    for (int e = 0; e < 8; ++e) split_f32<2, 0xFFFFE000u>(ul[e], h[e]);
 #pragma unroll
                     for (int sd = 0; sd < 2; ++sd) {
-                        *(uint4 *)(A + sd * G::A_SLICE + off) = make_uint4(h[0][sd], h[1][sd], h[2][sd], h[3][sd]);
-                        *(uint4 *)(A + sd * G::A_SLICE + off + 2048) = make_uint4(h[4][sd], h[5][sd], h[6][sd], h[7][sd]);
+                        sts128(dst + sd * G::SLICE, h[0][sd], h[1][sd], h[2][sd], h[3][sd]);
+                        sts128(dst + sd * G::SLICE + 2048, h[4][sd], h[5][sd], h[6][sd], h[7][sd]);
                     }
                 }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) bits[e] = nxt[e];
-                if (c == 1 || c == 3 || c == NGH - 1) {          // last group of a pair
-                    if (c == 1 && half == 0) rowE3[(it % 3) * kM + row] = mx == 0x7FF ? 0x7FFFFFFF : mxe - 1022;
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    bar_arrive(pfull[c == 1 ? 0 : c == 3 ? 1 : 2]);
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) bar_arrive(full(slot));
+                if (++slot == kSlots) {
+                    slot = 0;
+                    par ^= 1;
                 }
             }
-            if (!ok) { alive = false; break; }
-            ++it;
+            ++sl;
+            if (ends) {
+                if (strip >= nstrips) break;
+                sl = 0;
+                n_cur = nsl;
+                mxe = max(mx, 1);
+                mxs = (uint32_t)(mx + 1) << 20;
+                fast = !__any_sync(0xffffffffu, mx < 64);
+                if (SCH == SCH_EXACT && half == 0)
+                    rowE8[(si & 7) * kM + row] = (short)(mx == 0x7FF ? 0x7FFF : mxe - 1022);
+                ++si;
+            }
         }
     } else {
-        // ============ epilogue: warp group hf issues and drains TMEM half hf
-        // (output blocks 2hf, 2hf+1); thread = TMEM lane = tile row; 8 outputs
-        // per step
-        const int ew = warp - kProducers / 32;
+        // ============ epilogue: thread = TMEM lane = row; group hf takes the blocks
+        // whose number is hf modulo 2
+        const int ew = warp - kProdWarps;
         const int lq = ew & 3, hf = ew >> 2;
         const int row = lq * 32 + lane;
+        const uint64_t a_desc0 = umma_desc(saddr(A), 2048, 128);
+        const uint64_t b_desc0 = umma_desc(saddr(B), G::LBO_B, 128);
+        const uint64_t z_desc = umma_desc(saddr(Z), 2048, 128);
+        // the block to be issued next by some warp: strip, block j of nb, its
+        // number blk, and the number of its first slab since the launch began
+        long long istrip = skip_inactive(blockIdx.x);
+        int ij = 0, inb = 0;
+        uint32_t islab = 0, iblk = 0;
+        auto istrip_blocks = [&]() {
+            if (istrip < nstrips) {
+                const StripLoc loc = locate<BATCH>(S0, descs, prefix, nsweeps, istrip);
+                inb = strip_blocks<PB>(*loc.S, loc.seg);
+            }
+        };
+        istrip_blocks();
+        // step to the next block
+        auto istep = [&]() {
+            ++iblk;
+            ++islab;
+            if (++ij == inb) {
+                islab += W - 1;
+                ij = 0;
+                istrip = skip_inactive(istrip + gridDim.x);
+                istrip_blocks();
+            }
+        };
+        // block iblk (one of this group's): issued by one of the group's warps in
+        // turn once its TMEM slot is drained and its slabs are full; every warp
+        // steps to the group's next block
+        auto issue_next = [&]() -> bool {
+            if (istrip >= nstrips) return true;
+            if (lq == (int)((iblk >> 1) & 3)) {
+                const uint32_t ts = iblk & 3, last = islab + W - 1;
+                if (iblk >= 4 && !bar_wait(drained(ts), ((iblk >> 2) - 1) & 1)) return false;
+                if (!bar_wait(full(last % kSlots), (last / kSlots) & 1)) return false;
+                if (lane == 0) {
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    uint32_t sl[W];
+                    uint64_t a[W];
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        sl[w] = (islab + w) % kSlots;
+                        a[w] = a_desc0 + (uint64_t)((sl[w] * (uint32_t)G::SLAB) >> 4);
+                    }
+                    issue_block<KIND, NT, SCH>(tmem + ts * G::SLOT_COLS, a, b_desc0, z_desc);
+                    commit(tfull(ts));
+                    bar_arrive(tfull(ts));
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        commit(empty(sl[w]));
+                        // slab ij + w is read by `readers` blocks; the first of
+                        // them stands in for the W - readers others
+                        const int k = ij + w, first = max(0, k - W + 1);
+                        const int readers = min(k, inb - 1) - first + 1;
+                        if (first == ij && readers < W) bar_arrive_n(empty(sl[w]), W - readers);
+                    }
+                }
+                __syncwarp();
+            }
+            istep();
+            if (istrip < nstrips) istep();
+            return true;
+        };
+        if (hf == 1 && istrip < nstrips) istep();        // the group's first block
+        if (!issue_next()) alive = false;
+
         // dot products per array: each epilogue warp owns the slot
-        // dot_part[(arr * gridDim.x + blockIdx.x) * 8 + ew] of every array it
-        // visits (tiles are array-major, so a CTA meets the arrays in order)
+        // dot_part[(arr * gridDim.x + blockIdx.x) * kTcDotSlots + ew] of every array it
+        // visits (strips are array-major, so a CTA meets the arrays in order)
         double dot = 0.0;
         int dot_arr = -1;
         auto flush_dot = [&]() {
             for (int o = 16; o > 0; o >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, o);
-            if (lane == 0) S0.dot_part[((long long)dot_arr * gridDim.x + blockIdx.x) * 8 + ew] = dot;
+            if (lane == 0) S0.dot_part[((long long)dot_arr * gridDim.x + blockIdx.x) * kTcDotSlots + ew] = dot;
             dot = 0.0;
         };
-        uint32_t it = 0;                                  // tiles processed (inactive arrays skipped)
-        for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            if (!BATCH && S0.active && !S0.active[locate<BATCH>(S0, descs, prefix, nsweeps, tile).arr])
-                continue;                                 // the producers skip the same tiles
-            // the group issues its TMEM half's MMAs for this tile (the half was
-            // drained by the group at the end of the previous tile) once the
-            // chunk pairs they read are written: half 0 pairs 0-1, half 1 pairs 1-2
-            if (!bar_wait(pfull[hf], it & 1) || !bar_wait(pfull[hf + 1], it & 1)) { alive = false; break; }
-            if (ew == 4 * hf) {
-                if (lane == 0) {
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    if (hf == 0) issue_half<KIND, NT, SCH, 0>(tmem, a_desc0, b_desc0, z_desc);
-                    else issue_half<KIND, NT, SCH, 1>(tmem, a_desc0, b_desc0, z_desc);
-                    commit(bT_full[hf]);
-                    if (hf == 0) commit(pfree0);
-                    commit(pfree12);
-                }
-                __syncwarp();
-            }
-            if (!bar_wait(bT_full[hf], it & 1)) { alive = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const int Er = rowE3[(it % 3) * kM + row];
-            const TileLoc loc = locate<BATCH>(S0, descs, prefix, nsweeps, tile);
+        uint32_t blk0 = 0, si = 0;                       // strip's first block, strips begun
+        int nb = 0;
+        for (long long strip = skip_inactive(blockIdx.x); alive && strip < nstrips;
+             strip = skip_inactive(strip + gridDim.x), ++si, blk0 += (uint32_t)nb) {
+            const StripLoc loc = locate<BATCH>(S0, descs, prefix, nsweeps, strip);
             const Sweep &S = *loc.S;
             const int arr = loc.arr;
-            if (!BATCH && S0.has_dot && arr != dot_arr) {
+            if (!BATCH && FORM == FORM_ANY && S0.has_dot && arr != dot_arr) {
                 if (dot_arr >= 0) flush_dot();
                 dot_arr = arr;
             }
-            const int qc0 = S.qlo + loc.ch * G::QP;
+            nb = strip_blocks<PB>(S, loc.seg);
+            const int qs = S.qlo + loc.seg * S.seg_blocks * PB;
             const long long out_pext = (long long)S.out_ext * NCH;
             const uint32_t nlines = (uint32_t)S.nL * (uint32_t)S.nR;
             const uint32_t g = loc.lb * kM + row;
@@ -858,10 +880,11 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             const long long l = l32, rr = r32;
             double *__restrict__ y = S.y + (long long)arr * S.y_arr;
             const double *__restrict__ xa = S.x + (long long)arr * S.x_arr;
-            const double *__restrict__ x2 = S.x2 ? S.x2 + (long long)arr * S.x_arr : nullptr;
+            constexpr bool kMayX2 = KIND == KCONV && (FORM == FORM_X2 || FORM == FORM_ANY);
+            const double *__restrict__ x2 = kMayX2 && S.x2 ? S.x2 + (long long)arr * S.x_arr : nullptr;
             // this row's output element (position p, channel c) sits at
             // yrow + yps p + ycs c; its x2 partial at x2row + x2s q; its input
-            // at xrow + nL ps (row bases formed once per tile)
+            // at xrow + nL ps (row bases formed once per strip)
             const long long ys = S.transpose ? S.nR : S.nL;
             double *const yrow = S.transpose ? y + rr : y + l + (long long)S.nL * out_pext * rr;
             const long long yps = KIND == KREC ? 2 * ys : ys;
@@ -873,161 +896,267 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             const long long x2s = grow ? ys : S.nL;
             const int x2lo = grow ? S.out_lo : S.in_lo;
             const double *const xrow = xa + l + (long long)S.nL * S.in_ext * rr;
-            // a row holding an Inf or NaN gives NaN; farrow: the row's scale 2^se
-            // is outside the range of the fast conversion
-            const bool nanrow = SCH == SCH_EXACT && Er == 0x7FFFFFFF;
-            const int se = nanrow ? 0 : Er + F.ef - 58;
-            const bool farrow = nanrow || se < -1022 || se > 961;
-            const double scale = __longlong_as_double((long long)(se + 1023) << 52);
             // no dot, a_x or a_y term: every output is its value (plus x2), stored
-            const bool lean = !S.has_dot && !S.has_ax && S.ay_mode == 0;
+            const bool lean = FORM != FORM_ANY || (!S.has_dot && !S.has_ax && S.ay_mode == 0);
+            constexpr bool hands = FORM == FORM_HAND;
+            int se = 0;
+            bool farrow = false;
+            double scale = 1.0, scale2 = 1.0;                // 2^se = scale (scale scale2 in a far row)
+            const int j0 = (int)((blk0 ^ (uint32_t)hf) & 1u);   // the group's first block of the strip
+            if (SCH == SCH_EXACT && j0 < nb) {
+                // known with the strip's first slab; a row holding an Inf or NaN
+                // gives NaN; farrow: 2^se is outside the range of the fast
+                // conversion (two multiplications, the first one exact)
+                if (!bar_wait(tfull((blk0 + j0) & 3), ((blk0 + j0) >> 2) & 1)) { alive = false; break; }
+                const int Er = rowE8[(si & 7) * kM + row];
+                const bool nanrow = Er == 0x7FFF;
+                se = nanrow ? 0 : max(Er + F.ef - 58, -2000);
+                farrow = valid && (nanrow || se < -1022 || se > 961);
+                const int e1 = farrow ? se / 2 : se;
+                scale = __longlong_as_double(nanrow ? 0x7FF8000000000000LL : (long long)(e1 + 1023) << 52);
+                scale2 = __longlong_as_double((long long)(se - e1 + 1023) << 52);
+            }
+            // next sweep's line exponents: the warp's 32 rows belong to one of its lines in
+            // every output column (run_plan), so one maximum per column and one
+            // atomic from the lane that keeps it
+            int *const le_col = !hands ? nullptr
+                : S0.le_next + (long long)arr * S0.le_next_lines + (loc.lb * kM + 32 * lq) / (uint32_t)max(S0.le_n1, 1);
+            auto hand_on = [&](auto &v, int q0, auto N) {    // N outputs from position q0 on
+                constexpr int n = decltype(N)::value;
+                uint32_t mine = 0;
+#pragma unroll
+                for (int i = 0; i < n; ++i) {
+                    const uint32_t m = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(v[i]) & 0x7FFFFFFFu);
+                    if (lane == i) mine = m >> 20;
+                }
+                const int p = q0 + lane / NCH, c = lane % NCH;
+                if (lane < n && p <= S.qhi && valid) {
+                    const int e = KIND == KREC ? 2 * (p - S.out_lo) + c : p - S.out_lo + S.out_ext * c;
+                    atomicMax(le_col + (long long)S0.le_n2 * e, (int)mine);
+                }
+            };
+            // any block: partial ones, dot products, a_x and a_y terms, far rows; four
+            // outputs at a time
+            auto cold_block = [&](int j) {
+                const uint32_t blk = blk0 + j;
 #pragma unroll 1
-            for (int step = 0; step < 4; ++step) {             // 2 blocks x 2 x 8 outputs
-                const int jj = step >> 1, n0 = (step & 1) * 8;
-                const int e0 = 16 * (2 * hf + jj) + n0;         // first output element of the step
-                const int q0 = qc0 + e0 / NCH;                  // e0 is a multiple of 8
-                const int nv = (S.qhi - q0 + 1) * NCH;          // valid elements of the step
-                const bool plain = lean && nv >= 8;
-                // the x2 partials first, so their loads overlap the TMEM loads
-                double add[8];
-                if (KIND == KCONV && x2 && valid) {
-                    const double *xp = x2row + x2s * (q0 - x2lo);
+                for (int st = 0; st < 4; ++st) {
+                    const int q0 = qs + j * PB + st * (4 / NCH);    // first output position of the step
+                    const int nv = (S.qhi - q0 + 1) * NCH;          // valid elements of the step
+                    const bool plain = lean && nv >= 4;
+                    uint32_t acc[G::ORD][4];
+#pragma unroll
+                    for (int k = 0; k < G::ORD; ++k)
+                        tmem_ld4(tmem + ((uint32_t)(lq * 32) << 16) +
+                                     (uint32_t)((blk & 3) * G::SLOT_COLS + k * 16 + 4 * st),
+                                 acc[k]);
+                    double add[4];
+                    if (kMayX2 && x2 && valid) {
+                        const double *xp = x2row + x2s * (q0 - x2lo);
+#pragma unroll
+                        for (int n = 0; n < 4; ++n) {
+                            add[n] = n < nv ? *xp : 0.0;
+                            xp += x2s;
+                        }
+                    }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    if (st == 3) {                        // the slot may be reissued
+                        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(drained(blk & 3));
+                    }
+                    if (!valid || nv <= 0) continue;
+                    double *const ystep = yrow + yps * (q0 - S.out_lo);
+                    // the outputs' values first (independent chains), then their memory side
+                    double outv[4];
+                    if constexpr (SCH == SCH_EXACT) {
+                        long long Y[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            uint32_t bb[G::ORD];
+#pragma unroll
+                            for (int k = 0; k < G::ORD; ++k) bb[k] = acc[k][i];
+                            Y[i] = horner_bal<G::ORD>(bb, F, i % NCH);
+                        }
+                        if (farrow) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                outv[i] = __ll2double_rn(Y[i]) * scale * scale2;
+                                if (kMayX2 && x2 && plain) outv[i] += add[i];
+                            }
+                        } else if (kMayX2 && x2 && plain) {
+                            // scale and partial sum in one FP64 instruction (the
+                            // product is exact)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) outv[i] = fma(__ll2double_rn(Y[i]), scale, add[i]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) outv[i] = ll_scaled_fast(Y[i], se);
+                        }
+                    } else {                          // sum of the order accumulators
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float f = __uint_as_float(acc[0][i]);
+#pragma unroll
+                            for (int k = 1; k < G::ORD; ++k) f += __uint_as_float(acc[k][i]);
+                            outv[i] = f32_to_f64(__float_as_uint(f));
+                        }
+                    }
+                    if (hands) hand_on(outv, q0, std::integral_constant<int, 4>());
+                    double *yq = ystep;
+                    if (plain) {
+                        if (SCH != SCH_EXACT && kMayX2 && x2) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) outv[i] += add[i];
+                        }
+                        // a contiguous output line takes the step's 4 outputs as one run
+                        // of 32 bytes (convolution; synthesis, whose channels interleave)
+                        if (KIND != KDEC && ys == 1 && (((uintptr_t)ystep) & 31) == 0) {
+                            st256(ystep, outv[0], outv[1], outv[2], outv[3]);
+                        } else if (KIND == KDEC && ys == 1 && ((((uintptr_t)ystep) | ((uintptr_t)(ystep + ycs))) & 15) == 0) {
+                            *reinterpret_cast<double2 *>(ystep) = make_double2(outv[0], outv[2]);
+                            *reinterpret_cast<double2 *>(ystep + ycs) = make_double2(outv[1], outv[3]);
+                        } else {
+#pragma unroll
+                            for (int n = 0; n < 4; ++n) {
+                                const int c = n % NCH;
+                                *(c ? yq + ycs * c : yq) = outv[n];
+                                if (c == NCH - 1) yq += yps;
+                            }
+                        }
+                        continue;
+                    }
+                    if constexpr (FORM != FORM_ANY) {        // a partial step
+#pragma unroll
+                        for (int n = 0; n < 4; ++n) {
+                            const int c = n % NCH;
+                            if (n < nv) *(c ? yq + ycs : yq) = kMayX2 && x2 ? outv[n] + add[n] : outv[n];
+                            if (c == NCH - 1) yq += yps;
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        const int q = q0 + n / NCH, c = n % NCH;
+                        if (n >= nv) break;
+                        double out = outv[n];
+                        double *const yp = c ? yq + ycs * c : yq;
+                        if (KIND == KCONV) {
+                            const bool want_dot = !BATCH && S.has_dot;   // batched sweeps have no dot
+                            if ((want_dot || S.has_ax) && (!grow || (q >= 0 && q < S.n))) {
+                                                            const double xq = xrow[(long long)S.nL * (q - S.in_lo)];
+                                if (want_dot) dot = fma(xq, out, dot);
+                                if (S.has_ax) out = fma(xq, S.a_x, out);
+                            }
+                            if (kMayX2 && x2) out += add[n];
+                        }
+                        if (S.ay_mode == 2) out += *yp;
+                        else if (S.ay_mode == 1) out = fma(S.a_y, *yp, out);
+                        *yp = out;
+                        if (c == NCH - 1) yq += yps;
+                    }
+                }
+            };
+            // the common case, a whole block of a plain sweep: one tight loop of straight
+            // runs of eight outputs, so that recombination, conversion (the narrow
+            // FP64 pipe) and stores of neighbouring outputs overlap
+            double addn[8];                              // x2 partials of the next eight outputs
+            auto load_x2 = [&](const double *xp) {
+                if (valid) {
 #pragma unroll
                     for (int n = 0; n < 8; ++n) {
-                        add[n] = n < nv ? *xp : 0.0;
+                        addn[n] = *xp;
                         xp += x2s;
                     }
                 }
-                uint32_t acc[G::ORD][8];
+            };
+            auto full_block = [&](int j) { return j < nb && qs + (j + 1) * PB - 1 <= S.qhi; };
+            auto hot_block = [&](auto VEC, int j) {
+                constexpr bool kX2 = FORM == FORM_X2, kHands = FORM == FORM_HAND, kVec = decltype(VEC)::value;
+                const uint32_t blk = blk0 + j;
+                double *yb = yrow + yps * (qs + j * PB - S.out_lo);
+                const double *xb = kX2 ? x2row + x2s * (qs + j * PB + 8 - x2lo) : nullptr;   // the next eight
+                const uint32_t ta = tmem + ((uint32_t)(lq * 32) << 16) + (blk & 3) * G::SLOT_COLS;
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t acc[G::ORD][8];
 #pragma unroll
-                for (int k = 0; k < G::ORD; ++k)
-                    tmem_ld8(tmem + ((uint32_t)(lq * 32) << 16) +
-                                 (uint32_t)(hf * G::HALF_COLS + (jj * G::ORD + k) * 16 + n0),
-                             acc[k]);
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (!valid || nv <= 0) continue;
-                double *const ystep = yrow + yps * (q0 - S.out_lo);
-                // the 8 outputs' values first (independent, branch-free chains;
-                // one rare fix-up), then their memory side
-                double outv[8];
-                if constexpr (SCH == SCH_EXACT) {
-                    long long Y[8];
+                    for (int k = 0; k < G::ORD; ++k) tmem_ld8(ta + k * 16 + 8 * h, acc[k]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    if (h == 1) {             // the slot may be reissued
+                        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(drained(blk & 3));
+                    }
+                    double v[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        uint32_t bb[G::ORD];              // 0x4B400000 + Acc_k (biased start)
+                        if constexpr (SCH == SCH_EXACT) {
+                            uint32_t bb[G::ORD];
 #pragma unroll
-                        for (int k = 0; k < G::ORD; ++k) bb[k] = acc[k][i];
-                        Y[i] = horner_bal<G::ORD>(bb);
-                    }
-                    if (farrow) {
+                            for (int k = 0; k < G::ORD; ++k) bb[k] = acc[k][i];
+                            const long long Y = horner_bal<G::ORD>(bb, F, i % NCH);
+                            // x2: scale and partial sum in one FP64 instruction (the
+                            // product is exact)
+                            if (kX2) v[i] = fma(__ll2double_rn(Y), scale, addn[i]);
+                            else v[i] = ll_scaled_fast(Y, se);
+                        } else {                         // sum of the order accumulators
+                            float f = __uint_as_float(acc[0][i]);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            outv[i] = nanrow ? __longlong_as_double(0x7FF8000000000000LL)
-                                             : ll_scaled(Y[i], se);
-                            if (KIND == KCONV && x2 && plain) outv[i] += add[i];
+                            for (int k = 1; k < G::ORD; ++k) f += __uint_as_float(acc[k][i]);
+                            v[i] = f32_to_f64(__float_as_uint(f));
+                            if (kX2) v[i] += addn[i];
                         }
-                    } else if (KIND == KCONV && x2 && plain) {
-                        // scale and partial sum in one FP64 instruction (the
-                        // product is exact)
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) outv[i] = fma(__ll2double_rn(Y[i]), scale, add[i]);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) outv[i] = ll_scaled_fast(Y[i], se);
+                        if (!kVec) {
+                            const int c = i % NCH;
+                            if (valid) *(c ? yb + ycs : yb) = v[i];
+                            if (c == NCH - 1) yb += yps;
+                        }
                     }
-                } else {                          // sum of the order accumulators
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float f = __uint_as_float(acc[0][i]);
-#pragma unroll
-                        for (int k = 1; k < G::ORD; ++k) f += __uint_as_float(acc[k][i]);
-                        outv[i] = f32_to_f64(__float_as_uint(f));
+                    if (kVec) {
+                        // a contiguous output line takes its 8 outputs as two 32-byte
+                        // runs: elements 0-7 (convolution; synthesis, whose channels
+                        // interleave), or channel 0 and channel 1 (analysis)
+                        if (valid) {
+                            if (KIND == KDEC) {
+                                st256(yb, v[0], v[2], v[4], v[6]);
+                                st256(yb + ycs, v[1], v[3], v[5], v[7]);
+                            } else {
+                                st256(yb, v[0], v[1], v[2], v[3]);
+                                st256(yb + 4, v[4], v[5], v[6], v[7]);
+                            }
+                        }
+                        yb += 8 / NCH * yps;
                     }
+                    if (kX2) {                           // in flight until the next eight's conversion
+                        if (h == 0) load_x2(xb);
+                        else if (full_block(j + 2)) load_x2(xb + x2s * (2 * PB - 8));
+                    }
+                    if (kHands) hand_on(v, qs + j * PB + h * (8 / NCH), std::integral_constant<int, 8>());
                 }
-                double *yq = ystep;
-                if (plain) {
-                    if (SCH != SCH_EXACT && KIND == KCONV && x2) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) outv[i] += add[i];
-                    }
-                    if (!BATCH && KIND == KCONV && S0.le_next) {
-                        // the warp's maximum exponent field of each of the 8 output
-                        // columns (every lane is here: run_plan hands off only
-                        // whole tiles of valid lines); lane i keeps column i's
-                        uint32_t mine = 0;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const uint32_t ex = (uint32_t)((unsigned long long)__double_as_longlong(outv[i]) >> 52) & 0x7FFu;
-                            const uint32_t m = __reduce_max_sync(0xffffffffu, ex);
-                            if (lane == i) mine = m;
-                        }
-                        if (lane < 8) colE[(hf * 4 + lq) * 32 + step * 8 + lane] = (int)mine;
-                    }
-                    // a contiguous output line takes the step's 8 outputs as two
-                    // 32-byte runs: elements 0-7 (convolution; synthesis, whose
-                    // channels interleave), or channel 0 and channel 1 (analysis)
-                    double *const r1 = KIND == KDEC ? ystep + ycs : ystep + 4;
-                    if (ys == 1 && ((((uintptr_t)ystep) | ((uintptr_t)r1)) & 31) == 0) {
-                        if (KIND == KDEC) {
-                            st256(ystep, outv[0], outv[2], outv[4], outv[6]);
-                            st256(r1, outv[1], outv[3], outv[5], outv[7]);
-                        } else {
-                            st256(ystep, outv[0], outv[1], outv[2], outv[3]);
-                            st256(r1, outv[4], outv[5], outv[6], outv[7]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int n = 0; n < 8; ++n) {
-                            const int c = n % NCH;
-                            *(c ? yq + ycs * c : yq) = outv[n];
-                            if (c == NCH - 1) yq += yps;
-                        }
-                    }
-                    continue;
-                }
-#pragma unroll
-                for (int n = 0; n < 8; ++n) {
-                    const int q = q0 + n / NCH, c = n % NCH;
-                    if (n >= nv) break;
-                    double out = outv[n];
-                    double *const yp = c ? yq + ycs * c : yq;
-                    if (KIND == KCONV) {
-                        const bool want_dot = !BATCH && S.has_dot;   // batched sweeps have no dot
-                        if ((want_dot || S.has_ax) && (!grow || (q >= 0 && q < S.n))) {
-                            const int ps = S.bc == BC_PERIODIC ? imod(q, S.n) : q - S.in_lo;
-                            const double xq = xrow[(long long)S.nL * ps];
-                            if (want_dot) dot = fma(xq, out, dot);
-                            if (S.has_ax) out = fma(xq, S.a_x, out);
-                        }
-                        if (x2) out += add[n];
-                    }
-                    if (S.ay_mode == 2) out += *yp;
-                    else if (S.ay_mode == 1) out = fma(S.a_y, *yp, out);
-                    *yp = out;
-                    if (c == NCH - 1) yq += yps;
-                }
+            };
+            const bool vec = ys == 1 && (KIND == KDEC ? ((((uintptr_t)yrow | (uintptr_t)(yrow + ycs)) & 31) == 0)
+                                                      : (((uintptr_t)yrow) & 31) == 0) &&
+                             (yps * (qs - S.out_lo)) % 4 == 0;
+            const bool hot = FORM != FORM_ANY && !__any_sync(0xffffffffu, farrow);
+            const bool vecs = __all_sync(0xffffffffu, vec || !valid);
+            if (FORM == FORM_X2 && hot && full_block(j0)) load_x2(x2row + x2s * (qs + j0 * PB - x2lo));
+            const std::true_type yes{};
+            const std::false_type no{};
+#pragma unroll 1
+            for (int j = j0; j < nb; j += 2) {
+                const uint32_t blk = blk0 + j;
+                // issuing after the wait keeps the phases apart: the slabs that
+                // block blk + 2's replaced in the ring were read by block blk or
+                // an earlier one, so their phase is known to be over
+                if (!bar_wait(tfull(blk & 3), (blk >> 2) & 1) || !issue_next()) { alive = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                if (FORM == FORM_ANY || !hot || !full_block(j)) cold_block(j);
+                else if (vecs) hot_block(yes, j);
+                else hot_block(no, j);
             }
-            // the whole group has read TMEM half hf: it may be reissued
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            bar_arrive(gsync[hf]);
-            if (!bar_wait(gsync[hf], it & 1)) { alive = false; break; }
-            if (!BATCH && KIND == KCONV && S0.le_next && lq == 0) {
-                // lane c: output column 32 hf + c; the tile's 128 lines form 128 / n1
-                // of the next sweep's lines per column, warps (32 lq) / n1 == k the
-                // k-th (the group's other warps wrote colE before the barrier, and
-                // write it again only after this warp issues the next tile's MMAs)
-                const int n1 = S0.le_n1, per = kM / n1;
-                const int q = qc0 + 32 * hf + lane;
-                for (int k = 0; k < per; ++k) {
-                    int m = 0;
-                    for (int w = k * n1 / 32; w < (k + 1) * n1 / 32; ++w) m = max(m, colE[(hf * 4 + w) * 32 + lane]);
-                    const long long i2 = (long long)loc.lb * per + k;
-                    S0.le_next[(long long)arr * S0.le_next_lines + i2 + (long long)S0.le_n2 * (q - S0.out_lo)] = m;
-                }
-            }
-            ++it;
         }
-        if (!BATCH && S0.has_dot && dot_arr >= 0) flush_dot();
+        if (!BATCH && FORM == FORM_ANY && S0.has_dot && dot_arr >= 0) flush_dot();
     }
 
     if (!alive) atomicExch(status, 1);
@@ -1039,19 +1168,29 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                      : "memory");
 }
 
-template <int KIND, int NT, int SCH, bool BATCH>
+template <int KIND, int NT, int SCH, bool BATCH, int FORM>
 cudaError_t set_smem_attr() {
     using G = Geom<KIND, NT, SCH>;
     static bool attr[64] = {};   // the attribute is set once per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !attr[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(sweep_tc_kernel<KIND, NT, SCH, BATCH>,
+        cudaError_t e = cudaFuncSetAttribute(sweep_tc_kernel<KIND, NT, SCH, BATCH, FORM>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr[dev] = true;
     }
     return cudaSuccess;
+}
+
+template <int KIND, int NT, int SCH, int FORM>
+cudaError_t launch_form(const Sweep &S, const TcFilter &F, int *status, const int *lineE, cudaStream_t st) {
+    using G = Geom<KIND, NT, SCH>;
+    cudaError_t e = set_smem_attr<KIND, NT, SCH, false, FORM>();
+    if (e != cudaSuccess) return e;
+    sweep_tc_kernel<KIND, NT, SCH, false, FORM><<<(int)sweep_tc_blocks(S), kThreads, G::SMEM, st>>>(
+        S, F, status, nullptr, nullptr, 0, lineE);
+    return cudaGetLastError();
 }
 
 template <int KIND, int NT, int SCH>
@@ -1065,28 +1204,42 @@ cudaError_t launch(const Sweep &S_in, const TcFilter &F, int *status, const int 
     if (KIND == KCONV && G::KB - 15 - NT >= 3 && S.nL == 1 && S.bc == BC_PERIODIC && S.n % 4 == 0 &&
         S.in_ext % 4 == 0 && S.x_arr % 4 == 0 && (((uintptr_t)S.x) & 31) == 0)
         S.woff = ((S.qlo + S.lowfil) % 4 + 4) % 4;
-    cudaError_t e = set_smem_attr<KIND, NT, SCH, false>();
+    if (S.has_dot || S.has_ax || S.ay_mode || (S.x2 && NT != 29))
+        return launch_form<KIND, NT, SCH, FORM_ANY>(S, F, status, lineE, st);
+    if constexpr (KIND == KCONV && NT == 29)
+        if (S.x2) return launch_form<KIND, NT, SCH, FORM_X2>(S, F, status, lineE, st);
+    if constexpr (SCH == SCH_EXACT && (KIND != KCONV || NT == 16))
+        if (S.le_next) return launch_form<KIND, NT, SCH, FORM_HAND>(S, F, status, lineE, st);
+    return launch_form<KIND, NT, SCH, FORM_PLAIN>(S, F, status, lineE, st);
+}
+
+// Batched launch over nsweeps descriptors (device arrays) of the form of `like`;
+// S0 only carries has_dot = 0.  One CTA per SM.  lineE (exact scheme, or null):
+// line exponent maxima of every sweep's lines, sweep i's at descs[i].le_off.
+template <int KIND, int NT, int SCH, int FORM>
+cudaError_t launch_batch_form(const Sweep *descs, const long long *prefix, int nsweeps,
+                              const TcFilter &F, int *status, const int *lineE, cudaStream_t st) {
+    using G = Geom<KIND, NT, SCH>;
+    cudaError_t e = set_smem_attr<KIND, NT, SCH, true, FORM>();
     if (e != cudaSuccess) return e;
-    const long long tiles = tile_count_for(S, G::QP);
-    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    sweep_tc_kernel<KIND, NT, SCH, false><<<grid, kThreads, G::SMEM, st>>>(S, F, status, nullptr,
-                                                                           nullptr, 0, lineE);
+    Sweep S0{};
+    sweep_tc_kernel<KIND, NT, SCH, true, FORM><<<sm_count(), kThreads, G::SMEM, st>>>(
+        S0, F, status, descs, prefix, nsweeps, lineE);
     return cudaGetLastError();
 }
 
-// Batched launch over nsweeps descriptors (device arrays); S0 only carries
-// has_dot = 0.  One CTA per SM.  lineE (exact scheme, or null): line
-// exponent maxima of every sweep's lines, sweep i's at descs[i].le_off.
 template <int KIND, int NT, int SCH>
-cudaError_t launch_batch(const Sweep *descs, const long long *prefix, int nsweeps,
+cudaError_t launch_batch(const Sweep &like, const Sweep *descs, const long long *prefix, int nsweeps,
                          const TcFilter &F, int *status, const int *lineE, cudaStream_t st) {
-    using G = Geom<KIND, NT, SCH>;
-    cudaError_t e = set_smem_attr<KIND, NT, SCH, true>();
-    if (e != cudaSuccess) return e;
-    Sweep S0{};
-    sweep_tc_kernel<KIND, NT, SCH, true><<<sm_count(), kThreads, G::SMEM, st>>>(S0, F, status, descs,
-                                                                                prefix, nsweeps, lineE);
-    return cudaGetLastError();
+    if constexpr (NT == 29) {
+        if (like.has_ax || like.ay_mode)
+            return launch_batch_form<KIND, NT, SCH, FORM_ANY>(descs, prefix, nsweeps, F, status, lineE, st);
+        if (like.x2)
+            return launch_batch_form<KIND, NT, SCH, FORM_X2>(descs, prefix, nsweeps, F, status, lineE, st);
+    } else if (like.has_ax || like.ay_mode || like.x2) {
+        return cudaErrorInvalidValue;
+    }
+    return launch_batch_form<KIND, NT, SCH, FORM_PLAIN>(descs, prefix, nsweeps, F, status, lineE, st);
 }
 
 }  // namespace tck
