@@ -74,14 +74,14 @@
 // outputs held the whole operand buffer, so conversion, MMAs and drain of a tile
 // ran one after the other, and every tile converted its halo again; the kernel
 // was 190 KB of code with one epilogue for every case.  MagicFilter sweep 520 ->
-// 325 us, kinetic sweep along x 600 -> 361 us, with partial sums 640 -> 566 us
+// 325 us, kinetic sweep along x 600 -> 361 us, with partial sums 640 -> 485 us
 // (issue slots 46 %, FP64 pipe 31 %, tensor pipe 20 %, HBM 25-50 %).  What
 // mattered: the ring; one kernel per form of sweep with a short straight
 // epilogue loop (no spills, 50 KB: 436 -> 325 us for the MagicFilter sweep alone);
 // digits as FP16 subnormals; polls and shared-memory stores in few instructions.
 // Measured and slower: three epilogue groups and an issuer warp on 24 warps (80
 // registers: 1.58 ms against 1.52 for MagicFilter3D), TMEM loads one step ahead,
-// global loads two slabs ahead (kinetic 1.60 -> 1.65 ms), larger unrolled loops.
+// global loads two slabs ahead (kinetic 1.60 -> 1.65 ms; one slab ahead, the next on its way to L2), larger unrolled loops.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -951,8 +951,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     atomicMax(le_col + (long long)S0.le_n2 * e, (int)mine);
                 }
             };
-            // any block: partial ones, dot products, a_x and a_y terms, far rows; four
-            // outputs at a time
+            // any block: partial ones, far rows; four outputs at a time
             auto cold_block = [&](int j) {
                 const uint32_t blk = blk0 + j;
 #pragma unroll 1
@@ -1076,22 +1075,11 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             // the common case, a whole block of a plain sweep: one tight loop of straight
             // runs of eight outputs, so that recombination, conversion (the narrow
             // FP64 pipe) and stores of neighbouring outputs overlap
-            double addn[8];                              // x2 partials of the next eight outputs
-            auto load_x2 = [&](const double *xp) {
-                if (valid) {
-#pragma unroll
-                    for (int n = 0; n < 8; ++n) {
-                        addn[n] = *xp;
-                        xp += x2s;
-                    }
-                }
-            };
             auto full_block = [&](int j) { return j < nb && qs + (j + 1) * PB - 1 <= S.qhi; };
             auto hot_block = [&](auto VEC, int j) {
-                constexpr bool kX2 = FORM == FORM_X2, kHands = FORM == FORM_HAND, kVec = decltype(VEC)::value;
+                constexpr bool kHands = FORM == FORM_HAND, kVec = decltype(VEC)::value;
                 const uint32_t blk = blk0 + j;
                 double *yb = yrow + yps * (qs + j * PB - S.out_lo);
-                const double *xb = kX2 ? x2row + x2s * (qs + j * PB + 8 - x2lo) : nullptr;   // the next eight
                 const uint32_t ta = tmem + ((uint32_t)(lq * 32) << 16) + (blk & 3) * G::SLOT_COLS;
 #pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
@@ -1112,16 +1100,12 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
 #pragma unroll
                             for (int k = 0; k < G::ORD; ++k) bb[k] = acc[k][i];
                             const long long Y = horner_bal<G::ORD>(bb, F, i % NCH);
-                            // x2: scale and partial sum in one FP64 instruction (the
-                            // product is exact)
-                            if (kX2) v[i] = fma(__ll2double_rn(Y), scale, addn[i]);
-                            else v[i] = ll_scaled_fast(Y, se);
+                            v[i] = ll_scaled_fast(Y, se);
                         } else {                         // sum of the order accumulators
                             float f = __uint_as_float(acc[0][i]);
 #pragma unroll
                             for (int k = 1; k < G::ORD; ++k) f += __uint_as_float(acc[k][i]);
                             v[i] = f32_to_f64(__float_as_uint(f));
-                            if (kX2) v[i] += addn[i];
                         }
                         if (!kVec) {
                             const int c = i % NCH;
@@ -1144,21 +1128,139 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                         }
                         yb += 8 / NCH * yps;
                     }
-                    if (kX2) {                           // in flight until the next eight's conversion
-                        if (h == 0) load_x2(xb);
-                        else if (full_block(j + 2)) load_x2(xb + x2s * (2 * PB - 8));
-                    }
                     if (kHands) hand_on(v, qs + j * PB + h * (8 / NCH), std::integral_constant<int, 8>());
+                }
+            };
+            // a whole block with partial sums, dot product, a_x and a_y terms: four
+            // outputs at a time, the next four's operands in flight meanwhile and the
+            // group's next block's on their way to L2.  Bound by the chain of operand
+            // latency, conversion and FP64 arithmetic in two warps per scheduler;
+            // four outputs a step keep everything in registers (eight a step, and
+            // operands two or four steps ahead, spill or outgrow the loop: kinetic
+            // sweep with partial sums, 32 x 128^3, 580 us at eight, 485 at four, 515
+            // with operands two steps ahead).  Kinetic sweeps with energies (and a_y),
+            // 110^3 x 8, went through cold_block before: 213-349 us, now 164-199
+            const bool want_dot = !BATCH && FORM == FORM_ANY && S.has_dot;
+            const bool want_x = FORM == FORM_ANY && (want_dot || S.has_ax), want_y = FORM == FORM_ANY && S.ay_mode != 0;
+            double ta[4], tx[4], ty[4];                  // the next four outputs' x2, x and y
+            auto load_terms = [&](auto VEC, int q) {
+                if (!valid) return;
+                auto run = [&](double (&d)[4], const double *p, long long st) {
+                    if constexpr (decltype(VEC)::value) {
+                        long long b0, b1, b2, b3;
+                        ld256(reinterpret_cast<const long long *>(p), b0, b1, b2, b3);
+                        d[0] = __longlong_as_double(b0), d[1] = __longlong_as_double(b1);
+                        d[2] = __longlong_as_double(b2), d[3] = __longlong_as_double(b3);
+                    } else {
+#pragma unroll
+                        for (int n = 0; n < 4; ++n) {
+                            d[n] = *p;
+                            p += st;
+                        }
+                    }
+                };
+                if (x2) run(ta, x2row + x2s * (q - x2lo), x2s);
+                if (want_x) run(tx, xrow + (long long)S.nL * (q - S.in_lo), S.nL);
+                if (want_y) run(ty, yrow + yps * (q - S.out_lo), yps);
+            };
+            auto term_block = [&](auto VEC, int j) {
+                constexpr bool kVec = decltype(VEC)::value;
+                const uint32_t blk = blk0 + j;
+                const int q0 = qs + j * PB;
+                const uint32_t tb = tmem + ((uint32_t)(lq * 32) << 16) + (blk & 3) * G::SLOT_COLS;
+                const bool more = full_block(j + 2);
+                if (more && valid) {                     // the group's next block on its way to L2
+                    const int q = q0 + 2 * PB + (lane & 15);
+                    if (x2) prefetch_l2(x2row + x2s * (q - x2lo));
+                    if (want_x) prefetch_l2(xrow + (long long)S.nL * (q - S.in_lo));
+                    if (want_y) prefetch_l2(yrow + yps * (q - S.out_lo));
+                }
+                double *yb = yrow + yps * (q0 - S.out_lo);
+#pragma unroll 1
+                for (int st = 0; st < 4; ++st) {
+                    uint32_t acc[G::ORD][4];
+#pragma unroll
+                    for (int k = 0; k < G::ORD; ++k) tmem_ld4(tb + k * 16 + 4 * st, acc[k]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    if (st == 3) {                       // the slot may be reissued
+                        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(drained(blk & 3));
+                    }
+                    double v[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if constexpr (SCH == SCH_EXACT) {
+                            uint32_t bb[G::ORD];
+#pragma unroll
+                            for (int k = 0; k < G::ORD; ++k) bb[k] = acc[k][i];
+                            const long long Y = horner_bal<G::ORD>(bb, F, 0);
+                            // x2 alone: scale and partial sum in one FP64
+                            // instruction (the product is exact)
+                            if (x2 && !want_x) v[i] = fma(__ll2double_rn(Y), scale, ta[i]);
+                            else v[i] = ll_scaled_fast(Y, se);
+                        } else {
+                            float f = __uint_as_float(acc[0][i]);
+#pragma unroll
+                            for (int k = 1; k < G::ORD; ++k) f += __uint_as_float(acc[k][i]);
+                            v[i] = f32_to_f64(__float_as_uint(f));
+                            if (x2 && !want_x) v[i] += ta[i];
+                        }
+                    }
+                    if (want_x) {
+                        if (want_dot && valid) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) dot = fma(tx[i], v[i], dot);
+                        }
+                        if (S.has_ax) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) v[i] = fma(tx[i], S.a_x, v[i]);
+                        }
+                        if (x2) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) v[i] += ta[i];
+                        }
+                    }
+                    if (want_y) {
+                        const double ay = S.ay_mode == 1 ? S.a_y : 1.0;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) v[i] = fma(ay, ty[i], v[i]);
+                    }
+                    if (st < 3) load_terms(VEC, q0 + 4 * st + 4);
+                    else if (more) load_terms(VEC, q0 + 2 * PB);
+                    if (valid) {
+                        if (kVec) {
+                            st256(yb, v[0], v[1], v[2], v[3]);
+                        } else {
+                            double *yp = yb;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                *yp = v[i];
+                                yp += yps;
+                            }
+                        }
+                    }
+                    yb += 4 * yps;
                 }
             };
             const bool vec = ys == 1 && (KIND == KDEC ? ((((uintptr_t)yrow | (uintptr_t)(yrow + ycs)) & 31) == 0)
                                                       : (((uintptr_t)yrow) & 31) == 0) &&
                              (yps * (qs - S.out_lo)) % 4 == 0;
-            const bool hot = FORM != FORM_ANY && !__any_sync(0xffffffffu, farrow);
-            const bool vecs = __all_sync(0xffffffffu, vec || !valid);
-            if (FORM == FORM_X2 && hot && full_block(j0)) load_x2(x2row + x2s * (qs + j0 * PB - x2lo));
+            // cold_block: far rows, and a dot product or a_x term of a growing sweep,
+            // whose input has no element for its outer outputs
+            constexpr bool kTerms = KIND == KCONV && (FORM == FORM_ANY || FORM == FORM_X2);
+            const bool hot = (kTerms || FORM != FORM_ANY) && !__any_sync(0xffffffffu, farrow) && !(want_x && grow);
+            auto unit = [&](const double *p, long long st) { return st == 1 && (((uintptr_t)p) & 31) == 0; };
+            const bool tvec = vec && (!x2 || unit(x2row + x2s * (qs - x2lo), x2s)) &&
+                              (!want_x || unit(xrow + (long long)S.nL * (qs - S.in_lo), S.nL));
+            const bool vecs = __all_sync(0xffffffffu, (kTerms ? tvec : vec) || !valid);
             const std::true_type yes{};
             const std::false_type no{};
+            if constexpr (kTerms)
+                if (hot && full_block(j0)) {
+                    if (vecs) load_terms(yes, qs + j0 * PB);
+                    else load_terms(no, qs + j0 * PB);
+                }
 #pragma unroll 1
             for (int j = j0; j < nb; j += 2) {
                 const uint32_t blk = blk0 + j;
@@ -1167,9 +1269,16 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 // an earlier one, so their phase is known to be over
                 if (!bar_wait(tfull(blk & 3), (blk >> 2) & 1) || !issue_next()) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                if (FORM == FORM_ANY || !hot || !full_block(j)) cold_block(j);
-                else if (vecs) hot_block(yes, j);
-                else hot_block(no, j);
+                if (!hot || !full_block(j)) {
+                    cold_block(j);
+                } else if constexpr (kTerms) {
+                    if (vecs) term_block(yes, j);
+                    else term_block(no, j);
+                } else if (vecs) {
+                    hot_block(yes, j);
+                } else {
+                    hot_block(no, j);
+                }
             }
         }
         if (!BATCH && FORM == FORM_ANY && S0.has_dot && dot_arr >= 0) flush_dot();
