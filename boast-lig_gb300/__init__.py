@@ -342,10 +342,9 @@ class Hamiltonian:
 
     # kernel launches of one call on free boundaries: 15 sweeps, the potential
     # kernel and its reduction, and the three kinetic-energy reductions; in the
-    # exact tensor-core mode also 11 line-exponent passes (one for the three
-    # kinetic sweeps, one for the synthesis, whose sweeps hand on theirs when 2n
-    # is a multiple of 32; with other sizes 13)
-    LAUNCHES = {'exact': 31, 'other': 20}
+    # exact tensor-core mode also five line-exponent passes, one per operator
+    # (its sweeps hand on theirs; grids below 32 points an axis take more)
+    LAUNCHES = {'exact': 25, 'other': 20}
 
     def __call__(self, psig, pot, hpsig, rho=None, stream=None, energies=None):
         """energies: optional device tensor of norb * 4 doubles to receive the

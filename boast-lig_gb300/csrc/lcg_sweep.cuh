@@ -48,8 +48,8 @@ struct Sweep {
     // exponents (run_plan decides): the epilogue raises the largest exponent
     // field of each of the next sweep's lines, zeroed before the launch,
     // le_next[a le_next_lines + i2 + le_n2 e], for this sweep's line i1 + le_n1
-    // i2 and output element e (le_n1 = the next sweep's line length, a multiple
-    // of 32: a warp's 32 rows belong to one of its lines)
+    // i2 and output element e (le_n1 = the next sweep's line length, at least
+    // 32: a warp's 32 rows belong to one of its lines or two neighbouring ones)
     int *le_next = nullptr;
     long long le_next_lines = 0;
     int le_n1 = 0, le_n2 = 0;

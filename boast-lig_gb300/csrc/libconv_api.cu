@@ -420,13 +420,13 @@ struct Scratch {
 
 // Exact tensor-core step k hands its successor the line exponents of its
 // output (the epilogue's atomics, Sweep::le_next) instead of a pre-pass over
-// that output: k is a transposed sweep (16 taps, or a wavelet's) without dot, a_x,
-// a_y or x2, k + 1 reads
-// k's output along its fastest axis (n1 elements a line, none of them padding),
-// and n1 and k's lines are multiples of 32, so that each epilogue warp's rows
-// belong to one line of k + 1 in every output column: k's line i1 + n1 i2 and
-// output e are k + 1's line i2 + n2 e at element i1.
-// 32 arrays of 128^3: the pre-pass takes 81 us.
+// that output: k is a transposed sweep (16 taps, or a wavelet's) without dot,
+// a_x, a_y or x2, k + 1 reads k's output along its fastest axis (n1 elements a
+// line, none of them padding), and n1 >= 32, so that each epilogue warp's 32
+// rows belong to at most two lines of k + 1 in every output column: k's line
+// i1 + n1 i2 and output e are k + 1's line i2 + n2 e at element i1.  Shorter
+// lines keep the pre-pass.  32 arrays of 128^3: the pre-pass takes 81 us, handing
+// on 5; 8 of 110^3 to 125^3: 20-31 us a pre-pass (Hamiltonian 1932 -> 1855 us).
 bool exp_handoff(const Plan &P, size_t k, int &n1, int &n2) {
     if (t_mode != LIBCONV_MODE_TC_EXACT || k + 1 >= P.steps.size()) return false;
     const PlanStep &a = P.steps[k], &b = P.steps[k + 1];
@@ -439,7 +439,7 @@ bool exp_handoff(const Plan &P, size_t k, int &n1, int &n2) {
         return false;
     const int mA = A.kind == KCONV ? 1 : 2, mB = B.kind == KCONV ? 1 : 2;
     const long long lines = A.nR, len = (long long)B.in_ext * mB;
-    if (len % 32 || lines % 32 || lines % len) return false;
+    if (len < 32 || lines % len) return false;
     // every element of A's output is written, and every one of B's lines is used
     if (A.qhi - A.qlo + 1 != A.out_ext || A.qlo != A.out_lo) return false;
     const int used = B.bc == BC_SHRINK ? B.qhi + B.lowfil + B.ntaps - B.in_lo : B.n;

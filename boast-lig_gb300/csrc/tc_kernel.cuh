@@ -104,8 +104,12 @@ constexpr uint32_t kWaitPolls = 1u << 26;            // polls of a wait: seconds
 
 // Forms of a sweep, one kernel each, so that the epilogue of the common ones is
 // a short loop (code and registers): plain stores; plus a partial sum x2; plus
-// the next sweep's line exponents; anything (dot products, a_x, a_y).
-enum Form { FORM_PLAIN = 0, FORM_X2 = 1, FORM_HAND = 2, FORM_ANY = 3 };
+// the next sweep's line exponents, a warp's rows in one of its lines (HAND) or
+// in one or two (HAND2); anything (dot products, a_x, a_y).
+enum Form { FORM_PLAIN = 0, FORM_X2 = 1, FORM_HAND = 2, FORM_ANY = 3, FORM_HAND2 = 4 };
+// How a block's outputs lie in memory: 32-byte runs, anyhow, anyhow and the
+// line ends within the block.
+enum Run { RUN_VEC = 0, RUN_ANY = 1, RUN_PART = 2 };
 
 template <int KIND, int NT, int SCH> struct Geom {
     static constexpr int NCH = KIND == KCONV ? 1 : 2;            // elements per position
@@ -914,7 +918,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             const double *const xrow = xa + l + (long long)S.nL * S.in_ext * rr;
             // no dot, a_x or a_y term: every output is its value (plus x2), stored
             const bool lean = FORM != FORM_ANY || (!S.has_dot && !S.has_ax && S.ay_mode == 0);
-            constexpr bool hands = FORM == FORM_HAND;
+            constexpr bool hands = FORM == FORM_HAND || FORM == FORM_HAND2;
             int se = 0;
             bool farrow = false;
             double scale = 1.0, scale2 = 1.0;                // 2^se = scale (scale scale2 in a far row)
@@ -932,26 +936,36 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 scale = __longlong_as_double(nanrow ? 0x7FF8000000000000LL : (long long)(e1 + 1023) << 52);
                 scale2 = __longlong_as_double((long long)(se - e1 + 1023) << 52);
             }
-            // next sweep's line exponents: the warp's 32 rows belong to one of its lines in
-            // every output column (run_plan), so one maximum per column and one
-            // atomic from the lane that keeps it
-            int *const le_col = !hands ? nullptr
-                : S0.le_next + (long long)arr * S0.le_next_lines + (loc.lb * kM + 32 * lq) / (uint32_t)max(S0.le_n1, 1);
+            // next sweep's line exponents: the warp's 32 rows lie in one of its lines in
+            // every output column, or in two neighbouring ones (run_plan: lines of at
+            // least 32), so one or two maxima per column and an atomic from the
+            // lanes that keep them
+            const uint32_t g0 = loc.lb * kM + 32 * lq, ln = hands ? g0 / (uint32_t)max(S0.le_n1, 1) : 0;
+            const uint32_t cut = (ln + 1) * (uint32_t)S0.le_n1;      // first row of the second line
+            const bool two = FORM == FORM_HAND2 && g0 + 32 > cut && cut < nlines;
+            int *const le_col = !hands ? nullptr : S0.le_next + (long long)arr * S0.le_next_lines + ln;
+            const uint32_t sel = !valid ? 0u : g < cut || !two ? 0x7FFFFFFFu : 0u;     // rows of the first line
             auto hand_on = [&](auto &v, int q0, auto N) {    // N outputs from position q0 on
                 constexpr int n = decltype(N)::value;
-                uint32_t mine = 0;
-#pragma unroll
-                for (int i = 0; i < n; ++i) {
-                    const uint32_t m = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(v[i]) & 0x7FFFFFFFu);
-                    if (lane == i) mine = m >> 20;
-                }
                 const int p = q0 + lane / NCH, c = lane % NCH;
-                if (lane < n && p <= S.qhi && valid) {
-                    const int e = KIND == KREC ? 2 * (p - S.out_lo) + c : p - S.out_lo + S.out_ext * c;
-                    atomicMax(le_col + (long long)S0.le_n2 * e, (int)mine);
+                const int e = KIND == KREC ? 2 * (p - S.out_lo) + c : p - S.out_lo + S.out_ext * c;
+                int *const le = le_col + (long long)S0.le_n2 * e;
+                const bool keeps = lane < n && p <= S.qhi && g0 < nlines;
+                uint32_t mask = sel;
+#pragma unroll 1
+                for (int line = 0;; ++line) {
+                    uint32_t mine = 0;
+#pragma unroll
+                    for (int i = 0; i < n; ++i) {
+                        const uint32_t m = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(v[i]) & mask);
+                        if (lane == i) mine = m >> 20;
+                    }
+                    if (keeps) atomicMax(le + line, (int)mine);
+                    if (!two || line == 1) break;
+                    mask = valid ? 0x7FFFFFFFu - sel : 0u;
                 }
             };
-            // any block: partial ones, far rows; four outputs at a time
+            // blocks of far rows, and of sweeps that hot does not take; four outputs at a time
             auto cold_block = [&](int j) {
                 const uint32_t blk = blk0 + j;
 #pragma unroll 1
@@ -980,7 +994,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                         __syncwarp();
                         if (lane == 0) bar_arrive(drained(blk & 3));
                     }
-                    if (!valid || nv <= 0) continue;
+                    if ((!hands && !valid) || nv <= 0) continue;
                     double *const ystep = yrow + yps * (q0 - S.out_lo);
                     // the outputs' values first (independent chains), then their memory side
                     double outv[4];
@@ -1017,7 +1031,10 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                             outv[i] = f32_to_f64(__float_as_uint(f));
                         }
                     }
-                    if (hands) hand_on(outv, q0, std::integral_constant<int, 4>());
+                    if (hands) {
+                        hand_on(outv, q0, std::integral_constant<int, 4>());
+                        if (!valid) continue;
+                    }
                     double *yq = ystep;
                     if (plain) {
                         if (SCH != SCH_EXACT && kMayX2 && x2) {
@@ -1075,9 +1092,12 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             // the common case, a whole block of a plain sweep: one tight loop of straight
             // runs of eight outputs, so that recombination, conversion (the narrow
             // FP64 pipe) and stores of neighbouring outputs overlap
+            constexpr std::integral_constant<int, RUN_VEC> vec_run{};
+            constexpr std::integral_constant<int, RUN_ANY> any_run{};
+            constexpr std::integral_constant<int, RUN_PART> last_run{};
             auto full_block = [&](int j) { return j < nb && qs + (j + 1) * PB - 1 <= S.qhi; };
-            auto hot_block = [&](auto VEC, int j) {
-                constexpr bool kHands = FORM == FORM_HAND, kVec = decltype(VEC)::value;
+            auto hot_block = [&](auto MODE, int j) {
+                constexpr bool kHands = hands, kVec = MODE.value == RUN_VEC;
                 const uint32_t blk = blk0 + j;
                 double *yb = yrow + yps * (qs + j * PB - S.out_lo);
                 const uint32_t ta = tmem + ((uint32_t)(lq * 32) << 16) + (blk & 3) * G::SLOT_COLS;
@@ -1140,13 +1160,17 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             // sweep with partial sums, 32 x 128^3, 580 us at eight, 485 at four, 515
             // with operands two steps ahead).  Kinetic sweeps with energies (and a_y),
             // 110^3 x 8, went through cold_block before: 213-349 us, now 164-199
+            // a partial block in the same loop pays where the general block would have
+            // the more to do (110^3 x 8 with energies: 3 % of the Hamiltonian), not
+            // for partial sums alone (its code costs 32 x 128^3 2 %)
+            constexpr bool kPartial = FORM == FORM_ANY;
             const bool want_dot = !BATCH && FORM == FORM_ANY && S.has_dot;
             const bool want_x = FORM == FORM_ANY && (want_dot || S.has_ax), want_y = FORM == FORM_ANY && S.ay_mode != 0;
             double ta[4], tx[4], ty[4];                  // the next four outputs' x2, x and y
-            auto load_terms = [&](auto VEC, int q) {
+            auto load_terms = [&](auto MODE, int q) {
                 if (!valid) return;
                 auto run = [&](double (&d)[4], const double *p, long long st) {
-                    if constexpr (decltype(VEC)::value) {
+                    if constexpr (MODE.value == RUN_VEC) {
                         long long b0, b1, b2, b3;
                         ld256(reinterpret_cast<const long long *>(p), b0, b1, b2, b3);
                         d[0] = __longlong_as_double(b0), d[1] = __longlong_as_double(b1);
@@ -1154,7 +1178,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     } else {
 #pragma unroll
                         for (int n = 0; n < 4; ++n) {
-                            d[n] = *p;
+                            if (MODE.value != RUN_PART || q + n <= S.qhi) d[n] = *p;
                             p += st;
                         }
                     }
@@ -1163,12 +1187,13 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 if (want_x) run(tx, xrow + (long long)S.nL * (q - S.in_lo), S.nL);
                 if (want_y) run(ty, yrow + yps * (q - S.out_lo), yps);
             };
-            auto term_block = [&](auto VEC, int j) {
-                constexpr bool kVec = decltype(VEC)::value;
+            auto term_block = [&](auto MODE, int j) {
+                constexpr bool kVec = MODE.value == RUN_VEC, kPart = MODE.value == RUN_PART;
                 const uint32_t blk = blk0 + j;
                 const int q0 = qs + j * PB;
                 const uint32_t tb = tmem + ((uint32_t)(lq * 32) << 16) + (blk & 3) * G::SLOT_COLS;
-                const bool more = full_block(j + 2);
+                const bool more = full_block(j + 2), part = !more && j + 2 < nb;
+                int nv = kPart ? S.qhi - q0 + 1 : 16;            // outputs left
                 if (more && valid) {                     // the group's next block on its way to L2
                     const int q = q0 + 2 * PB + (lane & 15);
                     if (x2) prefetch_l2(x2row + x2s * (q - x2lo));
@@ -1210,7 +1235,8 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     if (want_x) {
                         if (want_dot && valid) {
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) dot = fma(tx[i], v[i], dot);
+                            for (int i = 0; i < 4; ++i)
+                                if (!kPart || i < nv) dot = fma(tx[i], v[i], dot);
                         }
                         if (S.has_ax) {
 #pragma unroll
@@ -1226,8 +1252,9 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
 #pragma unroll
                         for (int i = 0; i < 4; ++i) v[i] = fma(ay, ty[i], v[i]);
                     }
-                    if (st < 3) load_terms(VEC, q0 + 4 * st + 4);
-                    else if (more) load_terms(VEC, q0 + 2 * PB);
+                    if (st < 3) load_terms(MODE, q0 + 4 * st + 4);
+                    else if (more) load_terms(MODE, q0 + 2 * PB);
+                    else if (kPartial && part) load_terms(last_run, q0 + 2 * PB);
                     if (valid) {
                         if (kVec) {
                             st256(yb, v[0], v[1], v[2], v[3]);
@@ -1235,9 +1262,18 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                             double *yp = yb;
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
-                                *yp = v[i];
+                                if (!kPart || i < nv) *yp = v[i];
                                 yp += yps;
                             }
+                        }
+                    }
+                    if (kPart) {
+                        nv -= 4;
+                        if (nv <= 0 && st < 3) {         // the rest of the block is not there
+                            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                            __syncwarp();
+                            if (lane == 0) bar_arrive(drained(blk & 3));
+                            break;
                         }
                     }
                     yb += 4 * yps;
@@ -1254,12 +1290,11 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             const bool tvec = vec && (!x2 || unit(x2row + x2s * (qs - x2lo), x2s)) &&
                               (!want_x || unit(xrow + (long long)S.nL * (qs - S.in_lo), S.nL));
             const bool vecs = __all_sync(0xffffffffu, (kTerms ? tvec : vec) || !valid);
-            const std::true_type yes{};
-            const std::false_type no{};
             if constexpr (kTerms)
-                if (hot && full_block(j0)) {
-                    if (vecs) load_terms(yes, qs + j0 * PB);
-                    else load_terms(no, qs + j0 * PB);
+                if (hot && j0 < nb) {
+                    if (!full_block(j0)) { if (kPartial) load_terms(last_run, qs + j0 * PB); }
+                    else if (vecs) load_terms(vec_run, qs + j0 * PB);
+                    else load_terms(any_run, qs + j0 * PB);
                 }
 #pragma unroll 1
             for (int j = j0; j < nb; j += 2) {
@@ -1269,15 +1304,16 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 // an earlier one, so their phase is known to be over
                 if (!bar_wait(tfull(blk & 3), (blk >> 2) & 1) || !issue_next()) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                if (!hot || !full_block(j)) {
+                if (!hot || (!kPartial && !full_block(j))) {
                     cold_block(j);
                 } else if constexpr (kTerms) {
-                    if (vecs) term_block(yes, j);
-                    else term_block(no, j);
+                    if (kPartial && !full_block(j)) term_block(last_run, j);
+                    else if (vecs) term_block(vec_run, j);
+                    else term_block(any_run, j);
                 } else if (vecs) {
-                    hot_block(yes, j);
+                    hot_block(vec_run, j);
                 } else {
-                    hot_block(no, j);
+                    hot_block(any_run, j);
                 }
             }
         }
@@ -1334,7 +1370,12 @@ cudaError_t launch(const Sweep &S_in, const TcFilter &F, int *status, const int 
     if constexpr (KIND == KCONV && NT == 29)
         if (S.x2) return launch_form<KIND, NT, SCH, FORM_X2>(S, F, status, lineE, st);
     if constexpr (SCH == SCH_EXACT && (KIND != KCONV || NT == 16))
-        if (S.le_next) return launch_form<KIND, NT, SCH, FORM_HAND>(S, F, status, lineE, st);
+        if (S.le_next) {
+            // 32 x 128^3: a sweep that hands on takes 338 us as HAND, 346 as HAND2
+            if (S.le_n1 % 32 == 0 && (long long)S.nL * S.nR % 32 == 0)
+                return launch_form<KIND, NT, SCH, FORM_HAND>(S, F, status, lineE, st);
+            return launch_form<KIND, NT, SCH, FORM_HAND2>(S, F, status, lineE, st);
+        }
     return launch_form<KIND, NT, SCH, FORM_PLAIN>(S, F, status, lineE, st);
 }
 

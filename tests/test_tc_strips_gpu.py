@@ -65,9 +65,9 @@ def test_lines_of_every_length(pkg, O, op, n):
 
 
 # line counts and lengths that are multiples of 32 (a warp's rows lie in one line of the
-# next sweep), and one extent that is not (pre-pass instead)
+# next sweep), that are not (in one or two), and lengths below 32 (pre-pass instead)
 @pytest.mark.parametrize('bcs', [[0, 0, 0], [2, 2, 2], [1, 0, 2], [0, 2, 1], [-1, -1, -1]])
-@pytest.mark.parametrize('n', [[32, 32, 32], [64, 32, 96], [96, 160, 32], [48, 32, 64]])
+@pytest.mark.parametrize('n', [[32, 32, 32], [64, 32, 96], [96, 160, 32], [48, 32, 64], [34, 46, 66], [32, 24, 130], [62, 64, 34]])
 @pytest.mark.parametrize('op', ['magicfilter', 'd_dwt_sym8', 'd_idwt_sym8'])
 def test_handed_on_exponents(pkg, op, n, bcs):
     """The 3D operator, whose sweeps hand on line exponents, gives the bits of three 1D calls."""
