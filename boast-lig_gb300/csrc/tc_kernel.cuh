@@ -543,28 +543,38 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    // Toeplitz filter tiles B_t[n][kk], K-major core matrices
-    for (int idx = tid; idx < G::ORD * 16 * G::KBP; idx += kThreads) {
-        const int t = idx / (16 * G::KBP), rem = idx % (16 * G::KBP);
-        const int n = rem / G::KBP, k2 = rem % G::KBP;
-        // K index k2 = element kk, data plane pj within the slice: the pair
-        // (slice plane pj, filter digit t - pj) lands on order column t
-        const int kk = k2 / G::PL, pj = k2 % G::PL;
-        const int ti = kk / NCH - n / NCH - woff;
-        const uint32_t v = (ti >= 0 && ti < NT && t >= pj)
-                               ? F.dig[t - pj][filter_index<KIND>(n % NCH, kk % NCH) * NT + ti] : 0u;
-        const int row = 16 * t + n;                      // stacked filter planes
-        uint8_t *b = B + (k2 / G::CE) * G::LBO_B + (row >> 3) * 128 + (row & 7) * 16 +
-                     (k2 % G::CE) * G::ESZ;
-        if (G::ESZ == 4) *(uint32_t *)b = v;
-        else *(unsigned short *)b = (unsigned short)v;
+    // Toeplitz filter tiles B_t[n][kk], K-major core matrices, a 16-byte row of one
+    // per thread and step.  The filter's digits come through shared memory (the
+    // operand ring, not in use yet): read where they are, in the parameters, a
+    // warp's 32 addresses take turns.  A launch of a few blocks is mostly this
+    // prologue: MagicFilter3D of one 32^3 grid 39 us, element by element from the
+    // parameters 50
+    static_assert(TcFilter::kSlices * TcFilter::kMaxTaps == 4 * 128, "digit table");
+    uint32_t *const dig = (uint32_t *)A;
+    if (tid < 128) ((uint4 *)dig)[tid] = ((const uint4 *)F.dig)[tid];
+    __syncthreads();
+    for (int idx = tid; idx < G::ORD * 16 * (G::KBP / G::CE); idx += kThreads) {
+        const int row = idx % (G::ORD * 16), kc = idx / (G::ORD * 16);
+        const int t = row / 16, n = row % 16;            // stacked filter planes
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int e = 0; e < G::CE; ++e) {
+            // K index k2 = element kk, data plane pj within the slice: the pair
+            // (slice plane pj, filter digit t - pj) lands on order column t
+            const int k2 = kc * G::CE + e, kk = k2 / G::PL, pj = k2 % G::PL;
+            const int ti = kk / NCH - n / NCH - woff;
+            const uint32_t v = (ti >= 0 && ti < NT && t >= pj)
+                                   ? dig[(t - pj) * TcFilter::kMaxTaps + filter_index<KIND>(n % NCH, kk % NCH) * NT + ti]
+                                   : 0u;
+            if (G::ESZ == 4) w[e % 4] = v;
+            else w[e / 2] |= (v & 0xFFFFu) << (16 * (e & 1));
+        }
+        sts128(saddr(B) + kc * G::LBO_B + (row >> 3) * 128 + (row & 7) * 16, w[0], w[1], w[2], w[3]);
     }
     // bias tile, K-major core matrices like A: (row, k) at (k / 8) * 2048 +
-    // (row / 8) * 128 + (row % 8) * 16 + (k % 8) * 2; FP16 8 = 0x4800
-    for (int idx = tid; idx < G::Z_BYTES / 2; idx += kThreads) {
-        const int k8 = idx / 1024, rem = idx % 1024, k = rem % 8;
-        ((unsigned short *)Z)[idx] = (k8 == 0 && k < 3) ? (unsigned short)0x4800 : (unsigned short)0;
-    }
+    // (row / 8) * 128 + (row % 8) * 16 + (k % 8) * 2; FP16 8 = 0x4800 at k < 3
+    for (int idx = tid; idx < G::Z_BYTES / 16; idx += kThreads)
+        sts128(saddr(Z) + 16 * idx, idx < kM ? 0x48004800u : 0u, idx < kM ? 0x4800u : 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
