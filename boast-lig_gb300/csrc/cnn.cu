@@ -425,13 +425,29 @@ __device__ __forceinline__ void stage(const ConvArgs &A, uint8_t *halo, int s, i
     const int n = A.n;
     const long long base = (long long)s * n * n * n;
     if (SRC == SRC_ACT) {
-        const uint32_t hb = saddr(halo);
-        for (int idx = threadIdx.x; idx < 2 * G::HPTS; idx += kThreads) {
-            const int i = idx >> 1, c = idx & 1;
-            const int hx = i % kHX, hy = (i / kHX) % kHY, hz = i / (kHX * kHY);
-            const int gx = wrap(x0 + hx, n), gy = wrap(y0 + hy, n), gz = wrap(z0 + hz, n);
-            const long long p = base + gx + (long long)n * (gy + (long long)n * gz);
-            cp_async16(hb + c * G::PLANE + i * 16, A.src_act + p * 16 + c * 8);
+        // a thread keeps its 16-byte piece of a row (x, channel chunk) and steps
+        // through the rows, kRows at a time: a dozen instructions a copy (64 grids of
+        // 48^3: 184 us, 189 with every copy's point worked out from its number)
+        constexpr int kRow = 2 * kHX, kRows = kThreads / kRow;
+        static_assert(kRows < kHY, "one row wrap a step");
+        const int piece = threadIdx.x % kRow, r0 = threadIdx.x / kRow;
+        if (r0 < kRows) {
+            const int hx = piece >> 1, c = piece & 1;
+            uint32_t dst = saddr(halo) + c * G::PLANE + r0 * kRowB + hx * 16;
+            const __nv_bfloat16 *src =
+                reinterpret_cast<const __nv_bfloat16 *>(A.src_act) + (base + wrap(x0 + hx, n)) * 16 + c * 8;
+            int hy = r0, gz = wrap(z0, n);
+#pragma unroll 4
+            for (int row = r0; row < kHY * G::HZ; row += kRows) {
+                const int gy = wrap(y0 + hy, n);
+                cp_async16(dst, src + (long long)(gz * n + gy) * n * 16);
+                dst += kRows * kRowB;
+                hy += kRows;
+                if (hy >= kHY) {
+                    hy -= kHY;
+                    if (++gz == n) gz = 0;
+                }
+            }
         }
         asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;\n" ::: "memory");
     } else {
@@ -450,29 +466,31 @@ __device__ __forceinline__ void stage(const ConvArgs &A, uint8_t *halo, int s, i
     }
 }
 
-// The MMAs of one tile (thread 0).
+// The MMAs of one tile (thread 0).  One thread issues some 94 of them, so what
+// it computes in between sets their pace: descriptors are formed once and
+// advanced by adding to their start address field (16-byte units).  Formed anew
+// for each MMA, 64 grids of 48^3 took 199 us, so 189.  What is left is about 64
+// cycles an MMA on the tensor pipe, whatever N and the alignment of A (143 us for
+// that layer), behind the staging and drain of three CTAs a SM.
 template <int TZ>
 __device__ __forceinline__ void issue_tile(uint32_t tmem, uint32_t hb, uint32_t wb) {
     using G = Geo<TZ>;
+    const uint64_t a0 = sdesc(hb, G::PLANE, kRowB), b0 = sdesc(wb, 768, 128);
 #pragma unroll 1
     for (int h = 0; h < TZ + 2; ++h) {
         const int dmax = h < 2 ? h : 2, dmin = h > TZ - 1 ? h - (TZ - 1) : 0;
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            const int dx = j % 3, dy = j / 3;
-            const uint64_t a = sdesc(hb + (h * kHY + dy) * kRowB + dx * 16, G::PLANE, kRowB);
-            const uint32_t bj = wb + j * kJB;
-            if (j == 0 && h < TZ) {
-                // output plane h opens here (tap dz = 0, stack rows 32..47)
-                mma(tmem + 16 * h, a, sdesc(bj + 32 * 16, 768, 128), idesc(16), 0u);
-                if (dmax > 0)
-                    mma(tmem + 16 * (h - dmax), a, sdesc(bj + 16 * (2 - dmax) * 16, 768, 128),
-                        idesc(16 * dmax), 1u);
-            } else {
-                mma(tmem + 16 * (h - dmax), a, sdesc(bj + 16 * (2 - dmax) * 16, 768, 128),
-                    idesc(16 * (dmax - dmin + 1)), 1u);
-            }
+        const uint64_t ah = a0 + (uint32_t)(h * kHY * (kRowB / 16)), bh = b0 + (uint32_t)(16 * (2 - dmax));
+        const uint32_t d = tmem + 16 * (h - dmax), id = idesc(16 * (dmax - dmin + 1));
+        if (h < TZ) {
+            // output plane h opens here (tap dz = 0, stack rows 32..47)
+            mma(tmem + 16 * h, ah, b0 + 32u, idesc(16), 0u);
+            if (dmax > 0) mma(d, ah, bh, idesc(16 * dmax), 1u);
+        } else {
+            mma(d, ah, bh, id, 1u);
         }
+#pragma unroll
+        for (int j = 1; j < 9; ++j)
+            mma(d, ah + (uint32_t)((j / 3) * (kRowB / 16) + j % 3), bh + (uint32_t)(j * (kJB / 16)), id, 1u);
     }
 }
 
