@@ -8,6 +8,7 @@
 // reads are conflict-free and the stores of strided shapes and of the
 // rotated (transpose = 1) layout are coalesced.
 #include "lcg_sweep.cuh"
+#include "lcg_tc.cuh"
 #include "libconv_filters.h"
 
 namespace lcg {
@@ -21,31 +22,9 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kPad = kLines + 1;
 
-template <int KIND> struct Chunk { static constexpr int QC = KIND == KCONV ? 64 : 32; };
-
 __device__ __forceinline__ int imod(int a, int n) {
     int r = a % n;
     return r < 0 ? r + n : r;
-}
-
-// Input element of line g at logical processed index p (channel ch), with the
-// boundary condition applied; 0 outside the data of a free boundary.
-template <int KIND>
-__device__ __forceinline__ double fetch(const Sweep &S, const double *__restrict__ x, long long g,
-                                        int p, int ch, long long in_pext) {
-    int pos;
-    if (S.bc == BC_PERIODIC) {
-        pos = imod(p, S.n);
-    } else if (S.bc == BC_SHRINK) {
-        pos = p - S.in_lo;
-    } else {
-        if (p < 0 || p >= S.n) return 0.0;
-        pos = p;
-    }
-    const long long l = g % S.nL, r = g / S.nL;
-    const long long off = KIND == KDEC ? (long long)ch + 2LL * pos
-                                       : (long long)pos + (long long)S.in_ext * ch;
-    return x[l + (long long)S.nL * (off + in_pext * r)];
 }
 
 // One block of the sweep: lines [bx*32, bx*32+32) x output chunk by of array
@@ -60,6 +39,10 @@ __device__ __forceinline__ void sweep_block(const Sweep &S, long long bx, int by
     const int arr = bz;
     const long long nlines = (long long)S.nL * S.nR;
     const long long g0 = bx * kLines;
+    // this thread's line (fewer than 2^31 of them: 32-bit division)
+    const int w = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    const long long g = g0 + w;
+    const long long r = S.nL == 1 ? g : (long long)((uint32_t)g / (uint32_t)S.nL), l = g - r * S.nL;
     const int qc0 = S.qlo + by * QC;
     const int upfil = S.lowfil + NT - 1;
     const int plast = S.qhi + upfil;  // last logical input index any output needs
@@ -69,7 +52,24 @@ __device__ __forceinline__ void sweep_block(const Sweep &S, long long bx, int by
     double *__restrict__ y = S.y + (long long)arr * S.y_arr;
     const double *__restrict__ x2 = S.x2 ? S.x2 + (long long)arr * S.x_arr : nullptr;
 
-    // ---- stage the input segment: row j*NCH+ch holds logical index qc0+lowfil+j
+    // ---- stage the input segment: row j*NCH+ch holds logical index qc0+lowfil+j,
+    // with the boundary condition applied (0 outside the data of a free
+    // boundary).  No division per element: the window's start is wrapped once and
+    // a line is located once per thread (strided) or by its number (contiguous);
+    // kinetic 3D of eight 64^3 grids 383 -> 365 us, the FMAs alone take 316
+    const int p0 = qc0 + S.lowfil, n = S.n, bc = S.bc;
+    const int s0 = bc == BC_PERIODIC ? imod(p0, n) : bc == BC_SHRINK ? p0 - S.in_lo : p0;
+    auto fetch = [&](const double *__restrict__ line, int j, int ch) -> double {
+        int pos = s0 + j;
+        if (bc == BC_PERIODIC) {
+            if (n >= SPAN) pos -= pos >= n ? n : 0;
+            else pos %= n;
+        } else if (bc != BC_SHRINK && (pos < 0 || pos >= n)) {
+            return 0.0;
+        }
+        const long long off = KIND == KDEC ? (long long)ch + 2LL * pos : (long long)pos + (long long)S.in_ext * ch;
+        return line[(long long)S.nL * off];
+    };
     if (S.nL == 1) {
         // positions fastest: consecutive threads read consecutive memory of one line
         for (int idx = threadIdx.x; idx < NROW * kLines; idx += kThreads) {
@@ -79,29 +79,22 @@ __device__ __forceinline__ void sweep_block(const Sweep &S, long long bx, int by
             } else {                     // conv / interleaved input
                 const int k = idx % NROW; w = idx / NROW; j = k / NCH; ch = k % NCH;
             }
-            const long long g = g0 + w;
-            const int p = qc0 + S.lowfil + j;
             double v = 0.0;
-            if (g < nlines && p <= plast) v = fetch<KIND>(S, x, g, p, ch, in_pext);
+            if (g0 + w < nlines && p0 + j <= plast) v = fetch(x + in_pext * (g0 + w), j, ch);
             tile[(j * NCH + ch) * kPad + w] = v;
         }
     } else {
         // lines fastest: consecutive threads read consecutive l of one position
-        for (int idx = threadIdx.x; idx < NROW * kLines; idx += kThreads) {
-            const int w = idx % kLines, k = idx / kLines;
+        const double *const line = x + l + (long long)S.nL * in_pext * r;
+        for (int k = wi; k < NROW; k += kWarps) {
             const int j = k / NCH, ch = k % NCH;
-            const long long g = g0 + w;
-            const int p = qc0 + S.lowfil + j;
             double v = 0.0;
-            if (g < nlines && p <= plast) v = fetch<KIND>(S, x, g, p, ch, in_pext);
+            if (g < nlines && p0 + j <= plast) v = fetch(line, j, ch);
             tile[k * kPad + w] = v;
         }
     }
     __syncthreads();
 
-    const int w = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    const long long g = g0 + w;
-    const long long l = g % S.nL, r = g / S.nL;
     const double *f = c_ftab + S.ftab;
     double dot = 0.0;
     if (g < nlines) {
@@ -231,14 +224,30 @@ __global__ void dot_reduce_kernel(const double *__restrict__ part, long long cou
     if (threadIdx.x == 0) *out = accumulate ? *out + red[0] : red[0];
 }
 
-template <int KIND, int NT, int QC = Chunk<KIND>::QC>
-cudaError_t launch_t(const Sweep &S, cudaStream_t st) {
+template <int KIND, int NT, int QC>
+cudaError_t launch_qc(const Sweep &S, cudaStream_t st) {
     const long long nlines = (long long)S.nL * S.nR;
     const int nq = S.qhi - S.qlo + 1;
     dim3 grid((unsigned)((nlines + kLines - 1) / kLines), (unsigned)((nq + QC - 1) / QC),
               (unsigned)S.narr);
     sweep_fp64_kernel<KIND, NT, QC><<<grid, kThreads, 0, st>>>(S);
     return cudaGetLastError();
+}
+
+// Positions per block: chunks of 64 elements; 8 positions when those would give
+// fewer than two blocks per SM.  Few blocks leave SMs idle and run through chains
+// of dependent FMAs with two warps a scheduler; chunks of 8 read their halo more
+// often instead.  Kinetic 3D, 64 / 8: one 40^3 grid 52 / 31 us, 64^3 72 / 64 (128
+// blocks of 64), eight 64^3 365 / 384 (1024 blocks).
+int fp64_chunk(const Sweep &S) {
+    const int qc = S.kind == KCONV ? 64 : 32;
+    return blocks_of(S, qc) < 2LL * tck::sm_count() ? 8 : qc;
+}
+
+template <int KIND, int NT>
+cudaError_t launch_t(const Sweep &S, cudaStream_t st) {
+    constexpr int QC = KIND == KCONV ? 64 : 32;
+    return fp64_chunk(S) == QC ? launch_qc<KIND, NT, QC>(S, st) : launch_qc<KIND, NT, 8>(S, st);
 }
 
 template <int KIND, int NT, int QC>
@@ -284,10 +293,7 @@ cudaError_t launch_batch_qc(int kind, int ntaps, const Sweep *descs, const long 
 }  // namespace
 
 long long sweep_fp64_blocks(const Sweep &S) {
-    const long long nlines = (long long)S.nL * S.nR;
-    const int qc = S.kind == KCONV ? Chunk<KCONV>::QC : Chunk<KDEC>::QC;
-    const long long nq = S.qhi - S.qlo + 1;
-    return ((nlines + kLines - 1) / kLines) * ((nq + qc - 1) / qc) * S.narr;
+    return blocks_of(S, fp64_chunk(S));
 }
 
 cudaError_t launch_sweep_fp64(const Sweep &S, cudaStream_t st) {
