@@ -493,6 +493,25 @@ int host_scratch(const Plan &P, DevBuf &dot, DevBuf &le, Scratch &sc) {
     return LIBCONV_OK;
 }
 
+// Arrays of contiguous lines that lie back to back are more lines of one array.
+// A sweep's blocks (32 or 128 lines) do not reach across arrays, so 1024 arrays of
+// one line of 32 left 31 of 32 lanes idle: 41 us as arrays, 9 us as lines.
+// Line numbers over all arrays, and with them line exponents, stay what they
+// were.  Not with what is kept per array: dot products, active flags; nor with
+// a partial sum, whose lines may have another pitch.
+void fold_arrays(Sweep &S) {
+    const long long m = S.kind == KCONV ? 1 : 2, lines = (long long)S.nR * S.narr;
+    if (S.narr < 2 || S.nL != 1 || S.has_dot || S.active || S.x2 || S.le_next || lines > (1LL << 31) - 1 ||
+        S.x_arr != (long long)S.in_ext * m * S.nR || S.y_arr != (long long)S.out_ext * m * S.nR)
+        return;
+    if (S.transpose && S.nR != 1) return;       // lines of one array interleave in its output
+    S.transpose = 0;
+    S.nR = (int)lines;
+    S.x_arr *= S.narr;
+    S.y_arr *= S.narr;
+    S.narr = 1;
+}
+
 // Launch the plan's sweeps with bound device pointers.  dot_dev receives the
 // dot product (device) when the plan has one; the partials and line
 // exponents live in sc (at least plan_scratch's sizes).
@@ -538,6 +557,7 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
         S.x2 = ps.src2 >= 0 ? bufs[ps.src2] : nullptr;
         if (!S.x || !S.y || (ps.src2 >= 0 && !S.x2))
             return fail(LIBCONV_EARG, "null device buffer in plan");
+        fold_arrays(S);
         const bool tc = t_mode != LIBCONV_MODE_FP64 && sweep_tc_supported(S);
         long long nb = 0, seg = 0;   // dot partials: total, and per array (array-major)
         if (S.has_dot) {

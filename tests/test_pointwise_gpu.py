@@ -36,3 +36,26 @@ def test_potential_step_orbital_groups(pkg, norb):
         hj, ek, ep = pkg.hamiltonian(n, bc, a, psig[j * nsig:(j + 1) * nsig].copy(), pot)
         assert ep == en[j, 3]
         assert np.array_equal(hj, h[j * nsig:(j + 1) * nsig])
+
+
+@pytest.mark.parametrize('mode', ['fp64', 'tc_exact'])
+@pytest.mark.parametrize('op', ['d_s0s0_1d_sym8_md', 'd_s0s0_1d_sym8_d1', 'd_s0s1_1d_sym8', 'd_s1s0_1d_sym8'])
+def test_arrays_of_lines_are_one_array(pkg, op, mode):
+    """Contiguous sweeps over several arrays, padded leading dimensions included: the bits of one
+    call per array.  FP64 sweeps also at the sizes around the smaller chunks (8 positions)."""
+    wav = op in ('d_s0s1_1d_sym8', 'd_s1s0_1d_sym8')
+    m, taps = (2, 8) if wav else (1, 29 if op.endswith('d1') else 16)
+    with pkg.mode(pkg.MODE_FP64 if mode == 'fp64' else pkg.MODE_TC_EXACT):
+        K = pkg.Kernel(op)
+        for n, rows, narr, bc, pad in ((7, 1, 5, 0, 0), (9, 3, 40, 1, 2), (65, 2, 3, -1, 1), (8, 4, 130, 2, 0)):
+            nx, ny = n + (taps - 1) * (bc == -1) + pad, n + (taps - 1) * (bc == 1) + pad
+            sx, sy = nx * rows * m * m, ny * rows * m * m
+            r = np.random.default_rng(n)
+            x, y = r.uniform(-1, 1, narr * sx), r.uniform(-1, 1, narr * sy)
+            one = y.copy()
+            tail = (0.7, 1.5) if wav else (0.7, -0.3, 1.5)
+            K.run(2, 0, [n, rows], bc, [nx, rows], [ny, rows], narr, x, y, *tail)
+            for j in range(narr):
+                yj = one[j * sy:(j + 1) * sy].copy()
+                K.run(2, 0, [n, rows], bc, [nx, rows], [ny, rows], 1, x[j * sx:(j + 1) * sx].copy(), yj, *tail)
+                assert np.array_equal(y[j * sy:(j + 1) * sy], yj), (n, bc, j)
