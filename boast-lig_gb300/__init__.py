@@ -149,8 +149,12 @@ def set_mode(mode):
 def _ints(v):
     if v is None:
         return None
-    v = [int(t) for t in (v if hasattr(v, '__len__') else [v])]
-    return (ctypes.c_int * len(v))(*v)
+    if type(v) is not list:
+        v = list(v) if hasattr(v, '__len__') else [v]
+    try:
+        return (ctypes.c_int * len(v))(*v)
+    except TypeError:                            # numbers that are no integers by type
+        return (ctypes.c_int * len(v))(*[int(t) for t in v])
 
 
 def _host_ptr(a, writable):
@@ -165,16 +169,38 @@ def _host_ptr(a, writable):
     return ctypes.c_void_p(a.ctypes.data)
 
 
-def _dev_ptr(t):
-    if t is None:
-        return None
-    if isinstance(t, int):
-        return ctypes.c_void_p(t)
+_float64 = None                                  # torch.float64, once a tensor has been seen
+
+
+def _dev_addr(t):
+    """Address of a device array (for parameters declared void *)."""
+    global _float64
+    if t is None or isinstance(t, int):
+        return t
     if hasattr(t, 'data_ptr'):
-        if not t.is_cuda or str(t.dtype) != 'torch.float64' or not t.is_contiguous():
+        d = t.dtype
+        if d is not _float64:
+            if str(d) != 'torch.float64':
+                raise TypeError('device arrays must be contiguous float64 CUDA tensors')
+            _float64 = d
+        if not t.is_cuda or not t.is_contiguous():
             raise TypeError('device arrays must be contiguous float64 CUDA tensors')
-        return ctypes.c_void_p(t.data_ptr())
+        return t.data_ptr()
     raise TypeError(f'unsupported device array {type(t)}')
+
+
+def _dev_ptr(t):
+    a = _dev_addr(t)
+    return None if a is None else ctypes.c_void_p(a)
+
+
+def _same(v):
+    return v
+
+
+def _doubles(v):
+    vals = [float(t) for t in v]
+    return ctypes.cast((ctypes.c_double * len(vals))(*vals), _D)
 
 
 class Kernel:
@@ -188,6 +214,9 @@ class Kernel:
         L = lib()
         self._host = getattr(L, name)
         self._dev = getattr(L, name + '_dev')
+        # how run_dev passes each argument; small calls are bound by this path (one
+        # 32^3 sweep: 9 us a call, 11 deciding it anew each time)
+        self._dev_conv = [{_I: _ints, _D: _doubles, _vp: _dev_addr}.get(t, _same) for t in self.argtypes]
 
     def _convert(self, args, ptr):
         if len(args) != len(self.argtypes):
@@ -197,8 +226,7 @@ class Kernel:
             if t is _I:
                 out.append(_ints(a))
             elif t is _D:
-                vals = [float(v) for v in a]
-                out.append(ctypes.cast((ctypes.c_double * len(vals))(*vals), _D))
+                out.append(_doubles(a))
             elif t is _vp:
                 if self.name.endswith('dotin') and i == len(self.argtypes) - 1:
                     dot = a
@@ -225,13 +253,13 @@ class Kernel:
 
     def run_dev(self, *args, stream=None):
         """Device-pointer call (enqueue only); dot_in is a device pointer."""
-        conv, dot = self._convert(args, _dev_ptr)
-        if self.name.endswith('dotin'):
-            conv[-1] = _dev_ptr(dot)
+        if len(args) != len(self._dev_conv):
+            raise TypeError(f"{self.name} takes {len(self._dev_conv)} arguments, got {len(args)}")
+        conv = [f(a) for f, a in zip(self._dev_conv, args)]
         s = stream
         if s is not None and not isinstance(s, int):
             s = s.cuda_stream if hasattr(s, 'cuda_stream') else int(s)
-        st = self._dev(*conv, ctypes.c_void_p(s) if s else None)
+        st = self._dev(*conv, s or None)
         if st:
             raise LibconvError(st, self.name + '_dev', last_error())
 
