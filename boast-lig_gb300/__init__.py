@@ -369,10 +369,10 @@ class Hamiltonian:
         self.energies = torch.zeros(self.norb, 4, dtype=torch.float64, device=device)
 
     # kernel launches of one call on free boundaries: 15 sweeps, the potential
-    # kernel and its reduction, and the three kinetic-energy reductions; in the
+    # kernel and its reduction, and that of the three kinetic energies; in the
     # exact tensor-core mode also five line-exponent passes, one per operator
     # (its sweeps hand on theirs; grids below 32 points an axis take more)
-    LAUNCHES = {'exact': 25, 'other': 20}
+    LAUNCHES = {'exact': 23, 'other': 18}
 
     def __call__(self, psig, pot, hpsig, rho=None, stream=None, energies=None):
         """energies: optional device tensor of norb * 4 doubles to receive the

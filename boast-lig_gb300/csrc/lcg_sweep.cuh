@@ -53,6 +53,10 @@ struct Sweep {
     int *le_next = nullptr;
     long long le_next_lines = 0;
     int le_n1 = 0, le_n2 = 0;
+    // zeroed by the sweep (exact tensor-core): the exponents that its successor
+    // hands on
+    int *le_zero = nullptr;
+    long long le_zero_n = 0;
 };
 
 // Number of dot partials the FP64 sweep writes for S (grid size).
@@ -74,6 +78,17 @@ cudaError_t launch_dot_reduce(const double *part, long long count, double *out, 
                               cudaStream_t st);
 // Segmented form: out[j * out_stride] = sum of part[j*seg_len .. (j+1)*seg_len)
 // for j < nseg (fixed order), on `st`.
+// The same for a plan's dot products in one launch: product i's partials are
+// part + off[i], len[i] of them for each of nseg segments, its results at
+// out[slot[i] + segment out_stride].
+constexpr int kMaxDots = 16;
+struct DotList {
+    long long off[kMaxDots], len[kMaxDots];
+    int slot[kMaxDots];
+    int n = 0;
+};
+cudaError_t launch_dot_reduce_list(const double *part, const DotList &L, int nseg, double *out,
+                                   long long out_stride, cudaStream_t st);
 cudaError_t launch_dot_reduce_seg(const double *part, long long seg_len, int nseg, double *out,
                                   long long out_stride, cudaStream_t st);
 // The m = nord/2 one-sided outputs at each end of every line of a

@@ -464,16 +464,17 @@ void plan_scratch(const Plan &P, size_t &ndot, size_t &nle) {
         const bool tc = t_mode != LIBCONV_MODE_FP64 && sweep_tc_supported(S);
         if (S.has_dot) {
             const size_t nb = tc ? (size_t)sweep_tc_blocks(S) * kTcDotSlots * S.narr : (size_t)sweep_fp64_blocks(S);
-            if (nb > ndot) ndot = nb;
+            ndot += nb;                      // one reduction at the plan's end
         }
         const bool shared = exact && P.exp3[0] > 0 && ps.exp_axis >= 0 && ps.src == B_X;
         if (tc && exact && !shared && (size_t)sweep_tc_lines(S) > nle) nle = (size_t)sweep_tc_lines(S);
     }
-    // a hand-off writes the next step's exponents beside the ones being read
+    // a hand-off writes the next step's exponents beside the ones being read and
+    // zeroes those of the step after
     int n1, n2;
     for (size_t k = 0; k + 1 < P.steps.size(); ++k)
         if (!(P.exp3[0] > 0) && exp_handoff(P, k, n1, n2)) {
-            nle *= 2;
+            nle *= 3;
             break;
         }
 }
@@ -538,16 +539,20 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
         if (e != cudaSuccess) return cuda_fail(e, "line exponent launch");
     }
     if (P.active && P.has_dot) return fail(LIBCONV_EARG, "internal: active arrays with a dot product");
-    // exponents handed from step to step: the step reads le_cur (ready when the
-    // previous step wrote it) and writes its successor's into the other half
-    int *le_cur = sc.le, *le_other = nullptr;
+    // exponents handed from step to step: the step reads le[0] (ready when the
+    // previous step wrote it), writes its successor's into le[1], which the step
+    // before it or its own pre-pass zeroed, and zeroes le[2] for the step after
+    int *le[3] = {sc.le, nullptr, nullptr};
     bool le_ready = false;
     if (!shared_exp) {
-        size_t half = 0;
+        size_t most = 0;
         for (const PlanStep &ps : P.steps)
-            if ((size_t)sweep_tc_lines(ps.S) > half) half = (size_t)sweep_tc_lines(ps.S);
-        if (sc.le && sc.nle >= 2 * half) le_other = sc.le + half;
+            if ((size_t)sweep_tc_lines(ps.S) > most) most = (size_t)sweep_tc_lines(ps.S);
+        if (sc.le && sc.nle >= 3 * most) le[1] = sc.le + most, le[2] = sc.le + 2 * most;
     }
+    // dot products: each step's partials in their own place, reduced at the end
+    DotList dots;
+    long long dot_off = 0;
     for (size_t k = 0; k < P.steps.size(); ++k) {
         const PlanStep &ps = P.steps[k];
         Sweep S = ps.S;
@@ -568,11 +573,18 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
                 nb = sweep_fp64_blocks(S);
                 seg = nb / S.narr;
             }
-            S.dot_part = sc.dot;
-            if (tc && S.narr > 1) {   // slots of arrays a CTA has no strip of stay 0
-                cudaError_t e = cudaMemsetAsync(S.dot_part, 0, (size_t)nb * sizeof(double), st);
+            if (dots.n == kMaxDots) return fail(LIBCONV_EARG, "too many dot products");
+            S.dot_part = sc.dot + dot_off;
+            if (tc && S.narr > 1 && dots.n == 0) {   // slots of arrays a CTA has no strip of stay 0
+                size_t nd, nl;
+                plan_scratch(P, nd, nl);
+                cudaError_t e = cudaMemsetAsync(S.dot_part, 0, nd * sizeof(double), st);
                 if (e != cudaSuccess) return cuda_fail(e, "clear dot partials");
             }
+            dots.off[dots.n] = dot_off;
+            dots.len[dots.n] = ps.dot_stride > 0 ? seg : nb;
+            dots.slot[dots.n++] = ps.dot_slot;
+            dot_off += nb;
         }
         cudaError_t e;
         if (tc) {
@@ -591,35 +603,40 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
                 lineE = shared_exp + exp_off[ps.exp_axis];
             } else if (sch == SCH_EXACT) {
                 if (shared_exp) return fail(LIBCONV_EARG, "plan shares line exponents but a step does not");
-                lineE = le_cur;
+                lineE = le[0];
                 ready = le_ready;
                 int n1, n2;
-                if (le_other && exp_handoff(P, k, n1, n2)) {
+                if (le[1] && exp_handoff(P, k, n1, n2)) {
                     const Sweep &B = P.steps[k + 1].S;
-                    S.le_next = le_other;
+                    S.le_next = le[1];
                     S.le_next_lines = (long long)B.nL * B.nR;
                     S.le_n1 = n1;
                     S.le_n2 = n2;
                     handed = true;
-                    e = cudaMemsetAsync(le_other, 0, (size_t)S.le_next_lines * B.narr * sizeof(int), st);
-                    if (e != cudaSuccess) return cuda_fail(e, "clear line exponents");
+                    if (exp_handoff(P, k + 1, n1, n2)) {
+                        const Sweep &C = P.steps[k + 2].S;
+                        S.le_zero = le[2];
+                        S.le_zero_n = (long long)C.nL * C.nR * C.narr;
+                    }
                 }
             }
             e = launch_sweep_tc(S, F, sch, status, lineE, st, ready);
-            if (handed) std::swap(le_cur, le_other);
+            if (handed) {
+                int *const read = le[0];
+                le[0] = le[1], le[1] = le[2], le[2] = read;
+            }
             le_ready = handed;
         } else {
             e = launch_sweep_fp64(S, st);
             le_ready = false;
         }
         if (e != cudaSuccess) return cuda_fail(e, "sweep launch");
-        if (S.has_dot) {
-            e = ps.dot_stride > 0
-                    ? launch_dot_reduce_seg(S.dot_part, seg, S.narr, dot_dev + ps.dot_slot,
-                                            ps.dot_stride, st)
-                    : launch_dot_reduce(S.dot_part, nb, dot_dev + ps.dot_slot, 0, st);
-            if (e != cudaSuccess) return cuda_fail(e, "dot reduction launch");
-        }
+    }
+    if (dots.n) {
+        const PlanStep &ps = P.steps.back();
+        const cudaError_t e = launch_dot_reduce_list(sc.dot, dots, ps.dot_stride > 0 ? ps.S.narr : 1, dot_dev,
+                                                     ps.dot_stride, st);
+        if (e != cudaSuccess) return cuda_fail(e, "dot reduction launch");
     }
     return LIBCONV_OK;
 }

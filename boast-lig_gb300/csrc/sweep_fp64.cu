@@ -208,11 +208,9 @@ sweep_fp64_batch_kernel(const Sweep *__restrict__ descs, const long long *__rest
 
 // Block b sums part[b*count .. (b+1)*count) in a fixed order into
 // out[b*out_stride] (one block per segment: per-array dot products).
-__global__ void dot_reduce_kernel(const double *__restrict__ part, long long count, double *out,
-                                  long long out_stride, int accumulate) {
+__device__ __forceinline__ void dot_reduce(const double *__restrict__ part, long long count, double *out,
+                                           int accumulate) {
     __shared__ double red[256];
-    part += (long long)blockIdx.x * count;
-    out += (long long)blockIdx.x * out_stride;
     double s = 0.0;
     for (long long i = threadIdx.x; i < count; i += blockDim.x) s += part[i];
     red[threadIdx.x] = s;
@@ -222,6 +220,18 @@ __global__ void dot_reduce_kernel(const double *__restrict__ part, long long cou
         __syncthreads();
     }
     if (threadIdx.x == 0) *out = accumulate ? *out + red[0] : red[0];
+}
+
+__global__ void dot_reduce_kernel(const double *__restrict__ part, long long count, double *out,
+                                  long long out_stride, int accumulate) {
+    dot_reduce(part + (long long)blockIdx.x * count, count, out + (long long)blockIdx.x * out_stride, accumulate);
+}
+
+__global__ void dot_reduce_list_kernel(const double *__restrict__ part, const __grid_constant__ DotList L,
+                                       double *out, long long out_stride) {
+    const int i = blockIdx.y;
+    dot_reduce(part + L.off[i] + (long long)blockIdx.x * L.len[i], L.len[i],
+               out + L.slot[i] + (long long)blockIdx.x * out_stride, 0);
 }
 
 template <int KIND, int NT, int QC>
@@ -326,6 +336,12 @@ cudaError_t launch_sweep_fp64_batch(int kind, int ntaps, int qc, const Sweep *de
 cudaError_t launch_dot_reduce(const double *part, long long count, double *out, int accumulate,
                               cudaStream_t st) {
     dot_reduce_kernel<<<1, 256, 0, st>>>(part, count, out, 0, accumulate);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_dot_reduce_list(const double *part, const DotList &L, int nseg, double *out,
+                                   long long out_stride, cudaStream_t st) {
+    dot_reduce_list_kernel<<<dim3(nseg, L.n), 256, 0, st>>>(part, L, out, out_stride);
     return cudaGetLastError();
 }
 

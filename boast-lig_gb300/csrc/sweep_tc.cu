@@ -76,6 +76,10 @@ __device__ __forceinline__ void line_exp_lines(const Sweep &S, int plen, int *ou
 }
 
 __global__ void line_exp_kernel(const Sweep S, int plen, int *out) {
+    if (S.le_next)                       // the exponents that the sweep will hand on
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < S.le_next_lines * S.narr;
+             i += (long long)gridDim.x * blockDim.x)
+            S.le_next[i] = 0;
     line_exp_lines(S, plen, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
                    (long long)gridDim.x * blockDim.x);
 }
@@ -187,10 +191,16 @@ cudaError_t launch_line_exp3(const double *x, int n0, int n1, int n2, int narr, 
     if (nseg > most) nseg = most;
     if (nseg > 65535 / narr) nseg = 65535 / narr;
     if (nseg < 1) nseg = 1;
-    cudaError_t e = cudaMemsetAsync(e0, 0, (size_t)n1 * n2 * narr * sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(e1, 0, (size_t)n0 * n2 * narr * sizeof(int), st);
-    if (e == cudaSuccess && nseg > 1)
-        e = cudaMemsetAsync(e2, 0, (size_t)n0 * n1 * narr * sizeof(int), st);
+    // one clear when the three lie back to back
+    const size_t c0 = (size_t)n1 * n2 * narr, c1 = (size_t)n0 * n2 * narr, c2 = (size_t)n0 * n1 * narr;
+    cudaError_t e;
+    if (e1 == e0 + c0 && e2 == e1 + c1) {
+        e = cudaMemsetAsync(e0, 0, (c0 + c1 + (nseg > 1 ? c2 : 0)) * sizeof(int), st);
+    } else {
+        e = cudaMemsetAsync(e0, 0, c0 * sizeof(int), st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(e1, 0, c1 * sizeof(int), st);
+        if (e == cudaSuccess && nseg > 1) e = cudaMemsetAsync(e2, 0, c2 * sizeof(int), st);
+    }
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)(narr * nseg));
     tck::line_exp3_kernel<<<grid, 256, 0, st>>>(x, n0, n1, n2, (int)nseg, e0, e1, e2, active);

@@ -543,6 +543,9 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    if (!BATCH && (FORM == FORM_HAND || FORM == FORM_HAND2) && S0.le_zero)
+        for (long long i = (long long)blockIdx.x * kThreads + tid; i < S0.le_zero_n; i += (long long)gridDim.x * kThreads)
+            S0.le_zero[i] = 0;
     // Toeplitz filter tiles B_t[n][kk], K-major core matrices, a 16-byte row of one
     // per thread and step.  The filter's digits come through shared memory (the
     // operand ring, not in use yet): read where they are, in the parameters, a
