@@ -60,6 +60,9 @@ int extents(int op_id, int d, const int *n, const int *bc, int *in, int *out, lo
 // LIBCONV_BC_NPERIODIC), y = a d/dx_idim x, or y += ... when accumulate.
 int poisson_sweep(int nord, int idim, const int *nn, int bc, double a, bool accumulate,
                   const double *x, double *y, cudaStream_t st);
+// The same along up to three axes of one grid: y[k] along idim[k].
+int poisson_sweeps(int nord, int count, const int *idim, const int *nn, const int *bc, const double *a,
+                   bool accumulate, const double *x, double *const *y, cudaStream_t st);
 // Host-pointer composition: hold library_lock(), stage in host_staging(),
 // run on its stream, then host_finish() (synchronise + device status).
 std::unique_lock<std::recursive_mutex> library_lock();

@@ -169,9 +169,11 @@ int nabla3(int geocode, const int nn[3], const double *u, double *du, int nord,
            const double *hgrids, cudaStream_t st) {
     int bc[3], rc = geocode_bc(geocode, bc);
     const long long N = (long long)nn[0] * nn[1] * nn[2];
-    for (int i = 0; i < 3 && !rc; ++i)
-        rc = poisson_sweep(nord, i, nn, bc[i], 1.0 / hgrids[i], false, u, du + i * N, st);
-    return rc;
+    if (rc) return rc;
+    const int axis[3] = {0, 1, 2};
+    const double a[3] = {1.0 / hgrids[0], 1.0 / hgrids[1], 1.0 / hgrids[2]};
+    double *const y[3] = {du, du + N, du + 2 * N};
+    return poisson_sweeps(nord, 3, axis, nn, bc, a, false, u, y, st);
 }
 
 // ---- device implementations -------------------------------------------------------
@@ -189,11 +191,11 @@ int div_u_i_impl(int geocode, int n01, int n02, int n03, const double *u, double
         return rc;
     }
     if (!work) return report(LIBCONV_EARG, "div_u_i with cc needs a work array of 5 n01 n02 n03");
-    // (component, axis) of du and of the five temporaries
-    const int comp[6] = {0, 1, 2, 1, 2, 2}, axis[6] = {0, 1, 2, 0, 0, 1};
-    for (int k = 0; k < 6 && !rc; ++k)
-        rc = poisson_sweep(nord, axis[k], nn, bc[axis[k]], a[axis[k]], false, u + comp[k] * N,
-                           k == 0 ? du : work + (k - 1) * N, st);
+    // component by component: d0 u0; d0, d1 u1; d0, d1, d2 u2
+    double *const y[3][3] = {{du}, {work + 2 * N, work}, {work + 3 * N, work + 4 * N, work + N}};
+    const int axis[3] = {0, 1, 2};
+    for (int k = 0; k < 3 && !rc; ++k)
+        rc = poisson_sweeps(nord, k + 1, axis, nn, bc, a, false, u + k * N, y[k], st);
     if (rc) return rc;
     div_cc_kernel<<<grid_for(N), kThreads, 0, st>>>(u, du, work, cc, N);
     return cuda_rc(last(), "div_u_i cc launch");
