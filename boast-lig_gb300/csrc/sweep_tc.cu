@@ -76,6 +76,7 @@ __device__ __forceinline__ void line_exp_lines(const Sweep &S, int plen, int *ou
 }
 
 __global__ void line_exp_kernel(const Sweep S, int plen, int *out) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // the sweep's prologue may begin
     if (S.le_next)                       // the exponents that the sweep will hand on
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < S.le_next_lines * S.narr;
              i += (long long)gridDim.x * blockDim.x)
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(256)
 line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg,
                  int *__restrict__ e0, int *__restrict__ e1, int *__restrict__ e2,
                  const int *__restrict__ active) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     __shared__ int ys[kExpChunk][8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int i0 = blockIdx.x * 32 + tx, i1 = blockIdx.y * 8 + ty;

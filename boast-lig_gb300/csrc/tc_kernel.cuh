@@ -525,6 +525,8 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
         return strip;
     };
 
+    // the next kernel of the stream may start its own prologue (it waits below)
+    if (!BATCH) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                          saddr(tslot)),
@@ -543,9 +545,6 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (!BATCH && (FORM == FORM_HAND || FORM == FORM_HAND2) && S0.le_zero)
-        for (long long i = (long long)blockIdx.x * kThreads + tid; i < S0.le_zero_n; i += (long long)gridDim.x * kThreads)
-            S0.le_zero[i] = 0;
     // Toeplitz filter tiles B_t[n][kk], K-major core matrices, a 16-byte row of one
     // per thread and step.  The filter's digits come through shared memory (the
     // operand ring, not in use yet): read where they are, in the parameters, a
@@ -584,6 +583,12 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
     bool alive = true;
+    // everything above touches parameters and this CTA's own memory only; from here on
+    // the work of the kernels before is complete
+    if (!BATCH) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (!BATCH && (FORM == FORM_HAND || FORM == FORM_HAND2) && S0.le_zero)
+        for (long long i = (long long)blockIdx.x * kThreads + tid; i < S0.le_zero_n; i += (long long)gridDim.x * kThreads)
+            S0.le_zero[i] = 0;
 
     if (warp < kProdWarps) {
         // ============ producers: thread = (row, half of every slab); lanes 0-15
@@ -1362,8 +1367,23 @@ cudaError_t launch_form(const Sweep &S, const TcFilter &F, int *status, const in
     using G = Geom<KIND, NT, SCH>;
     cudaError_t e = set_smem_attr<KIND, NT, SCH, false, FORM>();
     if (e != cudaSuccess) return e;
-    sweep_tc_kernel<KIND, NT, SCH, false, FORM><<<(int)sweep_tc_blocks(S), kThreads, G::SMEM, st>>>(
-        S, F, status, nullptr, nullptr, 0, lineE);
+    // The sweep may start while the kernels before it in the stream finish: its
+    // prologue (filter tiles, barriers, TMEM) needs nothing of theirs, and it waits
+    // for their completion before its first access to the caller's or the scratch
+    // memory (griddepcontrol.wait).  MagicFilter3D of one 32^3 grid 36 -> 28 us,
+    // Hamiltonian 48^3 x 8 1655 -> 1589 us
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)sweep_tc_blocks(S));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = G::SMEM;
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, sweep_tc_kernel<KIND, NT, SCH, false, FORM>, S, F, status,
+                       (const Sweep *)nullptr, (const long long *)nullptr, 0, lineE);
     return cudaGetLastError();
 }
 

@@ -59,3 +59,48 @@ def test_arrays_of_lines_are_one_array(pkg, op, mode):
                 yj = one[j * sy:(j + 1) * sy].copy()
                 K.run(2, 0, [n, rows], bc, [nx, rows], [ny, rows], 1, x[j * sx:(j + 1) * sx].copy(), yj, *tail)
                 assert np.array_equal(y[j * sy:(j + 1) * sy], yj), (n, bc, j)
+
+
+@pytest.mark.parametrize('n', [[32, 32, 32], [40, 36, 50], [20, 70, 33]])
+def test_sweeps_of_a_plan_in_order(pkg, n):
+    """Sweeps start while the kernel before them ends: repeated calls on changing inputs, without
+    a synchronisation in between and on two streams, and as a replayed capture, give the bits of
+    calls that are each waited for."""
+    import torch
+    N, narr = int(np.prod(n)), 2
+    g = torch.Generator(device='cuda').manual_seed(N)
+    xs = [torch.randn(N * narr, dtype=torch.float64, device='cuda', generator=g) * 10.0 ** (3 * k) for k in range(6)]
+    new = lambda: torch.full((N * narr,), float('nan'), dtype=torch.float64, device='cuda')  # noqa: E731
+    mf, kin = pkg.Kernel('d_sfrf_ld_narr'), pkg.Kernel('d_kin_narr')
+    w1, w2 = [new() for _ in range(2)], [new() for _ in range(2)]
+
+    def step(x, y, z, s, k):
+        mf.run_dev(3, n, [0] * 3, n, n, narr, x, y, w1[k], w2[k], stream=s)
+        kin.run_dev(3, n, [2] * 3, narr, y, z, w1[k], w2[k], [-0.5, -0.6, -0.7], 0.0, 0.0, stream=s)
+
+    with pkg.mode(pkg.MODE_TC_EXACT):
+        ref = []
+        for x in xs:
+            y, z = new(), new()
+            step(x, y, z, None, 0)
+            torch.cuda.synchronize()
+            ref.append((y, z))
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        out = [(new(), new()) for _ in xs]
+        torch.cuda.synchronize()
+        for i, x in enumerate(xs):
+            step(x, *out[i], streams[i % 2], i % 2)
+        torch.cuda.synchronize()
+        for (y, z), (ry, rz) in zip(out, ref):
+            assert torch.equal(y, ry) and torch.equal(z, rz)
+        x, y, z = new(), new(), new()
+        s = streams[0]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s, capture_error_mode='relaxed'):   # scratch is allocated
+            step(x, y, z, s, 0)
+        for xi, (ry, rz) in zip(xs, ref):
+            x.copy_(xi)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, ry) and torch.equal(z, rz)
+        pkg.check()
