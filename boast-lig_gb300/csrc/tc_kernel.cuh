@@ -74,8 +74,8 @@
 // outputs held the whole operand buffer, so conversion, MMAs and drain of a tile
 // ran one after the other, and every tile converted its halo again; the kernel
 // was 190 KB of code with one epilogue for every case.  MagicFilter sweep 520 ->
-// 325 us, kinetic sweep along x 600 -> 361 us, with partial sums 640 -> 485 us
-// (issue slots 46 %, FP64 pipe 31 %, tensor pipe 20 %, HBM 25-50 %).  What
+// 286 us (340 handing on exponents), kinetic sweep along x 600 -> 328 us, with
+// partial sums 640 -> 470 us (issue slots 45 %, FP64 pipe 33-48 %, HBM 30-36 %).  What
 // mattered: the ring; one kernel per form of sweep with a short straight
 // epilogue loop (no spills, 50 KB: 436 -> 325 us for the MagicFilter sweep alone);
 // digits as FP16 subnormals; polls and shared-memory stores in few instructions.
@@ -1175,7 +1175,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             // latency, conversion and FP64 arithmetic in two warps per scheduler;
             // four outputs a step keep everything in registers (eight a step, and
             // operands two or four steps ahead, spill or outgrow the loop: kinetic
-            // sweep with partial sums, 32 x 128^3, 580 us at eight, 485 at four, 515
+            // sweep with partial sums, 32 x 128^3, 580 us at eight, 480 at four, 515
             // with operands two steps ahead).  Kinetic sweeps with energies (and a_y),
             // 110^3 x 8, went through cold_block before: 213-349 us, now 164-199
             // a partial block in the same loop pays where the general block would have
@@ -1404,7 +1404,7 @@ cudaError_t launch(const Sweep &S_in, const TcFilter &F, int *status, const int 
         if (S.x2) return launch_form<KIND, NT, SCH, FORM_X2>(S, F, status, lineE, st);
     if constexpr (SCH == SCH_EXACT && (KIND != KCONV || NT == 16))
         if (S.le_next) {
-            // 32 x 128^3: a sweep that hands on takes 338 us as HAND, 346 as HAND2
+            // MagicFilter3D on 32 x 128^3: 1.083 ms this way, 1.114 with HAND2 for all
             if (S.le_n1 % 32 == 0 && (long long)S.nL * S.nR % 32 == 0)
                 return launch_form<KIND, NT, SCH, FORM_HAND>(S, F, status, lineE, st);
             return launch_form<KIND, NT, SCH, FORM_HAND2>(S, F, status, lineE, st);
