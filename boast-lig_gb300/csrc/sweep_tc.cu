@@ -95,6 +95,7 @@ __host__ __device__ __forceinline__ int line_exp_plen(const Sweep &S) {
 // The same maxima for a batch of sweeps: blockIdx.y = sweep, its lines'
 // maxima written from out + le_off on.
 __global__ void line_exp_batch_kernel(const Sweep *__restrict__ descs, int *out) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const Sweep &S = descs[blockIdx.y];
     line_exp_lines(S, line_exp_plen(S), out + S.le_off,
                    (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
@@ -114,26 +115,20 @@ __global__ void line_exp_batch_kernel(const Sweep *__restrict__ descs, int *out)
 // combined across blocks with atomicMax (e0, e1 and, with several segments,
 // e2 zeroed first).
 constexpr int kExpChunk = 8;
-__global__ void __launch_bounds__(256)
-line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg,
-                 int *__restrict__ e0, int *__restrict__ e1, int *__restrict__ e2,
-                 const int *__restrict__ active) {
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+// The block's 32 i0 x 8 i1 columns from (b0, b1) on, planes [zb, ze) of one grid.
+__device__ __forceinline__ void line_exp3_block(const double *__restrict__ x, int n0, int n1, int n2, int b0, int b1,
+                                                int zb, int ze, int *__restrict__ e0, int *__restrict__ e1,
+                                                int *__restrict__ e2) {
     __shared__ int ys[kExpChunk][8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int i0 = blockIdx.x * 32 + tx, i1 = blockIdx.y * 8 + ty;
-    const long long a = blockIdx.z / nseg;
-    if (active && !active[a]) return;                   // grid skipped (uniform over the block)
-    const int seg = blockIdx.z % nseg, seglen = (n2 + nseg - 1) / nseg;
-    const int zb = seg * seglen, ze = min(n2, zb + seglen);
+    const int i0 = b0 + tx, i1 = b1 + ty;
     const bool valid = i0 < n0 && i1 < n1;
     const long long plane = (long long)n0 * n1;
-    const unsigned long long *xa =
-        reinterpret_cast<const unsigned long long *>(x) + a * plane * n2 + i0 + (long long)n0 * i1;
+    const unsigned long long *xa = reinterpret_cast<const unsigned long long *>(x) + i0 + (long long)n0 * i1;
     // e1 reader: column (c1, tx) of the chunk; e0 reader: quarter q0 of row (c0r, r0)
     const int c1 = ty, row = threadIdx.x >> 2, q0 = threadIdx.x & 3;
     const int c0r = row >> 3, r0 = row & 7;
-    const int i1r = blockIdx.y * 8 + r0;
+    const int i1r = b1 + r0;
     int zmax = 0;
     // the next chunk's loads are in flight while this chunk is reduced
     unsigned long long raw[kExpChunk];
@@ -156,7 +151,7 @@ line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg,
             int m = ys[c1][0][tx];
 #pragma unroll
             for (int r = 1; r < 8; ++r) m = max(m, ys[c1][r][tx]);
-            atomicMax(e1 + i0 + (long long)n0 * (c0 + c1 + (long long)n2 * a), m);
+            atomicMax(e1 + i0 + (long long)n0 * (c0 + c1), m);
         }
         {
             int m = ys[c0r][r0][8 * q0];
@@ -164,16 +159,42 @@ line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg,
             for (int k = 1; k < 8; ++k) m = max(m, ys[c0r][r0][8 * q0 + k]);
             m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
             m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            if (q0 == 0 && c0 + c0r < ze && i1r < n1)
-                atomicMax(e0 + i1r + (long long)n1 * (c0 + c0r + (long long)n2 * a), m);
+            if (q0 == 0 && c0 + c0r < ze && i1r < n1) atomicMax(e0 + i1r + (long long)n1 * (c0 + c0r), m);
         }
         __syncthreads();
     }
     if (valid) {
-        int *const p = e2 + i0 + (long long)n0 * (i1 + (long long)n1 * a);
-        if (nseg == 1) *p = zmax;
+        int *const p = e2 + i0 + (long long)n0 * i1;
+        if (zb == 0 && ze == n2) *p = zmax;
         else atomicMax(p, zmax);
     }
+}
+
+__global__ void __launch_bounds__(256)
+line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg,
+                 int *__restrict__ e0, int *__restrict__ e1, int *__restrict__ e2,
+                 const int *__restrict__ active) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const long long a = blockIdx.z / nseg;
+    if (active && !active[a]) return;                   // grid skipped (uniform over the block)
+    const int seg = blockIdx.z % nseg, seglen = (n2 + nseg - 1) / nseg, zb = seg * seglen;
+    if (zb >= n2) return;                               // more segments than seglen fills
+    line_exp3_block(x + a * n0 * n1 * n2, n0, n1, n2, blockIdx.x * 32, blockIdx.y * 8, zb, min(n2, zb + seglen),
+                    e0 + a * n1 * n2, e1 + a * n0 * n2, e2 + a * n0 * n1);
+}
+
+// The same for the grids of a batch: d0, d1, d2 describe the non-rotating sweeps
+// along axes 0, 1, 2 of each grid (all read the same x), whose exponents start at
+// their le_off.  blockIdx.y = grid.
+__global__ void __launch_bounds__(256)
+line_exp3_batch_kernel(const Sweep *__restrict__ d0, const Sweep *__restrict__ d1, const Sweep *__restrict__ d2,
+                       int *__restrict__ e0, int *__restrict__ e1, int *__restrict__ e2) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const Sweep &S = d1[blockIdx.y];
+    const int n0 = S.nL, n1 = S.n, n2 = S.nR, gx = (n0 + 31) / 32, tiles = gx * ((n1 + 7) / 8);
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x)
+        line_exp3_block(S.x, n0, n1, n2, t % gx * 32, t / gx * 8, 0, n2, e0 + d0[blockIdx.y].le_off, e1 + S.le_off,
+                        e2 + d2[blockIdx.y].le_off);
 }
 
 }  // namespace tck
@@ -398,11 +419,22 @@ int line_exp_batch_blocks(long long max_lines, bool contiguous) {
     return (int)(want < 1 ? 1 : want > 64 ? 64 : want);
 }
 
+cudaError_t launch_line_exp3_batch(const Sweep *d0, const Sweep *d1, const Sweep *d2, int nsweeps, int *e0,
+                                   long long lines0, int *e1, long long lines1, int *e2, int tiles,
+                                   cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(e0, 0, (size_t)lines0 * sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(e1, 0, (size_t)lines1 * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    tck::line_exp3_batch_kernel<<<dim3(tiles < 1 ? 1 : tiles > 256 ? 256 : tiles, nsweeps), 256, 0, st>>>(d0, d1, d2, e0,
+                                                                                                     e1, e2);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_sweep_tc_batch(int kind, int ntaps, const Sweep &like, const Sweep *descs, const long long *prefix,
                                   int nsweeps, const TcFilter &F, int sch, int *status,
-                                  int *lineE, int exp_blocks, cudaStream_t st) {
+                                  int *lineE, int exp_blocks, cudaStream_t st, bool lineE_ready) {
     if (sch == SCH_EXACT) {
-        if (lineE) {
+        if (lineE && !lineE_ready) {
             if (exp_blocks < 1 || nsweeps > 65535) return cudaErrorInvalidValue;
             tck::line_exp_batch_kernel<<<dim3(exp_blocks, nsweeps), 256, 0, st>>>(descs, lineE);
             cudaError_t e = cudaGetLastError();

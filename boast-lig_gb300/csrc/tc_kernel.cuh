@@ -526,7 +526,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
     };
 
     // the next kernel of the stream may start its own prologue (it waits below)
-    if (!BATCH) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                          saddr(tslot)),
@@ -585,7 +585,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
     bool alive = true;
     // everything above touches parameters and this CTA's own memory only; from here on
     // the work of the kernels before is complete
-    if (!BATCH) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     if (!BATCH && (FORM == FORM_HAND || FORM == FORM_HAND2) && S0.le_zero)
         for (long long i = (long long)blockIdx.x * kThreads + tid; i < S0.le_zero_n; i += (long long)gridDim.x * kThreads)
             S0.le_zero[i] = 0;
@@ -1362,28 +1362,33 @@ cudaError_t set_smem_attr() {
     return cudaSuccess;
 }
 
+// The sweep may start while the kernels before it in the stream finish: its
+// prologue (filter tiles, barriers, TMEM) needs nothing of theirs, and it waits
+// for their completion before its first access to the caller's or the scratch
+// memory (griddepcontrol.wait).  MagicFilter3D of one 32^3 grid 36 -> 28 us,
+// Hamiltonian 48^3 x 8 1655 -> 1589 us
+template <class Kernel, class... Args>
+void launch_early(Kernel *kernel, unsigned grid, int smem, cudaStream_t st, const Args &...args) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <int KIND, int NT, int SCH, int FORM>
 cudaError_t launch_form(const Sweep &S, const TcFilter &F, int *status, const int *lineE, cudaStream_t st) {
     using G = Geom<KIND, NT, SCH>;
     cudaError_t e = set_smem_attr<KIND, NT, SCH, false, FORM>();
     if (e != cudaSuccess) return e;
-    // The sweep may start while the kernels before it in the stream finish: its
-    // prologue (filter tiles, barriers, TMEM) needs nothing of theirs, and it waits
-    // for their completion before its first access to the caller's or the scratch
-    // memory (griddepcontrol.wait).  MagicFilter3D of one 32^3 grid 36 -> 28 us,
-    // Hamiltonian 48^3 x 8 1655 -> 1589 us
-    cudaLaunchAttribute early{};
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)sweep_tc_blocks(S));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = G::SMEM;
-    cfg.stream = st;
-    cfg.attrs = &early;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, sweep_tc_kernel<KIND, NT, SCH, false, FORM>, S, F, status,
-                       (const Sweep *)nullptr, (const long long *)nullptr, 0, lineE);
+    launch_early(sweep_tc_kernel<KIND, NT, SCH, false, FORM>, (unsigned)sweep_tc_blocks(S), G::SMEM, st, S, F, status,
+                 (const Sweep *)nullptr, (const long long *)nullptr, 0, lineE);
     return cudaGetLastError();
 }
 
@@ -1422,8 +1427,8 @@ cudaError_t launch_batch_form(const Sweep *descs, const long long *prefix, int n
     cudaError_t e = set_smem_attr<KIND, NT, SCH, true, FORM>();
     if (e != cudaSuccess) return e;
     Sweep S0{};
-    sweep_tc_kernel<KIND, NT, SCH, true, FORM><<<sm_count(), kThreads, G::SMEM, st>>>(
-        S0, F, status, descs, prefix, nsweeps, lineE);
+    launch_early(sweep_tc_kernel<KIND, NT, SCH, true, FORM>, (unsigned)sm_count(), G::SMEM, st, S0, F, status, descs,
+                 prefix, nsweeps, lineE);
     return cudaGetLastError();
 }
 
