@@ -28,9 +28,10 @@ int sm_count() {
 // Largest exponent field over the elements each line of S uses (positions
 // 0..plen-1 of every channel; ld padding is not read), one int per line of
 // every array.  Contiguous lines (nL == 1): a warp per line, lanes along the
-// line, four loads in flight (one by one, 110^3 x 8 took a
-// memory latency per 32 elements: 25 -> 16 us); strided lines: a thread per line,
+// line, L of them at a time with I loads each in flight (1 and 4: 110^3 x 8 16 us,
+// 25 one by one; a batch's short lines 4 and 2); strided lines: a thread per line,
 // consecutive lines in a warp.
+template <int L, int I>
 __device__ __forceinline__ void line_exp_lines(const Sweep &S, int plen, int *out, long long first,
                                                long long step) {
     const int nchan = S.kind == KCONV ? 1 : 2;
@@ -44,23 +45,36 @@ __device__ __forceinline__ void line_exp_lines(const Sweep &S, int plen, int *ou
     const int count = plen * nchan;
     if (S.nL == 1) {
         const int lane = threadIdx.x & 31;
-        for (long long w = first >> 5; w < total; w += step >> 5) {
-            const long long arr = w / nlines, r = w % nlines;
-            const long long *base = xb + arr * S.x_arr + pext * r;
-            uint32_t mx = 0;
-            for (int e0 = lane; e0 < count; e0 += 128) {
-                long long h[4];
+        const long long warps = step >> 5;
+        const bool packed = S.x_arr == pext * nlines;    // line w of all arrays at pext w
+        for (long long w = first >> 5; w < total; w += L * warps) {
+            const long long *base[L];
+            uint32_t mx[L];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+            for (int k = 0; k < L; ++k) {
+                const long long v = min(w + k * warps, total - 1);
+                base[k] = xb + (packed ? pext * v : v / nlines * S.x_arr + pext * (v % nlines));
+                mx[k] = 0;
+            }
+            for (int e0 = lane; e0 < count; e0 += 32 * I) {
+                long long h[L][I];
+#pragma unroll
+                for (int i = 0; i < I; ++i) {
                     const int e = e0 + 32 * i;
-                    h[i] = e < count ? base[offset(e)] : 0ll;
+#pragma unroll
+                    for (int k = 0; k < L; ++k) h[k][i] = e < count ? base[k][offset(e)] : 0ll;
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    mx = max(mx, (uint32_t)((unsigned long long)h[i] >> 32) & 0x7FF00000u);
+                for (int k = 0; k < L; ++k)
+#pragma unroll
+                    for (int i = 0; i < I; ++i)
+                        mx[k] = max(mx[k], (uint32_t)((unsigned long long)h[k][i] >> 32) & 0x7FF00000u);
             }
-            mx = __reduce_max_sync(0xffffffffu, mx);
-            if (lane == 0) out[w] = (int)(mx >> 20);
+#pragma unroll
+            for (int k = 0; k < L; ++k) {
+                const uint32_t m = __reduce_max_sync(0xffffffffu, mx[k]);
+                if (lane == 0 && w + k * warps < total) out[w + k * warps] = (int)(m >> 20);
+            }
         }
     } else {
         for (long long t = first; t < total; t += step) {
@@ -81,7 +95,7 @@ __global__ void line_exp_kernel(const Sweep S, int plen, int *out) {
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < S.le_next_lines * S.narr;
              i += (long long)gridDim.x * blockDim.x)
             S.le_next[i] = 0;
-    line_exp_lines(S, plen, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
+    line_exp_lines<1, 4>(S, plen, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
                    (long long)gridDim.x * blockDim.x);
 }
 
@@ -97,7 +111,7 @@ __host__ __device__ __forceinline__ int line_exp_plen(const Sweep &S) {
 __global__ void line_exp_batch_kernel(const Sweep *__restrict__ descs, int *out) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const Sweep &S = descs[blockIdx.y];
-    line_exp_lines(S, line_exp_plen(S), out + S.le_off,
+    line_exp_lines<4, 2>(S, line_exp_plen(S), out + S.le_off,
                    (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
@@ -414,9 +428,12 @@ bool sweep_tc_batch_supported(int kind, int ntaps) {
 }
 
 int line_exp_batch_blocks(long long max_lines, bool contiguous) {
-    const long long threads = contiguous ? max_lines * 32 : max_lines;
+    // four lines a warp; each block first waits for its descriptor, so not too many
+    // of them (128 grids, axes 24-72: a MagicFilter and kinetic run takes 1349, 1306,
+    // 1319 and 1384 us with at most 16, 32, 64 and 256 per grid)
+    const long long threads = contiguous ? max_lines * (32 / 4) : max_lines;
     const long long want = (threads + 255) / 256;
-    return (int)(want < 1 ? 1 : want > 64 ? 64 : want);
+    return (int)(want < 1 ? 1 : want > 32 ? 32 : want);
 }
 
 cudaError_t launch_line_exp3_batch(const Sweep *d0, const Sweep *d1, const Sweep *d2, int nsweeps, int *e0,
