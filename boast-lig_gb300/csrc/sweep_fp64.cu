@@ -230,6 +230,7 @@ __global__ void dot_reduce_kernel(const double *__restrict__ part, long long cou
 __global__ void dot_reduce_list_kernel(const double *__restrict__ part, const __grid_constant__ DotList L,
                                        double *out, long long out_stride) {
     const int i = blockIdx.y;
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     dot_reduce(part + L.off[i] + (long long)blockIdx.x * L.len[i], L.len[i],
                out + L.slot[i] + (long long)blockIdx.x * out_stride, 0);
 }
@@ -341,7 +342,19 @@ cudaError_t launch_dot_reduce(const double *part, long long count, double *out, 
 
 cudaError_t launch_dot_reduce_list(const double *part, const DotList &L, int nseg, double *out,
                                    long long out_stride, cudaStream_t st) {
-    dot_reduce_list_kernel<<<dim3(nseg, L.n), 256, 0, st>>>(part, L, out, out_stride);
+    // may be set up while the last sweep finishes (it waits before it reads).  FP64
+    // sweeps launched so were slower: their blocks take the running ones' places
+    // and wait there (kinetic 3D of one 96^3 grid 189 -> 291 us)
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nseg, L.n);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, dot_reduce_list_kernel, part, L, out, out_stride);
     return cudaGetLastError();
 }
 
