@@ -34,7 +34,7 @@ struct Stage {
     std::vector<Sweep> bound;                // per grid, pointers bound
     Sweep *d_desc = nullptr;
     long long *d_prefix = nullptr;
-    long long units = 0;                     // tiles / blocks of the stage
+    long long units = 0;                     // strips / blocks of the stage
     int grid = 0;                            // FP64 persistent grid
     TcFilter F;
     int *d_lineE = nullptr;                  // exact tensor-core sweeps: line exponents of all grids
@@ -109,7 +109,7 @@ int grid_plan(const libconv_batch *b, int o, int g, const int *ord, Plan &P) {
     return plan_kinetic(3, n, b->kin_bc, b->kin_a, b->kin_ax, ord, P);
 }
 
-// Build the stages of operator o for (engine, order): descriptors, tile /
+// Build the stages of operator o for (engine, order): descriptors, strip /
 // block prefix sums (device), filter operands.
 int configure(libconv_batch *b, int o, int engine, const int *ord) {
     OpConfig &C = b->op[o];

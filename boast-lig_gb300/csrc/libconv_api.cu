@@ -841,7 +841,7 @@ int exec_host(const Plan &P, const double *x, double *y, double *dot_host) {
 // -> dwt (shrink).  Free axes take that grow/shrink chain; periodic axes are
 // periodic in every step.  norb orbitals lie back to back and every step is
 // one launch over all of them (narr = norb), so a sweep covers norb grids'
-// worth of tiles; the energies are kept per orbital (segmented dots).
+// worth of strips; the energies are kept per orbital (segmented dots).
 struct Ham {
     Plan idwt, mf, imf, kin, dwt;
     int norb = 1;

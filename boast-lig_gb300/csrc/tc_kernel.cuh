@@ -75,13 +75,14 @@
 // ran one after the other, and every tile converted its halo again; the kernel
 // was 190 KB of code with one epilogue for every case.  MagicFilter sweep 520 ->
 // 286 us (340 handing on exponents), kinetic sweep along x 600 -> 328 us, with
-// partial sums 640 -> 470 us (issue slots 45 %, FP64 pipe 33-48 %, HBM 30-36 %).  What
-// mattered: the ring; one kernel per form of sweep with a short straight
+// partial sums 640 -> 470 us (issue slots 45 %, FP64 pipe 33-48 %, HBM 30-36 %).
+// What mattered: the ring; one kernel per form of sweep with a short straight
 // epilogue loop (no spills, 50 KB: 436 -> 325 us for the MagicFilter sweep alone);
-// digits as FP16 subnormals; polls and shared-memory stores in few instructions.
-// Measured and slower: three epilogue groups and an issuer warp on 24 warps (80
-// registers: 1.58 ms against 1.52 for MagicFilter3D), TMEM loads one step ahead,
-// global loads two slabs ahead (kinetic 1.60 -> 1.65 ms; one slab ahead, the next on its way to L2), larger unrolled loops.
+// digits as FP16 subnormals; polls and shared-memory stores in few instructions;
+// the slab after the next prefetched to L2.  Measured and slower: three epilogue
+// groups and an issuer warp on 24 warps (80 registers: 1.58 ms against 1.52 for
+// MagicFilter3D), TMEM loads one step ahead, global loads two slabs ahead in
+// registers (kinetic 1.60 -> 1.65 ms), larger unrolled loops.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -972,13 +973,16 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 uint32_t mask = sel;
 #pragma unroll 1
                 for (int line = 0;; ++line) {
-                    uint32_t mine = 0;
+                    uint32_t m[n];
 #pragma unroll
-                    for (int i = 0; i < n; ++i) {
-                        const uint32_t m = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(v[i]) & mask);
-                        if (lane == i) mine = m >> 20;
-                    }
-                    if (keeps) atomicMax(le + line, (int)mine);
+                    for (int i = 0; i < n; ++i) m[i] = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(v[i]) & mask);
+                    // m[lane % n], by the lane's bits (log2 n predicates instead of n:
+                    // MagicFilter3D on 32 x 128^3 1.055 -> 1.044 ms)
+#pragma unroll
+                    for (int w = 1; w < n; w *= 2)
+#pragma unroll
+                        for (int i = 0; i < n; i += 2 * w) m[i] = lane & w ? m[i + w] : m[i];
+                    if (keeps) atomicMax(le + line, (int)(m[0] >> 20));
                     if (!two || line == 1) break;
                     mask = valid ? 0x7FFFFFFFu - sel : 0u;
                 }
