@@ -208,7 +208,7 @@ sweep_fp64_batch_kernel(const Sweep *__restrict__ descs, const long long *__rest
 
 // Block b sums part[b*count .. (b+1)*count) in a fixed order into
 // out[b*out_stride] (one block per segment: per-array dot products).
-__device__ __forceinline__ void dot_reduce(const double *__restrict__ part, long long count, double *out,
+__device__ __forceinline__ void dot_reduce(const double *part, long long count, double *out,
                                            int accumulate) {
     __shared__ double red[256];
     double s = 0.0;
@@ -227,8 +227,9 @@ __global__ void dot_reduce_kernel(const double *__restrict__ part, long long cou
     dot_reduce(part + (long long)blockIdx.x * count, count, out + (long long)blockIdx.x * out_stride, accumulate);
 }
 
-__global__ void dot_reduce_list_kernel(const double *__restrict__ part, const __grid_constant__ DotList L,
-                                       double *out, long long out_stride) {
+// part without __restrict__: the sweep that writes it may still be running
+__global__ void dot_reduce_list_kernel(const double *part, const __grid_constant__ DotList L, double *out,
+                                       long long out_stride) {
     const int i = blockIdx.y;
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     dot_reduce(part + L.off[i] + (long long)blockIdx.x * L.len[i], L.len[i],

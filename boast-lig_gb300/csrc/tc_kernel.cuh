@@ -251,10 +251,15 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
     asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
 }
 
-// 32 bytes from global memory (a 32-byte aligned address) in one load.
+// 32 bytes from global memory (a 32-byte aligned address) in one load.  It keeps its
+// place among the waits and stores around it: the kernels before may still be
+// writing what it reads until griddepcontrol.wait, and y is read and rewritten.
 __device__ __forceinline__ void ld256(const long long *p, long long &a, long long &b, long long &c,
                                       long long &d) {
-    asm("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+    asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(a), "=l"(b), "=l"(c), "=l"(d)
+                 : "l"(p)
+                 : "memory");
 }
 
 // 32 bytes to global memory (a 32-byte aligned address) in one store.
@@ -495,7 +500,7 @@ template <int KIND, int NT, int SCH, bool BATCH, int FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilter F, int *status,
                 const Sweep *__restrict__ descs, const long long *__restrict__ prefix, int nsweeps,
-                const int *__restrict__ lineE) {
+                const int *lineE) {      // no __restrict__: a kernel still running may write it
     using G = Geom<KIND, NT, SCH>;
     constexpr int NCH = G::NCH, W = G::W, PB = G::PB;
     extern __shared__ uint8_t smem_raw[];

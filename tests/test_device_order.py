@@ -1,0 +1,49 @@
+"""Rules of the device sources that keep memory accesses in their order, read off the text:
+a compiler may move what it is not told about, and no run shows whether it will."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), 'boast-lig_gb300', 'csrc')
+SOURCES = sorted(glob.glob(os.path.join(CSRC, '*.cu')) + glob.glob(os.path.join(CSRC, '*.cuh')))
+
+
+def asm_statements(path):
+    """(volatile, text) of every inline assembly statement."""
+    text = open(path).read()
+    for m in re.finditer(r'\basm\s*(volatile)?\s*\(', text):
+        depth, i = 1, m.end()
+        quoted = False
+        while depth:
+            c = text[i]
+            if c == '"' and text[i - 1] != '\\':
+                quoted = not quoted
+            elif not quoted:
+                depth += (c == '(') - (c == ')')
+            i += 1
+        yield m.group(1) is not None, text[m.end():i - 1]
+
+
+@pytest.mark.parametrize('path', SOURCES, ids=os.path.basename)
+def test_memory_instructions_are_ordered(path):
+    """What reads or writes memory, barriers or tensor memory is volatile and clobbers memory:
+    otherwise a load's result is a function of its address to the compiler, which may move it
+    across a wait or a store."""
+    for volatile, text in asm_statements(path):
+        if re.search(r'\b(ld|st|red|atom|cp\.async|mbarrier|tcgen05\.(ld|mma|commit))\b', text):
+            assert volatile and '"memory"' in text, text
+
+
+@pytest.mark.parametrize('path', SOURCES, ids=os.path.basename)
+def test_early_kernels_read_no_constant_memory_of_their_predecessors(path):
+    """A kernel that starts before its predecessors end (griddepcontrol.wait) takes what those write
+    through plain pointers: const __restrict__ lets the compiler load it before the wait.  The
+    descriptors and prefix sums of a batch are written by no kernel."""
+    text = open(path).read()
+    for m in re.finditer(r'__global__[^;{]*?(\w+)\(([^{;]*?)\)\s*\{', text):
+        body = text[m.end():].split('__global__')[0]
+        if 'griddepcontrol.wait' in body:
+            params = re.findall(r'__restrict__\s*(\w+)', m.group(2))
+            assert set(params) <= {'descs', 'prefix'}, (m.group(1), params)
