@@ -518,19 +518,8 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
     auto drained = [&](uint32_t s) { return bar0 + 8 * (2 * kSlots + 4 + s); };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long nstrips =
-        BATCH ? prefix[nsweeps]
-              : ((long long)S0.nL * S0.nR + kM - 1) / kM * (long long)S0.tdiv_d[0] * S0.narr;
     // window offset of the convolution sweeps (0 in batched launches)
     const int woff = (!BATCH && KIND == KCONV) ? S0.woff : 0;
-    // the strip after `strip` for this CTA, skipping inactive arrays
-    auto skip_inactive = [&](long long strip) -> long long {
-        if (!BATCH && S0.active)
-            while (strip < nstrips && !S0.active[locate<BATCH>(S0, descs, prefix, nsweeps, strip).arr])
-                strip += gridDim.x;
-        return strip;
-    };
-
     // the next kernel of the stream may start its own prologue (it waits below)
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (warp == 0) {
@@ -592,6 +581,16 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
     // everything above touches parameters and this CTA's own memory only; from here on
     // the work of the kernels before is complete
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    const long long nstrips =
+        BATCH ? prefix[nsweeps]
+              : ((long long)S0.nL * S0.nR + kM - 1) / kM * (long long)S0.tdiv_d[0] * S0.narr;
+    // the strip after `strip` for this CTA, skipping inactive arrays
+    auto skip_inactive = [&](long long strip) -> long long {
+        if (!BATCH && S0.active)
+            while (strip < nstrips && !S0.active[locate<BATCH>(S0, descs, prefix, nsweeps, strip).arr])
+                strip += gridDim.x;
+        return strip;
+    };
     if (!BATCH && (FORM == FORM_HAND || FORM == FORM_HAND2) && S0.le_zero)
         for (long long i = (long long)blockIdx.x * kThreads + tid; i < S0.le_zero_n; i += (long long)gridDim.x * kThreads)
             S0.le_zero[i] = 0;

@@ -47,3 +47,14 @@ def test_early_kernels_read_no_constant_memory_of_their_predecessors(path):
         if 'griddepcontrol.wait' in body:
             params = re.findall(r'__restrict__\s*(\w+)', m.group(2))
             assert set(params) <= {'descs', 'prefix'}, (m.group(1), params)
+
+
+def test_sweep_prologue_reads_no_global_memory():
+    """Before griddepcontrol.wait the tensor-core sweep touches parameters and its own memory only:
+    nothing there goes through a pointer parameter, prefix sums and descriptors of a batch included."""
+    text = open(os.path.join(CSRC, 'tc_kernel.cuh')).read()
+    body = text[text.index('sweep_tc_kernel('):]
+    prologue = body[body.index('{') + 1:body.index('griddepcontrol.wait')]
+    prologue = re.sub(r'//[^\n]*', '', prologue)
+    assert not re.search(r'\b(descs|prefix|lineE|status|locate|skip_inactive)\b', prologue)
+    assert not re.search(r'S0\.(x|y|x2|active|dot_part|le_next|le_zero)\b', prologue)
