@@ -19,6 +19,7 @@
 #include "lcg_pool.cuh"
 #include "lcg_sweep.cuh"
 #include "lcg_tc.cuh"
+#include "lcg_wait.cuh"
 #include "libconv_filters.h"
 
 using namespace lcg;
@@ -1345,36 +1346,17 @@ int *device_status(int &rc) {
 
 namespace lcg {
 namespace {
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Self-test of the bounded device waits: one thread waits on an mbarrier that
-// nothing arrives at, with the same try_wait / sleep / limit loop as the
-// tensor-core kernels, gives up after `limit_ns` nanoseconds of the GPU's
-// global timer (independent of the SM clock) and sets the status word.
-// Nothing faults and the wait always ends.
+// Self-test of the bounded device waits: one thread waits, by the tensor-core
+// sweeps' own function, on an mbarrier that nothing arrives at, gives up after
+// `limit_ns` nanoseconds of the GPU's global timer (independent of the SM clock)
+// and sets the status word.  Nothing faults and the wait always ends.
 __global__ void selftest_wait_kernel(int *status, unsigned long long limit_ns) {
     __shared__ __align__(8) unsigned long long bar;
     if (threadIdx.x != 0) return;
     const uint32_t b = (uint32_t)__cvta_generic_to_shared(&bar);
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(b) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    const unsigned long long t0 = global_ns();
-    uint32_t ok = 0;
-    while (true) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(ok)
-            : "r"(b)
-            : "memory");
-        if (ok || global_ns() - t0 > limit_ns) break;
-        __nanosleep(128);
-    }
-    if (!ok) atomicExch(status, 1);
+    if (!bar_wait(b, 0, limit_ns)) atomicExch(status, 1);
 }
 
 // FP64 pipe probe: every thread runs 8 independent FMA chains (no dependency

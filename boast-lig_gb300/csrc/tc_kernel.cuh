@@ -64,8 +64,8 @@
 // producers (every block that reads a slab commits to it; the issuer of the
 // first reader adds the arrivals of the readers a strip's ends do not have),
 // tfull[slot] MMAs and issuer -> epilogue, drained[slot] epilogue -> issuer.
-// No phase can run two ahead of its waiter; every wait gives up after kWaitPolls
-// polls (status word set, TMEM freed, kernel returns).  In single-sweep launches
+// No phase can run two ahead of its waiter; every wait gives up after kWaitLimit
+// (lcg_wait.cuh: status word set, TMEM freed, kernel returns).  In single-sweep launches
 // every role skips the strips of an array whose S0.active flag is 0 (flags fixed
 // for the launch), so the roles still meet on the same strips.
 //
@@ -91,6 +91,7 @@
 
 #include "lcg_sweep.cuh"
 #include "lcg_tc.cuh"
+#include "lcg_wait.cuh"
 
 namespace lcg {
 namespace tck {
@@ -100,8 +101,6 @@ constexpr int kSlots = 6;        // slabs in the operand ring
 constexpr int kThreads = 512;    // 8 producer warps + 8 epilogue warps
 constexpr int kProdWarps = 8, kEpiWarps = 8;
 static_assert(kEpiWarps == kTcDotSlots, "dot partials per CTA");
-constexpr uint32_t kWaitSleep = 64;                  // ns
-constexpr uint32_t kWaitPolls = 1u << 26;            // polls of a wait: seconds at the least rate seen
 
 // Forms of a sweep, one kernel each, so that the epilogue of the common ones is
 // a short loop (code and registers): plain stores; plus a partial sum x2; plus
@@ -209,22 +208,6 @@ __device__ __forceinline__ void bar_arrive_n(uint32_t bar, uint32_t n) {
     asm volatile(
         "{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0], %1;\n\t}\n" ::"r"(bar), "r"(n)
         : "memory");
-}
-
-// Bounded wait for the phase of the given parity; false after kWaitPolls polls.
-// The loop is a few instructions: a waiting warp's polls come out of the working
-// warps' issue slots.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n"
-        "WAIT_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE_%=;\n\t"
-        "nanosleep.u32 %4;\n\tsub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra WAIT_%=;\n"
-        "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "n"(kWaitPolls), "n"(kWaitSleep)
-        : "memory");
-    return ok != 0;
 }
 
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {

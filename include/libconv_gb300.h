@@ -90,8 +90,9 @@ int libconv_gb300_check(void *stream);
  * a barrier that nothing arrives at, limited to wait_us microseconds (1 to
  * 1e6) of the GPU's global timer; it gives up, sets the device status word
  * and returns, so the next libconv_gb300_check reports LIBCONV_ETIMEOUT (and
- * clears the word).  (The kernels' own waits give up after 4e9 SM clock
- * cycles, about 2 s at the maximum clock, longer at lower clocks.) */
+ * clears the word).  The wait is the tensor-core sweeps' own function, which
+ * gives up after 2 s of the same timer.  (The network layers' waits: 4e9 SM
+ * clock cycles, about 2 s at the maximum clock, longer at lower clocks.) */
 int libconv_gb300_selftest_wait(int wait_us, void *stream);
 /* Diagnostic, no counterpart in the reference: measured FP64 FMA throughput
  * of this GPU (the roof of the plain FP64 sweeps).  Runs 8 independent FMA

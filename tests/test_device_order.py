@@ -58,3 +58,12 @@ def test_sweep_prologue_reads_no_global_memory():
     prologue = re.sub(r'//[^\n]*', '', prologue)
     assert not re.search(r'\b(descs|prefix|lineE|status|locate|skip_inactive)\b', prologue)
     assert not re.search(r'S0\.(x|y|x2|active|dot_part|le_next|le_zero)\b', prologue)
+
+
+def test_sweeps_and_self_test_share_the_bounded_wait():
+    """One wait function, limited by the GPU's global timer; no loop of polls beside it."""
+    for name in ('tc_kernel.cuh', 'libconv_api.cu'):
+        text = open(os.path.join(CSRC, name)).read()
+        assert 'mbarrier.try_wait' not in text and 'mbarrier.test_wait' not in text and 'bar_wait(' in text, name
+    wait = open(os.path.join(CSRC, 'lcg_wait.cuh')).read()
+    assert 'globaltimer' in wait and wait.count('mbarrier.try_wait') == 1
