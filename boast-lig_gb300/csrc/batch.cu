@@ -109,16 +109,9 @@ int grid_plan(const libconv_batch *b, int o, int g, const int *ord, Plan &P) {
     return plan_kinetic(3, n, b->kin_bc, b->kin_a, b->kin_ax, ord, P);
 }
 
-// Build the stages of operator o for (engine, order): descriptors, strip /
+// Build the stages of operator o for (engine, order) in C: descriptors, strip /
 // block prefix sums (device), filter operands.
-int configure(libconv_batch *b, int o, int engine, const int *ord) {
-    OpConfig &C = b->op[o];
-    if (!engine_allowed(b->mode, engine))
-        return report(LIBCONV_EMODE, "engine not available in this batch's compute mode");
-    if (o == LIBCONV_BATCH_OP_KIN && ord[0] < 0) return fail_arg("kinetic needs an explicit order");
-    for (Stage &s : C.stages) free_stage(s);
-    C.stages.clear();
-    drop_graph(b);
+int build_stages(const libconv_batch *b, int o, int engine, const int *ord, OpConfig &C) {
     const int G = b->ngrids;
     for (int g = 0; g < G; ++g) {
         Plan P;
@@ -202,7 +195,6 @@ int configure(libconv_batch *b, int o, int engine, const int *ord) {
     for (int i = 0; i < 3; ++i) C.order[i] = ord[i];
     // exact kinetic sweeps: all read x, along its three axes; one exponent pass serves
     // them (128 grids, axes 24-72, MagicFilter and kinetic: 1485 us with one each, 1338)
-    C.exp3_tiles = 0;
     if (tc && scheme_of(b->mode) == SCH_EXACT && o == LIBCONV_BATCH_OP_KIN) {
         const std::vector<Sweep> &A1 = C.stages[C.stage_of(1)].sw;
         for (const Sweep &S : A1) {
@@ -211,6 +203,23 @@ int configure(libconv_batch *b, int o, int engine, const int *ord) {
         }
     }
     return LIBCONV_OK;
+}
+
+// Set operator o to (engine, order).  A configuration that cannot be built leaves
+// the one before it in place.
+int configure(libconv_batch *b, int o, int engine, const int *ord) {
+    if (!engine_allowed(b->mode, engine))
+        return report(LIBCONV_EMODE, "engine not available in this batch's compute mode");
+    if (o == LIBCONV_BATCH_OP_KIN && ord[0] < 0) return fail_arg("kinetic needs an explicit order");
+    OpConfig C;
+    C.enabled = b->op[o].enabled;
+    const int rc = build_stages(b, o, engine, ord, C);
+    if (rc == LIBCONV_OK) {
+        drop_graph(b);
+        std::swap(C, b->op[o]);
+    }
+    for (Stage &s : C.stages) free_stage(s);
+    return rc;
 }
 
 // Bind the caller's buffers into the stage descriptors and upload them on st.
