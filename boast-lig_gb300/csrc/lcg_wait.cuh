@@ -34,7 +34,7 @@ __device__ __forceinline__ bool bar_polls(uint32_t bar, uint32_t parity) {
 
 // The rest of a wait that kWaitPolls polls did not end: out of line, the working
 // warps' loops stay short.
-__device__ __noinline__ bool bar_wait_long(uint32_t bar, uint32_t parity, unsigned long long limit_ns) {
+static __device__ __noinline__ bool bar_wait_long(uint32_t bar, uint32_t parity, unsigned long long limit_ns) {
     const unsigned long long t0 = global_ns();
     while (!bar_polls(bar, parity))
         if (global_ns() - t0 > limit_ns) return false;
