@@ -23,6 +23,6 @@ def test_wait_ends_at_its_limit(pkg, limit_us):
     torch.cuda.synchronize()
     us = 1e3 * e0.elapsed_time(e1)
     assert L.libconv_gb300_check(None) == -7 and L.libconv_gb300_check(None) == 0
-    # two runs of 256 polls, each at most 1 us suspended and 0.13 us (twice 64 ns) asleep, the
-    # timer's steps of 1 us, and 100 us for the launch between two events
+    # two runs of polls (together less than 512 of 1 us and twice 64 ns), the timer's steps of
+    # 1 us, and 100 us for the launch between two events
     assert limit_us <= us <= limit_us + 2 * 256 * 1.13 + 1 + 100
