@@ -98,6 +98,14 @@ namespace tck {
 
 constexpr int kM = 128;          // lines per strip (MMA M)
 constexpr int kSlots = 6;        // slabs in the operand ring
+constexpr int kTmemSlots = 4;    // output blocks in TMEM
+// Strips whose row exponents are kept.  Producers write strip s's once slab W s - 1
+// of strips of one block (the shortest: W slabs) is in the ring, so once slab
+// W s - 1 - kSlots has left it and block s - ceil((kSlots + 1) / W) was issued; that took
+// every warp of its group past the block kTmemSlots before, and of the same group.  An
+// epilogue warp still to read its exponents is then less than ceil((kSlots + 1) / W)
+// + kTmemSlots strips behind: 8 for W = 2, the ring's length (tests/test_tc_ring.py).
+constexpr int kExpRing = 8;
 constexpr int kThreads = 512;    // 8 producer warps + 8 epilogue warps
 constexpr int kProdWarps = 8, kEpiWarps = 8;
 static_assert(kEpiWarps == kTcDotSlots, "dot partials per CTA");
@@ -141,13 +149,14 @@ template <int KIND, int NT, int SCH> struct Geom {
     // as both operands of an N = 128 MMA it sets an output block's eight order
     // accumulators to 3 * 8^2 = 192 = 1.5 * 2^23 units of 2^-16
     static constexpr int Z_BYTES = SCH == SCH_EXACT ? kM * 16 * 2 : 0;
-    // barriers and TMEM address; row exponents of the last 8 strips
-    static constexpr int AUX = 256 + 8 * kM * 2;
+    // barriers and TMEM address; row exponents of the last kExpRing strips
+    static constexpr int AUX = 256 + kExpRing * kM * 2;
     static constexpr int SMEM = A_BYTES + B_BYTES + Z_BYTES + AUX + 1024;
     static constexpr int SLOT_COLS = ORD * 16;                   // one TMEM slot (a block)
-    static constexpr uint32_t TMEM_COLS = 4 * SLOT_COLS <= 128 ? 128 : 4 * SLOT_COLS <= 256 ? 256 : 512;
-    static_assert(4 * SLOT_COLS <= 512, "TMEM columns");
+    static constexpr uint32_t TMEM_COLS = kTmemSlots * SLOT_COLS <= 128 ? 128 : kTmemSlots * SLOT_COLS <= 256 ? 256 : 512;
+    static_assert(kTmemSlots * SLOT_COLS <= 512, "TMEM columns");
     static_assert(W >= 2 && W < kSlots, "slab ring");
+    static_assert(kExpRing >= (kSlots + W) / W + kTmemSlots, "row exponents in use");
     static_assert(ND % PL == 0 && CH % 2 == 0, "plane slices");
     static_assert(SMEM <= 232448, "shared memory");
     // Instruction descriptor (kind::f16 / kind::tf32): D F32; A and B F16
@@ -493,12 +502,12 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
     uint8_t *Z = B + G::B_BYTES;                      // exact scheme: accumulator bias tile
     uint8_t *aux = Z + G::Z_BYTES;
     uint32_t *tslot = (uint32_t *)(aux + 192);
-    short *rowE8 = (short *)(aux + 256);              // row exponents, by strip mod 8
+    short *rowE = (short *)(aux + 256);               // row exponents, by strip mod kExpRing
     const uint32_t bar0 = saddr(aux);
     auto full = [&](uint32_t s) { return bar0 + 8 * s; };
     auto empty = [&](uint32_t s) { return bar0 + 8 * (kSlots + s); };
     auto tfull = [&](uint32_t s) { return bar0 + 8 * (2 * kSlots + s); };
-    auto drained = [&](uint32_t s) { return bar0 + 8 * (2 * kSlots + 4 + s); };
+    auto drained = [&](uint32_t s) { return bar0 + 8 * (2 * kSlots + kTmemSlots + s); };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // window offset of the convolution sweeps (0 in batched launches)
@@ -517,7 +526,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
             bar_init(full(s), kProdWarps);
             bar_init(empty(s), W);                    // one arrival per block of a window
         }
-        for (int s = 0; s < 4; ++s) {
+        for (int s = 0; s < kTmemSlots; ++s) {
             bar_init(tfull(s), 2);                    // the issuer's commit and its own arrival
             bar_init(drained(s), kEpiWarps / 2);
         }
@@ -798,7 +807,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 mxs = (uint32_t)(mx + 1) << 20;
                 fast = !__any_sync(0xffffffffu, mx < 64);
                 if (SCH == SCH_EXACT && half == 0)
-                    rowE8[(si & 7) * kM + row] = (short)(mx == 0x7FF ? 0x7FFF : mxe - 1022);
+                    rowE[si % kExpRing * kM + row] = (short)(mx == 0x7FF ? 0x7FFF : mxe - 1022);
                 ++si;
             }
         }
@@ -840,8 +849,8 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
         auto issue_next = [&]() -> bool {
             if (istrip >= nstrips) return true;
             if (lq == (int)((iblk >> 1) & 3)) {
-                const uint32_t ts = iblk & 3, last = islab + W - 1;
-                if (iblk >= 4 && !bar_wait(drained(ts), ((iblk >> 2) - 1) & 1)) return false;
+                const uint32_t ts = iblk % kTmemSlots, last = islab + W - 1;
+                if (iblk >= kTmemSlots && !bar_wait(drained(ts), (iblk / kTmemSlots - 1) & 1)) return false;
                 if (!bar_wait(full(last % kSlots), (last / kSlots) & 1)) return false;
                 if (lane == 0) {
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -933,8 +942,8 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 // known with the strip's first slab; a row holding an Inf or NaN
                 // gives NaN; farrow: 2^se is outside the range of the fast
                 // conversion (two multiplications, the first one exact)
-                if (!bar_wait(tfull((blk0 + j0) & 3), ((blk0 + j0) >> 2) & 1)) { alive = false; break; }
-                const int Er = rowE8[(si & 7) * kM + row];
+                if (!bar_wait(tfull((blk0 + j0) % kTmemSlots), ((blk0 + j0) / kTmemSlots) & 1)) { alive = false; break; }
+                const int Er = rowE[si % kExpRing * kM + row];
                 const bool nanrow = Er == 0x7FFF;
                 se = nanrow ? 0 : max(Er + F.ef - 58, -2000);
                 farrow = valid && (nanrow || se < -1022 || se > 961);
@@ -986,7 +995,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
 #pragma unroll
                     for (int k = 0; k < G::ORD; ++k)
                         tmem_ld4(tmem + ((uint32_t)(lq * 32) << 16) +
-                                     (uint32_t)((blk & 3) * G::SLOT_COLS + k * 16 + 4 * st),
+                                     (uint32_t)((blk % kTmemSlots) * G::SLOT_COLS + k * 16 + 4 * st),
                                  acc[k]);
                     double add[4];
                     if (kMayX2 && x2 && valid) {
@@ -1001,7 +1010,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     if (st == 3) {                        // the slot may be reissued
                         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                         __syncwarp();
-                        if (lane == 0) bar_arrive(drained(blk & 3));
+                        if (lane == 0) bar_arrive(drained(blk % kTmemSlots));
                     }
                     if ((!hands && !valid) || nv <= 0) continue;
                     double *const ystep = yrow + yps * (q0 - S.out_lo);
@@ -1109,7 +1118,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 constexpr bool kHands = hands, kVec = MODE.value == RUN_VEC;
                 const uint32_t blk = blk0 + j;
                 double *yb = yrow + yps * (qs + j * PB - S.out_lo);
-                const uint32_t ta = tmem + ((uint32_t)(lq * 32) << 16) + (blk & 3) * G::SLOT_COLS;
+                const uint32_t ta = tmem + ((uint32_t)(lq * 32) << 16) + (blk % kTmemSlots) * G::SLOT_COLS;
 #pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
                     uint32_t acc[G::ORD][8];
@@ -1119,7 +1128,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     if (h == 1) {             // the slot may be reissued
                         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                         __syncwarp();
-                        if (lane == 0) bar_arrive(drained(blk & 3));
+                        if (lane == 0) bar_arrive(drained(blk % kTmemSlots));
                     }
                     double v[8];
 #pragma unroll
@@ -1200,7 +1209,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 constexpr bool kVec = MODE.value == RUN_VEC, kPart = MODE.value == RUN_PART;
                 const uint32_t blk = blk0 + j;
                 const int q0 = qs + j * PB;
-                const uint32_t tb = tmem + ((uint32_t)(lq * 32) << 16) + (blk & 3) * G::SLOT_COLS;
+                const uint32_t tb = tmem + ((uint32_t)(lq * 32) << 16) + (blk % kTmemSlots) * G::SLOT_COLS;
                 const bool more = full_block(j + 2), part = !more && j + 2 < nb;
                 int nv = kPart ? S.qhi - q0 + 1 : 16;            // outputs left
                 if (more && valid) {                     // the group's next block on its way to L2
@@ -1219,7 +1228,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     if (st == 3) {                       // the slot may be reissued
                         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                         __syncwarp();
-                        if (lane == 0) bar_arrive(drained(blk & 3));
+                        if (lane == 0) bar_arrive(drained(blk % kTmemSlots));
                     }
                     double v[4];
 #pragma unroll
@@ -1281,7 +1290,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                         if (nv <= 0 && st < 3) {         // the rest of the block is not there
                             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                             __syncwarp();
-                            if (lane == 0) bar_arrive(drained(blk & 3));
+                            if (lane == 0) bar_arrive(drained(blk % kTmemSlots));
                             break;
                         }
                     }
@@ -1311,7 +1320,7 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                 // issuing after the wait keeps the phases apart: the slabs that
                 // block blk + 2's replaced in the ring were read by block blk or
                 // an earlier one, so their phase is known to be over
-                if (!bar_wait(tfull(blk & 3), (blk >> 2) & 1) || !issue_next()) { alive = false; break; }
+                if (!bar_wait(tfull(blk % kTmemSlots), (blk / kTmemSlots) & 1) || !issue_next()) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 if (!hot || (!kPartial && !full_block(j))) {
                     cold_block(j);
