@@ -41,6 +41,9 @@ struct Sweep {
     // elements before the first input position, so that along contiguous
     // lines its 8-element groups start on 32-byte boundaries (0 otherwise)
     int woff = 0;
+    // exact tensor-core sweeps whose own pass takes an exponent per line and window
+    // (tc_windows): the windows of a line; 0: one exponent per line
+    int le_win = 0;
     // per array: 0 = skip the array's lines (its output is left as it is); null:
     // every array (sweeps without a dot product only)
     const int *active = nullptr;

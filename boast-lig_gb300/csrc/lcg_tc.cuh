@@ -48,11 +48,20 @@ long long sweep_tc_line_blocks(const Sweep &S);
 // slots of an array a CTA has no strip of are not written.
 constexpr int kTcDotSlots = 8;
 long long sweep_tc_blocks(const Sweep &S);
+// Windows of a line whose exponents an exact sweep takes one by one in its own
+// pass (one per run of 64 outputs, over the elements that run reads), for periodic
+// convolutions along lines at least as long as one window (16 taps 80 elements,
+// 29 taps 96); 0 for other sweeps, which have one exponent per line.
+int tc_windows(const Sweep &S);
+// Exponents of S: one per line, or per line and window when S.le_win is set
+// (entry window * sweep_tc_lines(S) + line).
+long long sweep_tc_exps(const Sweep &S);
 // status (device int) is set non-zero if a tensor-core wait timed out.
-// lineE (exact scheme, or null): device scratch of sweep_tc_lines(S) ints; the
-// largest exponent of each line is computed into it first (one read of the
-// input), so the tensor-core sweep reads its input once.
-// lineE_ready: lineE already holds the exponents (launch_line_exp3); no pre-pass.
+// lineE (exact scheme, or null): device scratch of sweep_tc_exps(S) ints; the
+// largest exponent of each line or window is computed into it first (one read of
+// the input), so the tensor-core sweep reads its input once.
+// lineE_ready: lineE already holds the lines' exponents (launch_line_exp3, or
+// handed on; S.le_win = 0); no pre-pass.
 cudaError_t launch_sweep_tc(const Sweep &S, const TcFilter &F, int sch, int *status, int *lineE,
                             cudaStream_t st, bool lineE_ready = false);
 // Line exponents of narr n0 x n1 x n2 grids along all three axes in one read

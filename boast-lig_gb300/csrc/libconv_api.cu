@@ -6,6 +6,7 @@
 //  - multi-D entry points follow GenericConvolutionOperator#procedure
 //    (BigDFT/GenericConvolution2.rb:1934-2243) for transpose = 1
 //    (MagicFilter, wavelets) and transpose = 0 with the kinetic options.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -426,7 +427,7 @@ struct Scratch {
 // line, none of them padding), and n1 >= 32, so that each epilogue warp's 32
 // rows belong to at most two lines of k + 1 in every output column: k's line
 // i1 + n1 i2 and output e are k + 1's line i2 + n2 e at element i1.  Shorter
-// lines keep the pre-pass.  32 arrays of 128^3: the pre-pass takes 81 us, handing
+// lines keep the pre-pass, and so do most long periodic ones (below).  32 arrays of 128^3: the pre-pass takes 81 us, handing
 // on 5; 8 of 110^3 to 125^3: 20-31 us a pre-pass (Hamiltonian 1932 -> 1855 us).
 bool exp_handoff(const Plan &P, size_t k, int &n1, int &n2) {
     if (t_mode != LIBCONV_MODE_TC_EXACT || k + 1 >= P.steps.size()) return false;
@@ -443,12 +444,29 @@ bool exp_handoff(const Plan &P, size_t k, int &n1, int &n2) {
     if (len < 32 || lines % len) return false;
     // every element of A's output is written, and every one of B's lines is used
     if (A.qhi - A.qlo + 1 != A.out_ext || A.qlo != A.out_lo) return false;
+    // B's lines long enough for an exponent per window (tc_windows) take those in a
+    // pass of their own.  128 points are the exception: whole blocks of A's lines hold
+    // one of B's each
+    if (tc_windows(B) && !(A.kind == KCONV && A.bc == BC_PERIODIC && len == 128 && lines % 128 == 0 && A.out_ext % 64 == 0))
+        return false;
     const int used = B.bc == BC_SHRINK ? B.qhi + B.lowfil + B.ntaps - B.in_lo : B.n;
     if (used != B.in_ext) return false;
     if ((long long)B.nR != lines / len * A.out_ext * mA) return false;
     n1 = (int)len;
     n2 = (int)(lines / len);
     return true;
+}
+
+// Whether step k's line exponents come from the plan's shared pass over x.
+bool exp_shared(const Plan &P, size_t k) {
+    return t_mode == LIBCONV_MODE_TC_EXACT && P.exp3[0] > 0 && P.steps[k].exp_axis >= 0 && P.steps[k].src == B_X;
+}
+
+// Exponent windows per line of step k: where its own pass takes the exponents.
+int exp_windows(const Plan &P, size_t k) {
+    int n1, n2;
+    if (t_mode != LIBCONV_MODE_TC_EXACT || exp_shared(P, k) || (k > 0 && exp_handoff(P, k - 1, n1, n2))) return 0;
+    return tc_windows(P.steps[k].S);
 }
 
 // Elements of dot partials and of line exponents that run_plan(P) needs in
@@ -460,15 +478,15 @@ void plan_scratch(const Plan &P, size_t &ndot, size_t &nle) {
         const size_t n0 = P.exp3[0], n1 = P.exp3[1], n2 = P.exp3[2], na = P.exp3[3];
         nle = (n1 * n2 + n0 * n2 + n0 * n1) * na;
     }
-    for (const PlanStep &ps : P.steps) {
-        const Sweep &S = ps.S;
+    for (size_t k = 0; k < P.steps.size(); ++k) {
+        Sweep S = P.steps[k].S;
+        S.le_win = exp_windows(P, k);
         const bool tc = t_mode != LIBCONV_MODE_FP64 && sweep_tc_supported(S);
         if (S.has_dot) {
             const size_t nb = tc ? (size_t)sweep_tc_blocks(S) * kTcDotSlots * S.narr : (size_t)sweep_fp64_blocks(S);
             ndot += nb;                      // one reduction at the plan's end
         }
-        const bool shared = exact && P.exp3[0] > 0 && ps.exp_axis >= 0 && ps.src == B_X;
-        if (tc && exact && !shared && (size_t)sweep_tc_lines(S) > nle) nle = (size_t)sweep_tc_lines(S);
+        if (tc && exact && !exp_shared(P, k)) nle = std::max(nle, (size_t)sweep_tc_exps(S));
     }
     // a hand-off writes the next step's exponents beside the ones being read and
     // zeroes those of the step after
@@ -547,8 +565,11 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
     bool le_ready = false;
     if (!shared_exp) {
         size_t most = 0;
-        for (const PlanStep &ps : P.steps)
-            if ((size_t)sweep_tc_lines(ps.S) > most) most = (size_t)sweep_tc_lines(ps.S);
+        for (size_t k = 0; k < P.steps.size(); ++k) {
+            Sweep S = P.steps[k].S;
+            S.le_win = exp_windows(P, k);
+            most = std::max(most, (size_t)sweep_tc_exps(S));
+        }
         if (sc.le && sc.nle >= 3 * most) le[1] = sc.le + most, le[2] = sc.le + 2 * most;
     }
     // dot products: each step's partials in their own place, reduced at the end
@@ -561,6 +582,7 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
         S.x = bufs[ps.src];
         S.y = bufs[ps.dst];
         S.x2 = ps.src2 >= 0 ? bufs[ps.src2] : nullptr;
+        S.le_win = exp_windows(P, k);
         if (!S.x || !S.y || (ps.src2 >= 0 && !S.x2))
             return fail(LIBCONV_EARG, "null device buffer in plan");
         fold_arrays(S);
@@ -598,7 +620,7 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
             else tc_filter_split(h_ftab + S.ftab, flat, S.has_a ? S.a : 1.0, sch, F);
             S.has_a = 0;   // folded into the filter operands
             int *lineE = nullptr;
-            const bool shared = sch == SCH_EXACT && shared_exp && ps.exp_axis >= 0 && ps.src == B_X;
+            const bool shared = exp_shared(P, k);
             bool ready = shared, handed = false;
             if (shared) {
                 lineE = shared_exp + exp_off[ps.exp_axis];
@@ -1266,9 +1288,12 @@ int poisson_sweeps(int nord, int count, const int *idim, const int *nn, const in
         bufs[dst[k]] = y[k];
         P.steps.push_back(ps);
     }
-    // several axes of one grid: one exponent pass for all (its grid takes 8 lines a
-    // block along the second axis).  Divergence with cc, 256^3: 1175 -> 1075 us
-    if (count > 1 && nn[1] <= 8 * 65535) {
+    // several axes of one grid whose lines have one exponent each: one pass for all (its
+    // grid takes 8 lines a block along the second axis); long periodic axes take an
+    // exponent per window in passes of their own
+    bool windows = false;
+    for (const PlanStep &ps : P.steps) windows |= tc_windows(ps.S) > 0;
+    if (count > 1 && !windows && nn[1] <= 8 * 65535) {
         P.exp3[0] = nn[0]; P.exp3[1] = nn[1]; P.exp3[2] = nn[2]; P.exp3[3] = 1;
     }
     std::lock_guard<std::recursive_mutex> lk(g_mu);

@@ -13,6 +13,8 @@ namespace {
 int g_sms[64] = {0};
 }
 
+constexpr int kWindow = 64;                  // outputs of an exponent window (tc_windows)
+
 int sm_count() {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -104,6 +106,92 @@ __global__ void line_exp_kernel(const Sweep S, int plen, int *out) {
 __host__ __device__ __forceinline__ int line_exp_plen(const Sweep &S) {
     const int up = S.lowfil + S.ntaps - 1;
     return S.bc == BC_SHRINK ? S.qhi + up - S.in_lo + 1 : S.n;
+}
+
+// Exponents per line and window (Sweep::le_win): window w of a line is what its
+// outputs 64 w .. 64 w + 63 read, positions qlo + 64 w + lowfil - woff on, at most
+// 63 + ntaps + woff of them.  Contiguous lines: a warp per window, four of them at a
+// time; strided lines: a thread per line, a warp's windows one after another.  Windows
+// of one line are neighbours, so what two of them read comes from L1 or L2 the second
+// time.  by[0..2]: divisors wins, nL nR and nL.
+struct FastDiv {
+    uint32_t d, m, s;
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
+        return (uint32_t)(((unsigned long long)n * m) >> s);
+    }
+};
+struct WindowDivs { FastDiv wins, lines, left; };
+
+__global__ void __launch_bounds__(256) window_exp_kernel(const Sweep S, const WindowDivs by, int *out) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // the sweep's prologue may begin
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    if (S.le_next)                       // the exponents that the sweep will hand on
+        for (long long i = first; i < S.le_next_lines * S.narr; i += step) S.le_next[i] = 0;
+    const long long *xb = reinterpret_cast<const long long *>(S.x);
+    const uint32_t nlines = by.lines.d, total = nlines * (uint32_t)S.narr;
+    const int n = S.n, lane = threadIdx.x & 31;
+    const uint32_t wins = by.wins.d, warps = step >> 5;
+    constexpr uint32_t kExp = 0x7FF00000u;
+    auto start = [&](int w) { return S.qlo + kWindow * w + S.lowfil - S.woff; };
+    auto count = [&](int w) {
+        return min(kWindow + S.ntaps - 1 + S.woff, S.qhi + S.lowfil + S.ntaps - start(w));
+    };
+    auto field = [&](long long h) { return (uint32_t)((unsigned long long)h >> 32) & kExp; };
+    if (S.nL == 1) {
+        constexpr int L = 4, I = 3;                      // windows, and loads that cover one
+        const uint32_t units = total * wins;
+        for (uint32_t u = first >> 5; u < units; u += L * warps) {
+            long long h[L][I];
+            uint32_t at[L];
+#pragma unroll
+            for (int k = 0; k < L; ++k) {
+                const uint32_t v = min(u + k * warps, units - 1), line = by.wins(v), w = v - line * wins;
+                const uint32_t arr = by.lines(line);
+                const long long *base = xb + arr * S.x_arr + (long long)S.in_ext * (line - arr * nlines);
+                const int c = count(w);
+                at[k] = w * total + line;
+                int p = start(w) + lane;
+#pragma unroll
+                for (int i = 0; i < I; ++i) {
+                    const int q = p < 0 ? p + n : p >= n ? p - n : p;
+                    h[k][i] = lane + 32 * i < c ? base[q] : 0ll;
+                    p += 32;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < L; ++k) {
+                uint32_t m = 0;
+#pragma unroll
+                for (int i = 0; i < I; ++i) m = max(m, field(h[k][i]));
+                m = __reduce_max_sync(0xffffffffu, m);
+                if (lane == 0 && u + k * warps < units) out[at[k]] = (int)(m >> 20);
+            }
+        }
+    } else {
+        const uint32_t units = (total + 31) / 32 * wins;
+        for (uint32_t u = first >> 5; u < units; u += warps) {
+            const uint32_t block = by.wins(u), w = u - block * wins, line = block * 32 + lane;
+            if (line >= total) continue;
+            const uint32_t arr = by.lines(line), g = line - arr * nlines, r = by.left(g);
+            const long long *base = xb + arr * S.x_arr + (g - r * S.nL) + (long long)S.nL * S.in_ext * r;
+            const int c = count(w);
+            int p = start(w);
+            if (p < 0) p += n;
+            uint32_t m = 0;
+            for (int e = 0; e < c;) {                    // up to the line's end, then from its start
+                const int run = min(c - e, n - p);
+                const long long *q = base + (long long)S.nL * p;
+#pragma unroll 8
+                for (int i = 0; i < run; ++i) {
+                    m = max(m, field(*q));
+                    q += S.nL;
+                }
+                e += run;
+                p = 0;
+            }
+            out[w * total + line] = (int)(m >> 20);
+        }
+    }
 }
 
 // The same maxima for a batch of sweeps: blockIdx.y = sweep, its lines'
@@ -217,6 +305,18 @@ constexpr int kExpChunkHost = tck::kExpChunk;
 
 long long sweep_tc_lines(const Sweep &S) { return (long long)S.nL * S.nR * S.narr; }
 
+// A window's scale is its own, so small values far from a line's large ones keep 62
+// bits below their neighbours' magnitude, and an Inf or NaN spoils 64 outputs, not the
+// line.  Only where a line's exponents come from the sweep's own pass: handed-on and
+// shared ones are the line's, as are those of lines of less than a window, of other
+// boundaries and of wavelets.
+int tc_windows(const Sweep &S) {
+    if (S.kind != KCONV || S.bc != BC_PERIODIC || S.n < tck::kWindow - 16 + (S.ntaps + 30) / 16 * 16) return 0;
+    return (S.qhi - S.qlo + tck::kWindow) / tck::kWindow;
+}
+
+long long sweep_tc_exps(const Sweep &S) { return sweep_tc_lines(S) * (S.le_win > 0 ? S.le_win : 1); }
+
 cudaError_t launch_line_exp3(const double *x, int n0, int n1, int n2, int narr, int *e0, int *e1,
                              int *e2, cudaStream_t st, const int *active) {
     if (n0 < 1 || n1 < 1 || n2 < 1 || narr < 1 || narr > 65535) return cudaErrorInvalidValue;
@@ -271,19 +371,24 @@ static int window_slabs(const Sweep &S) {
 
 // Output blocks per strip, for `blocks` line blocks in the launch: the split
 // of the lines that gives the busiest CTA the least slabs to convert (its
-// strips times nb + W - 1); whole lines unless a launch has few of them.
+// strips times nb + W - 1); whole lines unless a launch has few of them.  With an
+// exponent per window (4 blocks) a strip is a window, or a half or a quarter of one.
 static int strip_blocks(const Sweep &S, long long blocks) {
     const int n = out_blocks(S), halo = window_slabs(S) - 1, sms = tck::sm_count();
     int best = n;
     long long cost = -1;
-    for (int seg = 1; seg <= n && seg <= 64; ++seg) {
-        const int nb = (n + seg - 1) / seg;
+    auto consider = [&](int nb) {
         const long long strips = blocks * ((n + nb - 1) / nb);
         const long long c = (strips + sms - 1) / sms * (nb + halo);
         if (cost < 0 || c < cost) {
             cost = c;
             best = nb;
         }
+    };
+    if (S.le_win > 0) {
+        for (int nb = tck::kWindow / 16; nb >= 1; nb /= 2) consider(nb);
+    } else {
+        for (int seg = 1; seg <= n && seg <= 64; ++seg) consider((n + seg - 1) / seg);
     }
     return best;
 }
@@ -464,16 +569,33 @@ cudaError_t launch_sweep_tc_batch(int kind, int ntaps, const Sweep &like, const 
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_sweep_tc(const Sweep &S, const TcFilter &F, int sch, int *status, int *lineE,
+cudaError_t launch_sweep_tc(const Sweep &S_in, const TcFilter &F, int sch, int *status, int *lineE,
                             cudaStream_t st, bool lineE_ready) {
+    Sweep S = S_in;
+    // contiguous periodic lines of a filter whose K blocks leave room: start
+    // the window on a 4-element boundary (32-byte aligned groups)
+    if (S.kind == KCONV && 16 * window_slabs(S) - 15 - S.ntaps >= 3 && S.nL == 1 && S.bc == BC_PERIODIC &&
+        S.n % 4 == 0 && S.in_ext % 4 == 0 && S.x_arr % 4 == 0 && (((uintptr_t)S.x) & 31) == 0)
+        S.woff = ((S.qlo + S.lowfil) % 4 + 4) % 4;
     if (sch == SCH_EXACT) {
+        if (S.le_win > 0 && (lineE_ready || !lineE)) return cudaErrorInvalidValue;
         if (lineE && !lineE_ready) {
-            const int plen = tck::line_exp_plen(S);
             const long long total = sweep_tc_lines(S);
-            const long long threads = S.nL == 1 ? total * 32 : total;
-            const long long want = (threads + 255) / 256;
+            // threads with something to do: a warp per contiguous line or window, a
+            // thread per strided line (and window)
+            const long long units = S.nL == 1 ? total : (total + 31) / 32;
+            const long long want = (units * (S.le_win > 0 ? S.le_win : 1) + 7) / 8;
             const int grid = (int)(want < 8LL * tck::sm_count() ? want : 8LL * tck::sm_count());
-            tck::line_exp_kernel<<<grid > 0 ? grid : 1, 256, 0, st>>>(S, plen, lineE);
+            if (S.le_win > 0) {
+                if (sweep_tc_exps(S) >= (1LL << 31)) return cudaErrorInvalidValue;   // 32-bit window numbers
+                tck::WindowDivs by;
+                fast_div((unsigned int)S.le_win, by.wins.d, by.wins.m, by.wins.s);
+                fast_div((unsigned int)(total / S.narr), by.lines.d, by.lines.m, by.lines.s);
+                fast_div((unsigned int)S.nL, by.left.d, by.left.m, by.left.s);
+                tck::window_exp_kernel<<<grid > 0 ? grid : 1, 256, 0, st>>>(S, by, lineE);
+            } else {
+                tck::line_exp_kernel<<<grid > 0 ? grid : 1, 256, 0, st>>>(S, tck::line_exp_plen(S), lineE);
+            }
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }

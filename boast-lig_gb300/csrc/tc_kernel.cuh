@@ -11,7 +11,9 @@
 //
 // Scheme SCH_EXACT (FP64-accurate, exact integer arithmetic on FP16 operands)
 //   * each line is scaled by the power of two above its largest magnitude
-//     (line_exp_kernel, or the sweep before: Sweep::le_next) to signed 62-bit integers X = x 2^(62-E) (|X| <=
+//     (line_exp_kernel, or the sweep before: Sweep::le_next), each window of 64
+//     outputs of a long periodic one by its own (window_exp_kernel, Sweep::le_win),
+//     to signed 62-bit integers X = x 2^(62-E) (|X| <=
 //     2^62, truncated toward zero); X is cut into 8 balanced byte digits
 //     d_0 (top) .. d_7 in [-128, 127], X = sum_s d_s 256^(7-s): the bytes
 //     of X + 0x8080808080808080 minus 128.  The operand keeps the bytes d_s +
@@ -32,7 +34,7 @@
 //   Dropped orders (k >= 8) weigh below 2^-70 of the product of the line and
 //   filter scales; the data truncation (2^-62 of the line scale) and the
 //   final roundings stay below the rounding of an FP64 FMA chain.
-//   Lines never share a scale; a line holding an Inf or NaN gives NaN.
+//   Lines never share a scale; a line or window holding an Inf or NaN gives NaN.
 //
 // Split-precision schemes (FP32-class accuracy, reported per operator)
 //   * every element is rounded to FP32 (magnitudes outside the normal float
@@ -710,11 +712,16 @@ sweep_tc_kernel(const __grid_constant__ Sweep S0, const __grid_constant__ TcFilt
                     ps = ps < 0 ? ps + last : ps >= last ? ps - last : ps;
                 }
             }
-            // largest exponent field of the line (line_exp_kernel); a row past the
-            // last line is all zeros under any scale
+            // largest exponent field of the line, or of the strip's window of it; a row
+            // past the last line is all zeros under any scale
             mx = 0x7FE;
             if (!valid) left = 0;
-            else if (SCH == SCH_EXACT) mx = lineE[S->le_off + (long long)loc.arr * nlines + g];
+            else if (SCH == SCH_EXACT) {
+                long long le = S->le_off + (long long)loc.arr * nlines + g;
+                if (!BATCH && KIND == KCONV && S->le_win)            // the window (4 blocks) of the strip
+                    le += (long long)((loc.seg * S->seg_blocks) >> 2) * nlines * S->narr;
+                mx = lineE[le];
+            }
         };
         long long strip = skip_inactive(blockIdx.x);
         uint32_t slot = 0, par = 1;                      // ring position; empty phase to wait for
@@ -1398,11 +1405,6 @@ cudaError_t launch(const Sweep &S_in, const TcFilter &F, int *status, const int 
     using G = Geom<KIND, NT, SCH>;
     Sweep S = S_in;
     if (!tc_prepare(S)) return cudaErrorInvalidValue;
-    // contiguous periodic lines of a filter whose K blocks leave room: start
-    // the window on a 4-element boundary (32-byte aligned groups)
-    if (KIND == KCONV && G::KB - 15 - NT >= 3 && S.nL == 1 && S.bc == BC_PERIODIC && S.n % 4 == 0 &&
-        S.in_ext % 4 == 0 && S.x_arr % 4 == 0 && (((uintptr_t)S.x) & 31) == 0)
-        S.woff = ((S.qlo + S.lowfil) % 4 + 4) % 4;
     if (S.has_dot || S.has_ax || S.ay_mode || (S.x2 && NT != 29))
         return launch_form<KIND, NT, SCH, FORM_ANY>(S, F, status, lineE, st);
     if constexpr (KIND == KCONV && NT == 29)
