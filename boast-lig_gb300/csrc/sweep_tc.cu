@@ -110,7 +110,7 @@ __host__ __device__ __forceinline__ int line_exp_plen(const Sweep &S) {
 
 // Exponents per line and window (Sweep::le_win): window w of a line is what its
 // outputs 64 w .. 64 w + 63 read, positions qlo + 64 w + lowfil - woff on, at most
-// 63 + ntaps + woff of them.  Contiguous lines: a warp per window, four of them at a
+// 63 + ntaps + woff of them.  Contiguous lines: a warp per window, two of them at a
 // time; strided lines: a thread per line, a warp's windows one after another.  Windows
 // of one line are neighbours, so what two of them read comes from L1 or L2 the second
 // time.  by[0..2]: divisors wins, nL nR and nL.
@@ -122,7 +122,7 @@ struct FastDiv {
 };
 struct WindowDivs { FastDiv wins, lines, left; };
 
-__global__ void __launch_bounds__(256) window_exp_kernel(const Sweep S, const WindowDivs by, int *out) {
+__global__ void __launch_bounds__(256, 8) window_exp_kernel(const Sweep S, const WindowDivs by, int *out) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // the sweep's prologue may begin
     const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     if (S.le_next)                       // the exponents that the sweep will hand on
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256) window_exp_kernel(const Sweep S, const Wi
     };
     auto field = [&](long long h) { return (uint32_t)((unsigned long long)h >> 32) & kExp; };
     if (S.nL == 1) {
-        constexpr int L = 4, I = 3;                      // windows, and loads that cover one
+        constexpr int L = 2, I = 3;                      // windows, and loads that cover one
         const uint32_t units = total * wins;
         for (uint32_t u = first >> 5; u < units; u += L * warps) {
             long long h[L][I];
