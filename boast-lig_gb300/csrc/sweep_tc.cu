@@ -4,6 +4,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "lcg_tc.cuh"
 
 namespace lcg {
@@ -388,7 +390,11 @@ static int strip_blocks(const Sweep &S, long long blocks) {
     if (S.le_win > 0) {
         for (int nb = tck::kWindow / 16; nb >= 1; nb /= 2) consider(nb);
     } else {
-        for (int seg = 1; seg <= n && seg <= 64; ++seg) consider((n + seg - 1) / seg);
+        // as many segments as give every CTA a strip: 64 at most left 88 of 152 SMs idle
+        // for a few long lines (one of 10^6 points, kinetic filter, BF16x3: 2540 us, now
+        // 1084; 1217 as tiles of 64 outputs)
+        const long long most = std::max<long long>(64, (sms + blocks - 1) / blocks);
+        for (int seg = 1; seg <= n && seg <= most; ++seg) consider((n + seg - 1) / seg);
     }
     return best;
 }

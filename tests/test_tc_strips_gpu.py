@@ -110,3 +110,27 @@ def test_partial_sums_and_terms(pkg, O, n, a_x, a_y):
         pkg.Kernel('d_kin').run(3, n, bcs, x, yg, w, w, a, a_x, a_y)
         assert O.call('oracle_d_kin', 3, n, bcs, x, yo, np.zeros(N), np.zeros(N), np.array(a), a_x, a_y) == 0
         assert np.abs(yg - yo).max() <= TOL * np.abs(yo).max(), bcs
+
+
+# 128 lines or fewer: lines are cut into as many segments as there are SMs, the last one shorter
+@pytest.mark.parametrize('mode,tol', [('MODE_TC_EXACT', 1e-13), ('MODE_TC_BF16X3', 1e-5)])
+@pytest.mark.parametrize('lines,idim', [(1, 0), (3, 0), (2, 1), (130, 1)])
+@pytest.mark.parametrize('op', ['d_s0s0_1d_sym8_md', 'd_s0s0_1d_sym8_d1', 'd_s0s1_1d_sym8', 'd_s1s0_1d_sym8'])
+def test_few_long_lines(pkg, O, op, lines, idim, mode, tol):
+    wav = op in ('d_s0s1_1d_sym8', 'd_s1s0_1d_sym8')
+    m, n = (2, 6007) if wav else (1, 12007)
+    shape = [n, n]
+    shape[1 - idim] = lines
+    r = np.random.default_rng(n + lines)
+    x = r.uniform(-1, 1, m * m * n * lines)
+    for bc in (0, 1, 2):
+        ny = list(shape)
+        ny[idim] += TAPS[op] - 1 if bc == 1 else 0
+        y = np.zeros(m * m * int(np.prod(ny)))
+        yo = np.zeros_like(y)
+        args = [2, idim, shape, bc, shape, ny, 1, x]
+        tail = (1.0, 0.0) if wav else (0.7, 0.0, 0.0)
+        with pkg.mode(getattr(pkg, mode)):
+            pkg.Kernel(op).run(*args, y, *tail)
+        assert O.call('oracle_' + op, *args, yo, *tail) == 0
+        assert np.abs(y - yo).max() <= tol * np.abs(yo).max(), bc
