@@ -85,10 +85,11 @@ __device__ __forceinline__ void line_exp_lines(const Sweep &S, int plen, int *ou
             const long long arr = t / nlines, g = t % nlines;
             const long long l = g % S.nL, r = g / S.nL;
             const long long *base = xb + arr * S.x_arr + l + (long long)S.nL * pext * r;
-            int mx = 0;
+            uint32_t mx = 0;
+#pragma unroll 8
             for (int e = 0; e < count; ++e)
-                mx = max(mx, (int)(((unsigned long long)base[offset(e) * S.nL] >> 52) & 0x7FF));
-            out[t] = mx;
+                mx = max(mx, (uint32_t)((unsigned long long)base[offset(e) * S.nL] >> 32) & 0x7FF00000u);
+            out[t] = (int)(mx >> 20);
         }
     }
 }
