@@ -242,7 +242,16 @@ cudaError_t launch_qc(const Sweep &S, cudaStream_t st) {
     const int nq = S.qhi - S.qlo + 1;
     dim3 grid((unsigned)((nlines + kLines - 1) / kLines), (unsigned)((nq + QC - 1) / QC),
               (unsigned)S.narr);
-    sweep_fp64_kernel<KIND, NT, QC><<<grid, kThreads, 0, st>>>(S);
+    // convolutions in chunks of 64: five blocks an SM, held to that by unused shared
+    // memory.  Five saturate the FP64 pipe, and what is left over after whole rounds
+    // is the longer part of a smaller round; eight (all that registers allow) were 2-11 %
+    // slower where the last round is short (d2, 4 x 96^3 223 us, 237 with eight; MagicFilter
+    // of 100 lines of 20000, 88 and 96), six up to 8 % where seven a SM are all
+    // (kinetic, 8 x 64^3)
+    constexpr size_t own = sizeof(double) * ((QC + NT - 1) * kPad + kWarps);
+    constexpr size_t unused = KIND == KCONV && QC == 64 ? 40 * 1024 - own : 0;
+    static_assert(own < 40 * 1024 || KIND != KCONV || QC != 64, "shared memory of a fifth of an SM");
+    sweep_fp64_kernel<KIND, NT, QC><<<grid, kThreads, unused, st>>>(S);
     return cudaGetLastError();
 }
 
