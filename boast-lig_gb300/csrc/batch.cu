@@ -47,7 +47,8 @@ struct OpConfig {
     int engine = LIBCONV_ENGINE_FP64_Q64;
     int order[3] = {-1, 0, 0};               // MF: order[0] = -1 -> rotating sweeps
     std::vector<Stage> stages;
-    int exp3_tiles = 0;                      // > 0: one exponent pass for all stages, blocks per grid
+    int exp3_tiles = 0, exp3_seg = 1;        // tiles > 0: one exponent pass for all stages; its column
+                                             // tiles of the largest grid, and their segments
     int stage_of(int axis) const { return order[0] == axis ? 0 : order[1] == axis ? 1 : 2; }
 };
 
@@ -172,7 +173,7 @@ int build_stages(const libconv_batch *b, int o, int engine, const int *ord, OpCo
                     contiguous |= S.nL == 1;
                 }
                 st.lines = lines;
-                st.exp_blocks = line_exp_batch_blocks(most, contiguous);
+                st.exp_blocks = line_exp_batch_blocks(most, contiguous, G);
                 if (cudaMalloc(&st.d_lineE, sizeof(int) * (size_t)(lines > 0 ? lines : 1)) != cudaSuccess) {
                     cudaGetLastError();
                     return report(LIBCONV_ENOMEM, "batch line-exponent allocation failed");
@@ -197,10 +198,13 @@ int build_stages(const libconv_batch *b, int o, int engine, const int *ord, OpCo
     // them (128 grids, axes 24-72, MagicFilter and kinetic: 1485 us with one each, 1338)
     if (tc && scheme_of(b->mode) == SCH_EXACT && o == LIBCONV_BATCH_OP_KIN) {
         const std::vector<Sweep> &A1 = C.stages[C.stage_of(1)].sw;
+        int n2 = 1;
         for (const Sweep &S : A1) {
             const long long tiles = (long long)((S.nL + 31) / 32) * ((S.n + 7) / 8);
             if (tiles > C.exp3_tiles) C.exp3_tiles = (int)(tiles < 256 ? tiles : 256);
+            n2 = std::max(n2, S.nR);
         }
+        C.exp3_seg = line_exp3_batch_segments(C.exp3_tiles, n2, G);
     }
     return LIBCONV_OK;
 }
@@ -254,7 +258,8 @@ int launch_op(libconv_batch *b, int o, int *status, cudaStream_t stream) {
     if (C.exp3_tiles) {
         const Stage &A0 = C.stages[C.stage_of(0)], &A1 = C.stages[C.stage_of(1)], &A2 = C.stages[C.stage_of(2)];
         const cudaError_t e = launch_line_exp3_batch(A0.d_desc, A1.d_desc, A2.d_desc, b->ngrids, A0.d_lineE, A0.lines,
-                                                     A1.d_lineE, A1.lines, A2.d_lineE, C.exp3_tiles, stream);
+                                                     A1.d_lineE, A1.lines, A2.d_lineE, A2.lines, C.exp3_tiles,
+                                                     C.exp3_seg, stream);
         if (e != cudaSuccess) return report_cuda(e, "batched line exponent launch");
     }
     for (Stage &st : C.stages) {

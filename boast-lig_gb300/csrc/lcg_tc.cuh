@@ -84,14 +84,15 @@ cudaError_t launch_sweep_tc_batch(int kind, int ntaps, const Sweep &like, const 
                                   int *lineE, int exp_blocks, cudaStream_t st, bool lineE_ready = false);
 // Line exponents along all three axes of the grids of a batch in one read of x:
 // descriptors (device) of the non-rotating sweeps along axes 0, 1, 2, exponent
-// arrays of lines0, lines1 (and the third axis's) ints, at most tiles blocks of 32
-// x 8 columns per grid.
+// arrays of lines0, lines1 and lines2 ints; at most tiles tiles of 32 x 8 columns per
+// grid, each in nseg segments of the third axis (line_exp3_batch_segments).
 cudaError_t launch_line_exp3_batch(const Sweep *d0, const Sweep *d1, const Sweep *d2, int nsweeps, int *e0,
-                                   long long lines0, int *e1, long long lines1, int *e2, int tiles,
-                                   cudaStream_t st);
-// Blocks per sweep of the batched line-exponent pass for sweeps whose largest
+                                   long long lines0, int *e1, long long lines1, int *e2, long long lines2, int tiles,
+                                   int nseg, cudaStream_t st);
+int line_exp3_batch_segments(int tiles, int n2, int ngrids);
+// Blocks per sweep of the batched line-exponent pass for ngrids sweeps whose largest
 // line count (lines x narr) is max_lines, contiguous lines (nL == 1) or not.
-int line_exp_batch_blocks(long long max_lines, bool contiguous);
+int line_exp_batch_blocks(long long max_lines, bool contiguous, int ngrids);
 
 namespace tck {
 // 17-tap convolution (the Poisson finite differences), every scheme; its own

@@ -290,16 +290,21 @@ line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg,
 
 // The same for the grids of a batch: d0, d1, d2 describe the non-rotating sweeps
 // along axes 0, 1, 2 of each grid (all read the same x), whose exponents start at
-// their le_off.  blockIdx.y = grid.
+// their le_off.  blockIdx.y = grid, whose 32 x 8 columns and nseg segments of the third
+// axis its blocks share.
 __global__ void __launch_bounds__(256)
 line_exp3_batch_kernel(const Sweep *__restrict__ d0, const Sweep *__restrict__ d1, const Sweep *__restrict__ d2,
-                       int *__restrict__ e0, int *__restrict__ e1, int *__restrict__ e2) {
+                       int *__restrict__ e0, int *__restrict__ e1, int *__restrict__ e2, int nseg) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const Sweep &S = d1[blockIdx.y];
     const int n0 = S.nL, n1 = S.n, n2 = S.nR, gx = (n0 + 31) / 32, tiles = gx * ((n1 + 7) / 8);
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x)
-        line_exp3_block(S.x, n0, n1, n2, t % gx * 32, t / gx * 8, 0, n2, e0 + d0[blockIdx.y].le_off, e1 + S.le_off,
-                        e2 + d2[blockIdx.y].le_off);
+    const int seglen = (n2 + nseg - 1) / nseg;
+    for (int t = blockIdx.x; t < tiles * nseg; t += gridDim.x) {
+        const int tile = t % tiles, zb = t / tiles * seglen;
+        if (zb < n2)
+            line_exp3_block(S.x, n0, n1, n2, tile % gx * 32, tile / gx * 8, zb, min(n2, zb + seglen),
+                            e0 + d0[blockIdx.y].le_off, e1 + S.le_off, e2 + d2[blockIdx.y].le_off);
+    }
 }
 
 }  // namespace tck
@@ -539,24 +544,36 @@ bool sweep_tc_batch_supported(int kind, int ntaps) {
     return kind == KCONV && (ntaps == 16 || ntaps == 29);
 }
 
-int line_exp_batch_blocks(long long max_lines, bool contiguous) {
+int line_exp_batch_blocks(long long max_lines, bool contiguous, int ngrids) {
     // four lines a warp; each block first waits for its descriptor, so not too many
-    // of them (128 grids, axes 24-72: a MagicFilter and kinetic run takes 1349, 1306,
-    // 1319 and 1384 us with at most 16, 32, 64 and 256 per grid)
+    // of them (128 grids, axes 24-72, a MagicFilter and kinetic run: 1349, 1306, 1319 and
+    // 1384 us with at most 16, 32, 64 and 256 per grid), but two for every SM in all:
+    // with these and the segments of the shared pass, runs over one grid of 72^3
+    // 126 -> 87 us, two 158 -> 123, three of 120^3 579 -> 419, four of 40-72 125 -> 113
     const long long threads = contiguous ? max_lines * (32 / 4) : max_lines;
     const long long want = (threads + 255) / 256;
-    return (int)(want < 1 ? 1 : want > 32 ? 32 : want);
+    const long long most = std::max<long long>(32, (2LL * tck::sm_count() + ngrids - 1) / ngrids);
+    return (int)(want < 1 ? 1 : want > most ? most : want);
 }
 
 cudaError_t launch_line_exp3_batch(const Sweep *d0, const Sweep *d1, const Sweep *d2, int nsweeps, int *e0,
-                                   long long lines0, int *e1, long long lines1, int *e2, int tiles,
-                                   cudaStream_t st) {
+                                   long long lines0, int *e1, long long lines1, int *e2, long long lines2, int tiles,
+                                   int nseg, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(e0, 0, (size_t)lines0 * sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(e1, 0, (size_t)lines1 * sizeof(int), st);
+    if (e == cudaSuccess && nseg > 1) e = cudaMemsetAsync(e2, 0, (size_t)lines2 * sizeof(int), st);
     if (e != cudaSuccess) return e;
-    tck::line_exp3_batch_kernel<<<dim3(tiles < 1 ? 1 : tiles > 256 ? 256 : tiles, nsweeps), 256, 0, st>>>(d0, d1, d2, e0,
-                                                                                                     e1, e2);
+    const int blocks = std::min(256, tiles * nseg);
+    tck::line_exp3_batch_kernel<<<dim3(blocks < 1 ? 1 : blocks, nsweeps), 256, 0, st>>>(d0, d1, d2, e0, e1, e2, nseg);
     return cudaGetLastError();
+}
+
+// Segments of the third axis (n2 long) that give ngrids grids of `tiles` 32 x 8 column
+// tiles two blocks for every SM; chunks of 8 planes are the shortest.
+int line_exp3_batch_segments(int tiles, int n2, int ngrids) {
+    const long long blocks = std::max(1LL, (long long)tiles * ngrids), want = 2LL * tck::sm_count();
+    const long long most = (n2 + kExpChunkHost - 1) / kExpChunkHost;
+    return (int)std::max(1LL, std::min(most, (want + blocks - 1) / blocks));
 }
 
 cudaError_t launch_sweep_tc_batch(int kind, int ntaps, const Sweep &like, const Sweep *descs, const long long *prefix,
