@@ -6,6 +6,7 @@
 //  - multi-D entry points follow GenericConvolutionOperator#procedure
 //    (BigDFT/GenericConvolution2.rb:1934-2243) for transpose = 1
 //    (MagicFilter, wavelets) and transpose = 0 with the kinetic options.
+#include <cuda_fp16.h>
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
@@ -1447,6 +1448,21 @@ int libconv_gb300_selftest_wait(int wait_us, void *stream) {
                                                                   1000ull * (unsigned long long)wait_us);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LIBCONV_OK : cuda_fail(e, "self-test launch");
+}
+
+int libconv_gb300_selftest_digits(int kind, const double *taps, int ntaps, double a, int *digits, int *ef,
+                                  long long *k64, unsigned *k67) {
+    if (kind < KCONV || kind > KREC || !taps || ntaps < 1 || ntaps > TcFilter::kMaxTaps || (kind != KCONV && ntaps % 4) ||
+        !digits || !ef || !k64 || !k67)
+        return fail(LIBCONV_EARG, "kind in [0, 2], ntaps in [1, %d], no null array", TcFilter::kMaxTaps);
+    TcFilter F;
+    tc_filter_digits(kind, taps, ntaps, a, F);
+    for (int t = 0; t < TcFilter::kSlices; ++t)
+        for (int i = 0; i < ntaps; ++i)
+            digits[t * ntaps + i] = (int)(__half2float(__ushort_as_half((unsigned short)F.dig[t][i])) / 256.0f);
+    *ef = F.ef;
+    for (int c = 0; c < 2; ++c) k64[c] = F.k64[c], k67[c] = F.k67[c];
+    return LIBCONV_OK;
 }
 
 int libconv_gb300_fp64_peak(int iters, double *tflops, void *stream) {

@@ -94,6 +94,13 @@ int libconv_gb300_check(void *stream);
  * gives up after 2 s of the same timer.  (The network layers' waits: 4e9 SM
  * clock cycles, about 2 s at the maximum clock, longer at lower clocks.) */
 int libconv_gb300_selftest_wait(int wait_us, void *stream);
+/* Self-test of the exact sweeps' filter operands (host only): the eight digit
+ * planes of a * taps[0..ntaps) (digits[8][ntaps], top digit first), the
+ * exponent ef of their scale (a tap = 2^(ef-62) sum_t digit_t 256^(7-t)) and,
+ * per output channel, the constants of the recombination (k64[2], k67[2]).
+ * kind: 0 convolution, 1 wavelet analysis, 2 synthesis (taps LE|LO|HE|HO). */
+int libconv_gb300_selftest_digits(int kind, const double *taps, int ntaps, double a, int *digits,
+                                  int *ef, long long *k64, unsigned *k67);
 /* Diagnostic, no counterpart in the reference: measured FP64 FMA throughput
  * of this GPU (the roof of the plain FP64 sweeps).  Runs 8 independent FMA
  * chains of `iters` steps in 8 x SMs blocks of 256 threads on `stream`, times
