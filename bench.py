@@ -655,6 +655,31 @@ def cpu_model():
     return 'unknown'
 
 
+def link_rates(torch, src, dst, dev):
+    """GB/s of plain copies of the host-pointer calls' own pinned buffers, host to device, device to
+    host and both at once (the best of four each): what the end-to-end value ran on."""
+    n = min(src.numel(), dst.numel())
+    a, b = (torch.empty(n, dtype=torch.float64, device=dev) for _ in range(2))
+    streams = [torch.cuda.Stream(dev), torch.cuda.Stream(dev)]
+
+    def rate(h2d, d2h):
+        best = float('inf')
+        for _ in range(4):
+            torch.cuda.synchronize(dev)
+            t0 = time.perf_counter()
+            if h2d:
+                with torch.cuda.stream(streams[0]):
+                    a.copy_(src[:n], non_blocking=True)
+            if d2h:
+                with torch.cuda.stream(streams[1]):
+                    dst[:n].copy_(b, non_blocking=True)
+            torch.cuda.synchronize(dev)
+            best = min(best, time.perf_counter() - t0)
+        return 8.0 * n * (h2d + d2h) / best / 1e9
+
+    return {'h2d': rate(1, 0), 'd2h': rate(0, 1), 'both': rate(1, 1)}
+
+
 def cpu_timed(W, B, hx, repeats=5, seconds=None):
     """The oracle restatement's -O3 OpenMP timing build on the workload's own
     batch: all host threads over the B grids of hx (one grid per thread at a
@@ -1467,8 +1492,8 @@ def run_poisson(args, W):
                      'achieved_gbs': W.bytes_per_pt * N / step_s / 1e9,
                      'frac': W.bytes_per_pt * N / step_s / 1e9 / pk['hbm']}}
     # six sweeps, the edge kernels of the two sweeps along the non-periodic axis and the cc
-    # kernel; in the exact mode a line-exponent pass per component
-    launches = {'tc_exact': 12, 'fp64': 9}.get(args.mode, 9)
+    # kernel; in the exact mode an exponent pass before each sweep (the periodic ones' per window)
+    launches = {'tc_exact': 15, 'fp64': 9}.get(args.mode, 9)
     exact = args.mode in ('fp64', 'tc_exact')
     line = {'metric': W.metric, 'value': value, 'unit': UNIT, 'n_gpus': world, 'steps': args.steps,
             'warmup': max(args.warmup, 3), 'ms_per_step': ms / args.steps,
@@ -1595,7 +1620,8 @@ def run_gpu(args):
                 'in_pts_per_s': B * 64 ** 3 / (g_ms / 1e3), 'out_pts_per_s': B * 79 ** 3 / (g_ms / 1e3)}
 
     # e2e: the public host-pointer C-ABI with pinned host buffers, copies inside
-    ho0 = torch.empty(B * max(Ni, No), dtype=torch.float64, pin_memory=True).numpy()
+    pin0 = torch.empty(B * max(Ni, No), dtype=torch.float64, pin_memory=True)
+    ho0 = pin0.numpy()
     ho1 = torch.empty(B * max(Ni, No), dtype=torch.float64, pin_memory=True).numpy()
     W.host_step(pkg, B, hx, ho0, ho1)
     barrier()
@@ -1611,7 +1637,8 @@ def run_gpu(args):
     else:
         h2d, d2h = B * (Ni + No) * 8, B * (Ni + No) * 8
     e2e = {'value': pts_step / e_t, 'unit': UNIT, 'h2d_bytes_per_step': h2d,
-           'd2h_bytes_per_step': d2h, 'note': W.e2e_note}
+           'd2h_bytes_per_step': d2h, 'plain_copy_gbs': link_rates(torch, host_x, pin0, dev),
+           'note': W.e2e_note}
 
     # roofline of the dominant kernel
     pk = peaks()
