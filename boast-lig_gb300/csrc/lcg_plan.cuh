@@ -27,6 +27,7 @@ struct Plan {
     int ndot = 1;                     // dot outputs (one per kinetic direction for ekin)
     int exp3[4] = {0, 0, 0, 0};       // n0, n1, n2, narr of the x grid whose line exponents
                                       // the exact tensor-core steps share (0: none)
+    int exp3_wins[3] = {0, 0, 0};     // exponent windows of its axes (0: one per line)
     const int *active = nullptr;      // device flags per array: 0 = skip it (no dot plans)
 };
 

@@ -60,15 +60,18 @@ long long sweep_tc_exps(const Sweep &S);
 // lineE (exact scheme, or null): device scratch of sweep_tc_exps(S) ints; the
 // largest exponent of each line or window is computed into it first (one read of
 // the input), so the tensor-core sweep reads its input once.
-// lineE_ready: lineE already holds the lines' exponents (launch_line_exp3, or
-// handed on; S.le_win = 0); no pre-pass.
+// lineE_ready: lineE already holds the exponents (launch_line_exp3, or the lines'
+// handed on); no pre-pass.
 cudaError_t launch_sweep_tc(const Sweep &S, const TcFilter &F, int sch, int *status, int *lineE,
                             cudaStream_t st, bool lineE_ready = false);
 // Line exponents of narr n0 x n1 x n2 grids along all three axes in one read
 // of x (e0: n1 n2 narr, e1: n0 n2 narr, e2: n0 n1 narr ints), in the line
-// order of the non-rotating sweeps along axes 0, 1, 2.  active (or null):
+// order of the non-rotating sweeps along axes 0, 1, 2; wins (or null): the axes'
+// exponent windows (tc_windows; 0: one exponent per line), each axis's ints times
+// as many, for sweeps that line_exp3_windows takes.  active (or null):
 // grids with active[a] == 0 are skipped (their entries stay 0).
-cudaError_t launch_line_exp3(const double *x, int n0, int n1, int n2, int narr, int *e0, int *e1,
+bool line_exp3_windows(const Sweep &S);
+cudaError_t launch_line_exp3(const double *x, int n0, int n1, int n2, int narr, const int *wins, int *e0, int *e1,
                              int *e2, cudaStream_t st, const int *active = nullptr);
 long long sweep_tc_lines(const Sweep &S);
 // Strips of one sweep (the unit a batched launch numbers consecutively).

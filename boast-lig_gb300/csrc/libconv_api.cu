@@ -463,11 +463,19 @@ bool exp_shared(const Plan &P, size_t k) {
     return t_mode == LIBCONV_MODE_TC_EXACT && P.exp3[0] > 0 && P.steps[k].exp_axis >= 0 && P.steps[k].src == B_X;
 }
 
-// Exponent windows per line of step k: where its own pass takes the exponents.
+// Exponent windows per line of step k: of the shared pass, or of its own.
 int exp_windows(const Plan &P, size_t k) {
     int n1, n2;
-    if (t_mode != LIBCONV_MODE_TC_EXACT || exp_shared(P, k) || (k > 0 && exp_handoff(P, k - 1, n1, n2))) return 0;
-    return tc_windows(P.steps[k].S);
+    if (t_mode != LIBCONV_MODE_TC_EXACT) return 0;
+    if (exp_shared(P, k)) return P.exp3_wins[P.steps[k].exp_axis];
+    return k > 0 && exp_handoff(P, k - 1, n1, n2) ? 0 : tc_windows(P.steps[k].S);
+}
+
+// Ints of the shared pass's exponents along axis k.
+size_t exp3_size(const Plan &P, int k) {
+    size_t c = (size_t)P.exp3[3] * std::max(P.exp3_wins[k], 1);
+    for (int i = 0; i < 3; ++i) if (i != k) c *= (size_t)P.exp3[i];
+    return c;
 }
 
 // Elements of dot partials and of line exponents that run_plan(P) needs in
@@ -475,10 +483,7 @@ int exp_windows(const Plan &P, size_t k) {
 void plan_scratch(const Plan &P, size_t &ndot, size_t &nle) {
     ndot = nle = 0;
     const bool exact = t_mode == LIBCONV_MODE_TC_EXACT;
-    if (exact && P.exp3[0] > 0) {
-        const size_t n0 = P.exp3[0], n1 = P.exp3[1], n2 = P.exp3[2], na = P.exp3[3];
-        nle = (n1 * n2 + n0 * n2 + n0 * n1) * na;
-    }
+    if (exact && P.exp3[0] > 0) nle = exp3_size(P, 0) + exp3_size(P, 1) + exp3_size(P, 2);
     for (size_t k = 0; k < P.steps.size(); ++k) {
         Sweep S = P.steps[k].S;
         S.le_win = exp_windows(P, k);
@@ -550,11 +555,10 @@ int run_plan(const Plan &P, double *const bufs[4], const Scratch &sc, double *do
     int *shared_exp = nullptr;
     long long exp_off[3] = {0, 0, 0};
     if (t_mode == LIBCONV_MODE_TC_EXACT && P.exp3[0] > 0) {
-        const long long n0 = P.exp3[0], n1 = P.exp3[1], n2 = P.exp3[2], na = P.exp3[3];
-        exp_off[1] = n1 * n2 * na;
-        exp_off[2] = exp_off[1] + n0 * n2 * na;
+        exp_off[1] = (long long)exp3_size(P, 0);
+        exp_off[2] = exp_off[1] + (long long)exp3_size(P, 1);
         shared_exp = sc.le;
-        cudaError_t e = launch_line_exp3(bufs[B_X], (int)n0, (int)n1, (int)n2, (int)na, shared_exp,
+        cudaError_t e = launch_line_exp3(bufs[B_X], P.exp3[0], P.exp3[1], P.exp3[2], P.exp3[3], P.exp3_wins, shared_exp,
                                          shared_exp + exp_off[1], shared_exp + exp_off[2], st, P.active);
         if (e != cudaSuccess) return cuda_fail(e, "line exponent launch");
     }
@@ -1289,13 +1293,14 @@ int poisson_sweeps(int nord, int count, const int *idim, const int *nn, const in
         bufs[dst[k]] = y[k];
         P.steps.push_back(ps);
     }
-    // several axes of one grid whose lines have one exponent each: one pass for all (its
-    // grid takes 8 lines a block along the second axis); long periodic axes take an
-    // exponent per window in passes of their own
-    bool windows = false;
-    for (const PlanStep &ps : P.steps) windows |= tc_windows(ps.S) > 0;
-    if (count > 1 && !windows && nn[1] <= 8 * 65535) {
+    // several axes of one grid: one exponent pass for all (its grid takes 8 lines a
+    // block along the second axis, and windows of whole pieces of 8 elements only).
+    // Divergence with cc, 256^3: 1209 us with a pass before each sweep, 1086
+    bool together = count > 1 && nn[1] <= 8 * 65535;
+    for (const PlanStep &ps : P.steps) together = together && (!tc_windows(ps.S) || line_exp3_windows(ps.S));
+    if (together) {
         P.exp3[0] = nn[0]; P.exp3[1] = nn[1]; P.exp3[2] = nn[2]; P.exp3[3] = 1;
+        for (const PlanStep &ps : P.steps) P.exp3_wins[ps.exp_axis] = tc_windows(ps.S);
     }
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     int rc;

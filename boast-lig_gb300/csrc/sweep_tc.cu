@@ -220,10 +220,37 @@ __global__ void line_exp_batch_kernel(const Sweep *__restrict__ descs, int *out)
 // combined across blocks with atomicMax (e0, e1 and, with several segments,
 // e2 zeroed first).
 constexpr int kExpChunk = 8;
+// Exponent windows of the three axes (0: the axis has one exponent per line), each
+// axis's lines in all grids, and its pieces of 8.
+struct Exp3Windows {
+    int wins[3] = {0, 0, 0};
+    long long lines[3] = {0, 0, 0};
+};
+
+// Raise to m the exponent of the line at e, or those of its windows that read piece c
+// (elements 8 c .. 8 c + 7 of n): a 17-tap window, elements 64 w - 8 .. 64 w + 71, is
+// ten such pieces, the first and the last of them its neighbours' too.
+__device__ __forceinline__ void exp3_edges(int *e, int c, int n, int wins, long long lines, int m) {
+    const int w = c >> 3;
+    if ((c & 7) == 0) atomicMax(e + (w ? w - 1 : wins - 1) * lines, m);
+    if ((c & 7) == 7 || 8 * (c + 1) >= n) atomicMax(e + (w + 1 < wins ? w + 1 : 0) * lines, m);
+}
+template <bool WIN>
+__device__ __forceinline__ void exp3_raise(int *e, int c, int n, int wins, long long lines, int m) {
+    if (!WIN || !wins) {
+        atomicMax(e, m);
+        return;
+    }
+    atomicMax(e + (c >> 3) * lines, m);
+    exp3_edges(e, c, n, wins, lines, m);
+}
+
 // The block's 32 i0 x 8 i1 columns from (b0, b1) on, planes [zb, ze) of one grid.
+// WIN: some axis has windows (its extent and zb are multiples of 8).
+template <bool WIN>
 __device__ __forceinline__ void line_exp3_block(const double *__restrict__ x, int n0, int n1, int n2, int b0, int b1,
                                                 int zb, int ze, int *__restrict__ e0, int *__restrict__ e1,
-                                                int *__restrict__ e2) {
+                                                int *__restrict__ e2, const Exp3Windows &W = Exp3Windows()) {
     __shared__ int ys[kExpChunk][8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int i0 = b0 + tx, i1 = b1 + ty;
@@ -234,6 +261,7 @@ __device__ __forceinline__ void line_exp3_block(const double *__restrict__ x, in
     const int c1 = ty, row = threadIdx.x >> 2, q0 = threadIdx.x & 3;
     const int c0r = row >> 3, r0 = row & 7;
     const int i1r = b1 + r0;
+    int *const column = e2 + i0 + (long long)n0 * i1;
     int zmax = 0;
     // the next chunk's loads are in flight while this chunk is reduced
     unsigned long long raw[kExpChunk];
@@ -246,46 +274,52 @@ __device__ __forceinline__ void line_exp3_block(const double *__restrict__ x, in
         const int c1n = c0 + kExpChunk;
 #pragma unroll
         for (int c = 0; c < kExpChunk; ++c) raw[c] = (valid && c1n + c < ze) ? xa[plane * (c1n + c)] : 0ull;
+        if (WIN && W.wins[2]) zmax = 0;
 #pragma unroll
         for (int c = 0; c < kExpChunk; ++c) {
             zmax = max(zmax, e[c]);
             ys[c][ty][tx] = e[c];
         }
+        if (WIN && W.wins[2] && valid) exp3_raise<true>(column, c0 / 8, n2, W.wins[2], W.lines[2], zmax);
         __syncthreads();
         if (c0 + c1 < ze && i0 < n0) {
             int m = ys[c1][0][tx];
 #pragma unroll
             for (int r = 1; r < 8; ++r) m = max(m, ys[c1][r][tx]);
-            atomicMax(e1 + i0 + (long long)n0 * (c0 + c1), m);
+            exp3_raise<WIN>(e1 + i0 + (long long)n0 * (c0 + c1), b1 / 8, n1, W.wins[1], W.lines[1], m);
         }
         {
             int m = ys[c0r][r0][8 * q0];
 #pragma unroll
             for (int k = 1; k < 8; ++k) m = max(m, ys[c0r][r0][8 * q0 + k]);
+            const bool keeps = c0 + c0r < ze && i1r < n1;
+            int *const line = e0 + i1r + (long long)n1 * (c0 + c0r);
+            // the four quarters lie in one run of 64; its ends are the outer ones'
+            if (WIN && W.wins[0] && keeps && b0 + 8 * q0 < n0) exp3_edges(line, b0 / 8 + q0, n0, W.wins[0], W.lines[0], m);
             m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
             m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            if (q0 == 0 && c0 + c0r < ze && i1r < n1) atomicMax(e0 + i1r + (long long)n1 * (c0 + c0r), m);
+            if (q0 == 0 && keeps) atomicMax(line + (WIN && W.wins[0] ? (b0 >> 6) * W.lines[0] : 0), m);
         }
         __syncthreads();
     }
-    if (valid) {
-        int *const p = e2 + i0 + (long long)n0 * i1;
-        if (zb == 0 && ze == n2) *p = zmax;
-        else atomicMax(p, zmax);
+    if (valid && !(WIN && W.wins[2])) {
+        if (zb == 0 && ze == n2) *column = zmax;
+        else atomicMax(column, zmax);
     }
 }
 
+template <bool WIN>
 __global__ void __launch_bounds__(256)
-line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg,
+line_exp3_kernel(const double *__restrict__ x, int n0, int n1, int n2, int nseg, int seglen,
                  int *__restrict__ e0, int *__restrict__ e1, int *__restrict__ e2,
-                 const int *__restrict__ active) {
+                 const int *__restrict__ active, const __grid_constant__ Exp3Windows W) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const long long a = blockIdx.z / nseg;
     if (active && !active[a]) return;                   // grid skipped (uniform over the block)
-    const int seg = blockIdx.z % nseg, seglen = (n2 + nseg - 1) / nseg, zb = seg * seglen;
+    const int zb = blockIdx.z % nseg * seglen;
     if (zb >= n2) return;                               // more segments than seglen fills
-    line_exp3_block(x + a * n0 * n1 * n2, n0, n1, n2, blockIdx.x * 32, blockIdx.y * 8, zb, min(n2, zb + seglen),
-                    e0 + a * n1 * n2, e1 + a * n0 * n2, e2 + a * n0 * n1);
+    line_exp3_block<WIN>(x + a * n0 * n1 * n2, n0, n1, n2, blockIdx.x * 32, blockIdx.y * 8, zb, min(n2, zb + seglen),
+                         e0 + a * n1 * n2, e1 + a * n0 * n2, e2 + a * n0 * n1, W);
 }
 
 // The same for the grids of a batch: d0, d1, d2 describe the non-rotating sweeps
@@ -302,7 +336,7 @@ line_exp3_batch_kernel(const Sweep *__restrict__ d0, const Sweep *__restrict__ d
     for (int t = blockIdx.x; t < tiles * nseg; t += gridDim.x) {
         const int tile = t % tiles, zb = t / tiles * seglen;
         if (zb < n2)
-            line_exp3_block(S.x, n0, n1, n2, tile % gx * 32, tile / gx * 8, zb, min(n2, zb + seglen),
+            line_exp3_block<false>(S.x, n0, n1, n2, tile % gx * 32, tile / gx * 8, zb, min(n2, zb + seglen),
                             e0 + d0[blockIdx.y].le_off, e1 + S.le_off, e2 + d2[blockIdx.y].le_off);
     }
 }
@@ -325,7 +359,11 @@ int tc_windows(const Sweep &S) {
 
 long long sweep_tc_exps(const Sweep &S) { return sweep_tc_lines(S) * (S.le_win > 0 ? S.le_win : 1); }
 
-cudaError_t launch_line_exp3(const double *x, int n0, int n1, int n2, int narr, int *e0, int *e1,
+// Extents whose exponent windows the shared pass can take: the windows of a 17-tap
+// filter (8 elements on each side) over whole pieces of 8.
+bool line_exp3_windows(const Sweep &S) { return S.ntaps == 17 && S.lowfil == -8 && S.qlo == 0 && S.n % 8 == 0; }
+
+cudaError_t launch_line_exp3(const double *x, int n0, int n1, int n2, int narr, const int *wins, int *e0, int *e1,
                              int *e2, cudaStream_t st, const int *active) {
     if (n0 < 1 || n1 < 1 || n2 < 1 || narr < 1 || narr > 65535) return cudaErrorInvalidValue;
     const long long gx = (n0 + 31) / 32, gy = (n1 + 7) / 8;
@@ -336,19 +374,30 @@ cudaError_t launch_line_exp3(const double *x, int n0, int n1, int n2, int narr, 
     if (nseg > most) nseg = most;
     if (nseg > 65535 / narr) nseg = 65535 / narr;
     if (nseg < 1) nseg = 1;
+    int seglen = (int)((n2 + nseg - 1) / nseg);
+    tck::Exp3Windows W;
+    size_t c[3] = {(size_t)n1 * n2 * narr, (size_t)n0 * n2 * narr, (size_t)n0 * n1 * narr};
+    bool win = false;
+    for (int k = 0; k < 3; ++k) {
+        W.lines[k] = (long long)c[k];
+        W.wins[k] = wins ? wins[k] : 0;
+        if (W.wins[k] > 0) win = true, c[k] *= (size_t)W.wins[k];
+    }
+    if (W.wins[2] > 0) seglen = (seglen + 7) / 8 * 8;
     // one clear when the three lie back to back
-    const size_t c0 = (size_t)n1 * n2 * narr, c1 = (size_t)n0 * n2 * narr, c2 = (size_t)n0 * n1 * narr;
+    const bool clear2 = nseg > 1 || W.wins[2] > 0;
     cudaError_t e;
-    if (e1 == e0 + c0 && e2 == e1 + c1) {
-        e = cudaMemsetAsync(e0, 0, (c0 + c1 + (nseg > 1 ? c2 : 0)) * sizeof(int), st);
+    if (e1 == e0 + c[0] && e2 == e1 + c[1]) {
+        e = cudaMemsetAsync(e0, 0, (c[0] + c[1] + (clear2 ? c[2] : 0)) * sizeof(int), st);
     } else {
-        e = cudaMemsetAsync(e0, 0, c0 * sizeof(int), st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(e1, 0, c1 * sizeof(int), st);
-        if (e == cudaSuccess && nseg > 1) e = cudaMemsetAsync(e2, 0, c2 * sizeof(int), st);
+        e = cudaMemsetAsync(e0, 0, c[0] * sizeof(int), st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(e1, 0, c[1] * sizeof(int), st);
+        if (e == cudaSuccess && clear2) e = cudaMemsetAsync(e2, 0, c[2] * sizeof(int), st);
     }
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)(narr * nseg));
-    tck::line_exp3_kernel<<<grid, 256, 0, st>>>(x, n0, n1, n2, (int)nseg, e0, e1, e2, active);
+    if (win) tck::line_exp3_kernel<true><<<grid, 256, 0, st>>>(x, n0, n1, n2, (int)nseg, seglen, e0, e1, e2, active, W);
+    else tck::line_exp3_kernel<false><<<grid, 256, 0, st>>>(x, n0, n1, n2, (int)nseg, seglen, e0, e1, e2, active, W);
     return cudaGetLastError();
 }
 
@@ -602,7 +651,7 @@ cudaError_t launch_sweep_tc(const Sweep &S_in, const TcFilter &F, int sch, int *
         S.n % 4 == 0 && S.in_ext % 4 == 0 && S.x_arr % 4 == 0 && (((uintptr_t)S.x) & 31) == 0)
         S.woff = ((S.qlo + S.lowfil) % 4 + 4) % 4;
     if (sch == SCH_EXACT) {
-        if (S.le_win > 0 && (lineE_ready || !lineE)) return cudaErrorInvalidValue;
+        if (S.le_win > 0 && !lineE) return cudaErrorInvalidValue;
         if (lineE && !lineE_ready) {
             const long long total = sweep_tc_lines(S);
             // threads with something to do: a warp per contiguous line or window, a

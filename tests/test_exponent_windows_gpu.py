@@ -144,3 +144,26 @@ def test_poisson_derivatives_of_long_lines(pkg, O, nord):
         bound = np.moveaxis(TOL * taps * run_scales(line, -8, 17), -1, 2 - axis)
         err = np.abs(np.asarray(du).ravel()[axis * N:(axis + 1) * N] - do[axis * N:(axis + 1) * N])
         assert np.all(err.reshape(u.shape) <= bound), axis
+
+
+# windows shared by the three axes' sweeps (whole pieces of 8; runs of 64 whole and partial, the
+# last one a single piece), mixed with axes below a window, and extents that keep passes of their own
+@pytest.mark.parametrize('geocode', [1, 2, 3])
+@pytest.mark.parametrize('n', [[96, 88, 80], [128, 64, 72], [136, 200, 64], [40, 96, 264], [90, 96, 104], [80, 80, 81]])
+def test_shared_windows_are_those_of_single_sweeps(pkg, n, geocode):
+    """nabla, whose three sweeps share one exponent pass, gives the bits of three single derivatives."""
+    h = np.array([0.1, 0.12, 0.09])
+    N = int(np.prod(n))
+    r = np.random.default_rng(N + geocode)
+    u = r.uniform(-1, 1, n[::-1])
+    for ax in range(3):
+        k = np.arange(n[ax]) * 3 // n[ax] - 1
+        u = u * (2.0 ** (-35.0 * k * k)).reshape([-1 if 2 - d == ax else 1 for d in range(3)])
+    u[3, 5] = 0.0
+    u = u.ravel()
+    P = pkg.Poisson()
+    bc = {1: [-2, -2, -2], 2: [0, 0, 0], 3: [0, -2, 0]}[geocode]
+    du = np.asarray(P.nabla_u(geocode, n, u, 16, h)).ravel()
+    for ax in range(3):
+        one = np.asarray(P.broker(16, ax, n, bc[ax], u, 1.0 / h[ax])).ravel()
+        assert np.array_equal(du[ax * N:(ax + 1) * N], one), ax
