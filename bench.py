@@ -1627,8 +1627,11 @@ def run_gpu(args):
     barrier()
     e_steps = max(2, min(args.steps, 5))
     t0 = time.perf_counter()
-    for _ in range(e_steps):
+    e_ms = []
+    for _ in range(e_steps):                         # host-pointer calls return when they are done
+        t1 = time.perf_counter()
         W.host_step(pkg, B, hx, ho0, ho1)
+        e_ms.append(1e3 * (time.perf_counter() - t1))
     torch.cuda.synchronize()
     barrier()
     e_t = (time.perf_counter() - t0) / e_steps
@@ -1638,6 +1641,9 @@ def run_gpu(args):
         h2d, d2h = B * (Ni + No) * 8, B * (Ni + No) * 8
     e2e = {'value': pts_step / e_t, 'unit': UNIT, 'h2d_bytes_per_step': h2d,
            'd2h_bytes_per_step': d2h, 'plain_copy_gbs': link_rates(torch, host_x, pin0, dev),
+           # single steps that take several times the others are the host's (they come every
+           # half second or so, with every version of the library)
+           'ms_per_step': {'min': min(e_ms), 'median': float(np.median(e_ms)), 'max': max(e_ms)},
            'note': W.e2e_note}
 
     # roofline of the dominant kernel
