@@ -94,14 +94,15 @@ __device__ __forceinline__ void line_exp_lines(const Sweep &S, int plen, int *ou
     }
 }
 
+template <int I>
 __global__ void line_exp_kernel(const Sweep S, int plen, int *out) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // the sweep's prologue may begin
     if (S.le_next)                       // the exponents that the sweep will hand on
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < S.le_next_lines * S.narr;
              i += (long long)gridDim.x * blockDim.x)
             S.le_next[i] = 0;
-    line_exp_lines<1, 4>(S, plen, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
-                   (long long)gridDim.x * blockDim.x);
+    line_exp_lines<1, I>(S, plen, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
+                         (long long)gridDim.x * blockDim.x);
 }
 
 // Input positions 0..plen-1 a sweep's outputs read along its line: the whole
@@ -689,7 +690,11 @@ cudaError_t launch_sweep_tc(const Sweep &S_in, const TcFilter &F, int sch, int *
                 fast_div((unsigned int)S.nL, by.left.d, by.left.m, by.left.s);
                 tck::window_exp_kernel<<<grid > 0 ? grid : 1, 256, 0, st>>>(S, by, lineE);
             } else {
-                tck::line_exp_kernel<<<grid > 0 ? grid : 1, 256, 0, st>>>(S, tck::line_exp_plen(S), lineE);
+                // a warp or two an SM: more loads in flight for each (one line of 10^6 points,
+                // kinetic filter: the call 2773 us with four, 2121 with eight)
+                const int plen = tck::line_exp_plen(S);
+                if (units < 2LL * tck::sm_count()) tck::line_exp_kernel<8><<<grid > 0 ? grid : 1, 256, 0, st>>>(S, plen, lineE);
+                else tck::line_exp_kernel<4><<<grid, 256, 0, st>>>(S, plen, lineE);
             }
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
