@@ -329,7 +329,7 @@ __global__ void reduce_parts(const float *part, int nparts, int len, float *out)
 // the output planes (bias + ReLU / mask / field scale, 32 B stored per
 // point).  Several CTAs reside per SM (three at TZ = 8), so one CTA's
 // staging overlaps another's MMAs and epilogue; on GB300 one M = 128 MMA of
-// this shape costs about 80 cycles whatever N (16-48), following its 4 KB A
+// this shape costs 64 to 76 cycles whatever N (16-48), following its 4 KB A
 // tile, so the layer is bound by the number of A tiles read, which is what
 // the z-tap stacking cuts.  Every wait is bounded; a wait that gives up sets
 // the device status word.
@@ -466,12 +466,12 @@ __device__ __forceinline__ void stage(const ConvArgs &A, uint8_t *halo, int s, i
     }
 }
 
-// The MMAs of one tile (thread 0).  One thread issues some 94 of them, so what
+// The MMAs of one tile (thread 0).  One thread issues 97 of them (TZ = 8), so what
 // it computes in between sets their pace: descriptors are formed once and
 // advanced by adding to their start address field (16-byte units).  Formed anew
-// for each MMA, 64 grids of 48^3 took 199 us, so 189.  What is left is about 64
-// cycles an MMA on the tensor pipe, whatever N and the alignment of A (143 us for
-// that layer), behind the staging and drain of three CTAs a SM.
+// for each MMA, 64 grids of 48^3 took 199 us, so 189.  What is left is 64 to 76
+// cycles an MMA on the tensor pipe, whatever N and the alignment of A (136 us for
+// that layer at 64), behind the staging and drain of three CTAs a SM.
 template <int TZ>
 __device__ __forceinline__ void issue_tile(uint32_t tmem, uint32_t hb, uint32_t wb) {
     using G = Geo<TZ>;

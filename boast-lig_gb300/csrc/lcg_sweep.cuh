@@ -81,6 +81,8 @@ cudaError_t launch_dot_reduce(const double *part, long long count, double *out, 
                               cudaStream_t st);
 // Segmented form: out[j * out_stride] = sum of part[j*seg_len .. (j+1)*seg_len)
 // for j < nseg (fixed order), on `st`.
+cudaError_t launch_dot_reduce_seg(const double *part, long long seg_len, int nseg, double *out,
+                                  long long out_stride, cudaStream_t st);
 // The same for a plan's dot products in one launch: product i's partials are
 // part + off[i], len[i] of them for each of nseg segments, its results at
 // out[slot[i] + segment out_stride].
@@ -92,8 +94,6 @@ struct DotList {
 };
 cudaError_t launch_dot_reduce_list(const double *part, const DotList &L, int nseg, double *out,
                                    long long out_stride, cudaStream_t st);
-cudaError_t launch_dot_reduce_seg(const double *part, long long seg_len, int nseg, double *out,
-                                  long long out_stride, cudaStream_t st);
 // The m = nord/2 one-sided outputs at each end of every line of a
 // non-periodic Poisson sweep (c1D(:, i-m) on the first nord+1 points, c1D(:,
 // i-n+m+1) on the last), y = a * sum (or y += when accumulate).

@@ -67,6 +67,12 @@ extern "C" {
  *   FP64:      plain FP64 FMA kernels on the CUDA cores (default).
  *   TC_EXACT:  tcgen05 tensor cores with exact integer digit arithmetic (FP16
  *              byte digits, FP32 accumulation kept exact); FP64-class accuracy.
+ *              Results are accurate relative to the largest input of their
+ *              line (62 bits below it are kept); along periodic lines of 96
+ *              points or more (80 for filters of 16 and 17 taps), of their run
+ *              of 64 outputs, except in 3D kinetic operators, batches and
+ *              MagicFilter3D along 128 points.  An Inf or NaN makes NaN of
+ *              the line, or of the runs that read it.
  *   TC_BF16X3: split precision, 3 bfloat16 terms per operand, 6 products,
  *              FP32 accumulation; relative error near 1e-7.
  *   TC_TF32X3: split precision, 2 tf32 terms per operand, 3 products, FP32
